@@ -48,26 +48,26 @@ def listed():
         # a frame loop's energy probe on device buffers: the smallest call, two launches
         dict(name="energy on device arrays", kind="energy", shape="bar", nx=9, ny=7, nz=31),
         # one body of an interactive scene: a step that is nothing but latency
-        dict(name="step, small bar", kind="step", shape="bar", nx=3, ny=3, nz=9, fp64=False),
+        dict(name="small bar step", kind="step", shape="bar", nx=3, ny=3, nz=9, fp64=False),
         # the headline workload: one normal-flow step of the 220k-tet blob
-        dict(name="step, large blob", kind="step", shape="blob", n=64, fp64=False),
+        dict(name="large blob step", kind="step", shape="blob", n=64, fp64=False),
         # the plain FP64 path on a mid-size body (reference results)
-        dict(name="step, blob in FP64", kind="step", shape="blob", n=30, fp64=True),
+        dict(name="FP64 blob step", kind="step", shape="blob", n=30, fp64=True),
         # many independent bodies with self-contact in one arena
-        dict(name="step, batch in contact", kind="batch", count=20, tmin=200, tmax=6000, fp64=False),
+        dict(name="contact batch step", kind="batch", count=20, tmin=200, tmax=6000, fp64=False),
         # the reference's normal-flow script on a shell about the size of its cat.obj
-        dict(name="flow step, shell", kind="flow", n=48, fp64=False),
+        dict(name="shell flow step", kind="flow", n=48, fp64=False),
         # the character-sequence script under gravity: next frame as rest shape, velocity and DBC targets
-        dict(name="sequence frame, elastic shell", kind="shell", n=41, fp64=False),
+        dict(name="elastic shell frame", kind="shell", n=41, fp64=False),
         # a program with its own outer loop: the linear solve alone, to FP64 accuracy
         dict(name="Newton direction", kind="direction", shape="blob", n=45, fp64=False),
         # an optimiser's objective and gradient at an odd small size
         dict(name="energy and gradient", kind="gradient", shape="bar", nx=7, ny=5, nz=13, fp64=False),
         # operator product in FP64 (eigenvalue or sensitivity codes)
-        dict(name="Hessian product in FP64", kind="hessian", shape="bar", nx=11, ny=13, nz=45, fp64=True),
+        dict(name="FP64 Hessian product", kind="hessian", shape="bar", nx=11, ny=13, nz=45, fp64=True),
         # contact queries of a packed scene
-        dict(name="constraint set, plate stack", kind="contacts", nx=33, ny=29, plates=7),
-        dict(name="CCD step size, plate stack", kind="ccd", nx=33, ny=29, plates=7),
+        dict(name="plate stack contacts", kind="contacts", nx=33, ny=29, plates=7),
+        dict(name="plate stack CCD", kind="ccd", nx=33, ny=29, plates=7),
     ]
 
 
