@@ -1548,9 +1548,10 @@ int pcg_solve(Arena& A, Work& W, const ContactSet& cs, bool fp64, const double* 
             if (rc) return rc;
             hrr_current = true;
             for (int i = 0; i < nI; ++i) {
+                if (!act[i]) continue;  // stopped at an earlier sweep: its residual stands
                 const double ti = tol_host ? std::max(rel_tol, tol_host[i]) : rel_tol;
-                const bool stalled = act[i] && hrr[i] > 0.25 * prev[i];
-                act[i] = act[i] && b2[i] > 0 && hrr[i] > ti * ti * b2[i] && !stalled;
+                const bool stalled = hrr[i] > 0.25 * prev[i];
+                act[i] = b2[i] > 0 && hrr[i] > ti * ti * b2[i] && !stalled;
                 relres_out[i] = b2[i] > 0 ? std::sqrt(hrr[i] / b2[i]) : 0.0;
                 prev[i] = hrr[i];
                 any |= act[i] != 0;
@@ -1588,8 +1589,8 @@ int pcg_solve(Arena& A, Work& W, const ContactSet& cs, bool fp64, const double* 
     if (!hrr_current) {
         rc = residual(hrr);
         if (rc) return rc;
+        for (int i = 0; i < nI; ++i) relres_out[i] = b2[i] > 0 ? std::sqrt(hrr[i] / b2[i]) : 0.0;
     }
-    for (int i = 0; i < nI; ++i) relres_out[i] = b2[i] > 0 ? std::sqrt(hrr[i] / b2[i]) : 0.0;
     return IDP_OK;
 }
 
