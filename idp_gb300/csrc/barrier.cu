@@ -327,7 +327,7 @@ __global__ void k_barrier_gh(long C, const int4* __restrict__ cons, const int* _
     T H[144];
     for (int k = 0; k < n * n; ++k) H[k] = (T)Hd[k];
     if (!chol_pd(H, n)) {
-        // indefinite: projected by k_psd_warp (one warp per matrix)
+        // indefinite: projected by k_psd_project
         T* hl = hloc + 144 * i;
         for (int k = 0; k < n * n; ++k) hl[k] = H[k];
         hn[i] = n;
@@ -338,38 +338,35 @@ __global__ void k_barrier_gh(long C, const int4* __restrict__ cons, const int* _
 }
 
 // The 12x12 PSD projection of makePD (Math/UTILS.h:10-27) for the matrices
-// k_barrier_gh found indefinite, one warp per matrix (psd_warp_project).
+// k_barrier_gh found indefinite, 16 lanes per matrix (psd_group_project)
 template <class T>
-__global__ void __launch_bounds__(32 * kPsdWarps) k_psd_warp(const int* __restrict__ plist,
-                                                               const unsigned int* __restrict__ pcount,
-                                                               const T* __restrict__ hloc,
-                                                               const int* __restrict__ hn, T* __restrict__ hout) {
-    __shared__ T sA[kPsdWarps][144], sV[kPsdWarps][144], sCS[kPsdWarps][6][2], sW[kPsdWarps][12];
-    __shared__ int sPQ[kPsdWarps][6][2];
-    const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    T* A = sA[w];
-    T* Vm = sV[w];
+__global__ void __launch_bounds__(kPsdThreads) k_psd_project(const int* __restrict__ plist,
+                                                             const unsigned int* __restrict__ pcount,
+                                                             const T* __restrict__ hloc,
+                                                             const int* __restrict__ hn, T* __restrict__ hout) {
+    __shared__ PsdScratch<T> scr[kPsdPerCta];
+    const int grp = threadIdx.x / kPsdGroup, j = threadIdx.x % kPsdGroup;
+    PsdScratch<T>& sc = scr[grp];
     const unsigned int cnt = *pcount;
-    for (unsigned int item = blockIdx.x * kPsdWarps + w; item < cnt; item += gridDim.x * kPsdWarps) {
-        const int i = plist[item];
-        const int n = hn[i];
-        for (int k = lane; k < n * n; k += 32) {
-            A[k] = hloc[144L * i + k];
-            Vm[k] = (k / n == k % n) ? T(1) : T(0);
+    // both groups of a warp run the same number of rounds (shuffles cross them)
+    for (unsigned int first = blockIdx.x * kPsdPerCta; first < cnt; first += gridDim.x * kPsdPerCta) {
+        const unsigned int item = first + grp;
+        const int i = item < cnt ? plist[item] : -1;
+        const int n = i >= 0 ? hn[i] : 0;
+        for (int t = j; t < kPsdDim * kPsdDim; t += kPsdGroup) {
+            const int r = t / kPsdDim, c = t % kPsdDim;
+            sc.A[t] = r < n && c < n ? hloc[144L * i + r * n + c] : T(0);
         }
         __syncwarp();
-        psd_warp_project(A, Vm, n, sCS[w], sPQ[w], sW[w], lane);
+        psd_group_project(sc, n, j);
         const int nv = n / 3;
-        T* ho = hout + 90L * i;
-        for (int t = lane; t < 90; t += 32) {
-            const int blk = t / 9, d = (t % 9) / 3, e = t % 3;
-            int a = 0, b = 0, kk = blk;
-            for (a = 0; a < 4; ++a) {
-                if (kk < 4 - a) { b = a + kk; break; }
-                kk -= 4 - a;
+        if (i >= 0)
+            for (int t = j; t < 90; t += kPsdGroup) {
+                int a = 0, kk = t / 9;
+                while (kk >= 4 - a) { kk -= 4 - a; ++a; }
+                const int b = a + kk, d = (t % 9) / 3, e = t % 3;
+                hout[90L * i + t] = (a < nv && b < nv) ? psd_entry(sc, n, 3 * a + d, 3 * b + e) : T(0);
             }
-            ho[t] = (a < nv && b < nv) ? A[(3 * a + d) * n + 3 * b + e] : T(0);
-        }
         __syncwarp();
     }
 }
@@ -513,13 +510,13 @@ static int barrier_gh(Arena& A, Work& W, const double* X, const ContactSet& cs, 
             int* plist = reinterpret_cast<int*>(pb + o_l);
             unsigned int* pcount = reinterpret_cast<unsigned int*>(pb + o_c);
             IDP_CUDA_TRY(cudaMemsetAsync(pcount, 0, sizeof(unsigned int), s));
-            const int pgrid = (int)std::min<long>((C + kPsdWarps - 1) / kPsdWarps, 8L * 152);
+            const int pgrid = (int)std::min<long>((C + kPsdPerCta - 1) / kPsdPerCta, 16L * 152);
             if (hess_mode == 1) {
                 (::idp::count_launch(), k_barrier_gh<double><<<grid_for(C, 64), 64, 0, s>>>(
                                             C, cons, cinst, A.active, X, A.X0, A.dHat2, A.kappa, A.thickness,
                                             W[W_BG].as<double>(), W[W_BH].as<double>(), reinterpret_cast<double*>(pb),
                                             hn, plist, pcount));
-                (::idp::count_launch(), k_psd_warp<double><<<pgrid, 32 * kPsdWarps, 0, s>>>(
+                (::idp::count_launch(), k_psd_project<double><<<pgrid, kPsdThreads, 0, s>>>(
                                             plist, pcount, reinterpret_cast<const double*>(pb), hn,
                                             W[W_BH].as<double>()));
             } else {
@@ -527,7 +524,7 @@ static int barrier_gh(Arena& A, Work& W, const double* X, const ContactSet& cs, 
                                             C, cons, cinst, A.active, X, A.X0, A.dHat2, A.kappa, A.thickness,
                                             W[W_BG].as<double>(), W[W_BH].as<float>(), reinterpret_cast<float*>(pb),
                                             hn, plist, pcount));
-                (::idp::count_launch(), k_psd_warp<float><<<pgrid, 32 * kPsdWarps, 0, s>>>(
+                (::idp::count_launch(), k_psd_project<float><<<pgrid, kPsdThreads, 0, s>>>(
                                             plist, pcount, reinterpret_cast<const float*>(pb), hn,
                                             W[W_BH].as<float>()));
             }

@@ -326,115 +326,78 @@ __global__ void k_grad_gather_shell(long V, const int* __restrict__ vinst, const
     g[3 * v + 2] += s2;
 }
 
-// the upper 3x3 blocks (a <= b) of an nv-vertex element's 3nv x 3nv matrix
-template <class S, class T>
-__device__ __forceinline__ void store_blocks(const S* H, int nv, T* ho) {
-    const int n = 3 * nv;
-    int k = 0;
-    for (int a = 0; a < nv; ++a)
-        for (int b = a; b < nv; ++b, ++k)
-            for (int d = 0; d < 3; ++d)
-                for (int e = 0; e < 3; ++e) ho[k * 9 + d * 3 + e] = (T)H[(3 * a + d) * n + 3 * b + e];
-}
-
 // blocks of shell element e: faces e < Fm (6 blocks at 54 e), then hinges
 // (10 blocks at 54 Fm + 90 (e - Fm))
 __device__ __forceinline__ long shell_block_off(long e, long Fm) { return e < Fm ? 54 * e : 54 * Fm + 90 * (e - Fm); }
 
-// an element Hessian (n x n, FP64) in the working precision T: stored as it
-// is when the Cholesky test finds it positive definite, else queued for the
-// warp projection (an element Hessian is singular along its rigid motions,
-// so nearly all are queued)
+// an element Hessian (n x n, FP64) in the working precision T, left for the
+// projection: every one is singular along its rigid motions, so none would
+// pass a Cholesky test
 template <class T>
-__device__ void shell_element_out(const double* H, int n, long e, long Fm, T* __restrict__ hout,
-                                  T* __restrict__ hloc, int* __restrict__ hn, int* __restrict__ plist,
-                                  unsigned int* __restrict__ pcount) {
-    T Ht[144];
-    for (int k = 0; k < n * n; ++k) Ht[k] = (T)H[k];
-    if (chol_pd(Ht, n)) {
-        store_blocks(Ht, n / 3, hout + shell_block_off(e, Fm));
-        return;
-    }
-    T* hl = hloc + 144 * e;
-    for (int k = 0; k < n * n; ++k) hl[k] = Ht[k];
-    hn[e] = n;
-    plist[atomicAdd(pcount, 1u)] = (int)e;
+__device__ __forceinline__ void shell_element_out(const double* H, int n, T* __restrict__ hl) {
+    for (int k = 0; k < n * n; ++k) hl[k] = (T)H[k];
 }
 
 template <class T>
 __global__ void k_membrane_hess(long Fm, const int* __restrict__ finst, const unsigned char* __restrict__ active,
                                 const double* __restrict__ X, const int* __restrict__ mface,
                                 const double* __restrict__ mem, const unsigned char* __restrict__ dbc, double w,
-                                T* __restrict__ hout, T* __restrict__ hloc, int* __restrict__ hn,
-                                int* __restrict__ plist, unsigned int* __restrict__ pcount) {
+                                T* __restrict__ hloc, int* __restrict__ hn) {
     const long f = (long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (f >= Fm || !active[finst[f]]) return;
+    if (f >= Fm) return;
     const int* t = mface + 3 * f;
-    if (all_fixed(dbc, t, 3)) {
-        for (int k = 0; k < 54; ++k) hout[54 * f + k] = T(0);
-        return;
-    }
+    const bool act = active[finst[f]] != 0, fixed = act && all_fixed(dbc, t, 3);
+    hn[f] = !act ? -1 : (fixed ? 0 : 9);  // -1: blocks left as they are, 0: zero blocks
+    if (!act || fixed) return;
     double H[81];
     membrane_face(ld(X, t[0]), ld(X, t[1]), ld(X, t[2]), mem + 7 * f, w, nullptr, H);
-    shell_element_out(H, 9, f, Fm, hout, hloc, hn, plist, pcount);
+    shell_element_out(H, 9, hloc + 144 * f);
 }
 
 template <class T>
 __global__ void k_bending_hess(long Hn, long Fm, const int* __restrict__ hinst, const unsigned char* __restrict__ active,
                                const double* __restrict__ X, const int4* __restrict__ hinge,
                                const double* __restrict__ hk, const unsigned char* __restrict__ dbc, double w,
-                               T* __restrict__ hout, T* __restrict__ hloc, int* __restrict__ hn,
-                               int* __restrict__ plist, unsigned int* __restrict__ pcount) {
+                               T* __restrict__ hloc, int* __restrict__ hn) {
     const long i = (long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= Hn || !active[hinst[i]]) return;
+    if (i >= Hn) return;
     const int4 hh = hinge[i];
     const int v[4] = {hh.x, hh.y, hh.z, hh.w};
-    if (all_fixed(dbc, v, 4)) {
-        for (int q = 0; q < 90; ++q) hout[54 * Fm + 90 * i + q] = T(0);
-        return;
-    }
+    const bool act = active[hinst[i]] != 0, fixed = act && all_fixed(dbc, v, 4);
+    hn[Fm + i] = !act ? -1 : (fixed ? 0 : 12);
+    if (!act || fixed) return;
     double H[144];
     bending_hinge(ld(X, v[0]), ld(X, v[1]), ld(X, v[2]), ld(X, v[3]), hk + 2 * i, w, nullptr, H);
-    shell_element_out(H, 12, Fm + i, Fm, hout, hloc, hn, plist, pcount);
+    shell_element_out(H, 12, hloc + 144 * (Fm + i));
 }
 
-// makePD of the queued element Hessians, one warp per matrix
-// (psd_warp_project), written to the element's blocks
+// makePD of the element Hessians, 16 lanes per matrix (psd_group_project),
+// written to the element's upper 3x3 blocks
 template <class T>
-__global__ void __launch_bounds__(32 * kPsdWarps) k_shell_psd_warp(const int* __restrict__ plist,
-                                                                     const unsigned int* __restrict__ pcount,
-                                                                     const T* __restrict__ hloc,
-                                                                     const int* __restrict__ hn, long Fm,
-                                                                     T* __restrict__ hout) {
-    __shared__ T sA[kPsdWarps][144], sV[kPsdWarps][144], sCS[kPsdWarps][6][2], sW[kPsdWarps][12];
-    __shared__ int sPQ[kPsdWarps][6][2];
-    const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    T* A = sA[w];
-    T* Vm = sV[w];
-    const unsigned int cnt = *pcount;
-    for (unsigned int item = blockIdx.x * kPsdWarps + w; item < cnt; item += gridDim.x * kPsdWarps) {
-        const long e = plist[item];
-        const int n = hn[e];
-        for (int k = lane; k < n * n; k += 32) {
-            A[k] = hloc[144 * e + k];
-            Vm[k] = (k / n == k % n) ? T(1) : T(0);
+__global__ void __launch_bounds__(kPsdThreads) k_shell_psd(long Ne, const T* __restrict__ hloc,
+                                                           const int* __restrict__ hn, long Fm,
+                                                           T* __restrict__ hout) {
+    __shared__ PsdScratch<T> scr[kPsdPerCta];
+    const int grp = threadIdx.x / kPsdGroup, j = threadIdx.x % kPsdGroup;
+    PsdScratch<T>& sc = scr[grp];
+    // both groups of a warp run the same number of rounds (shuffles cross them)
+    for (long first = (long)blockIdx.x * kPsdPerCta; first < Ne; first += (long)gridDim.x * kPsdPerCta) {
+        const long e = first + grp;
+        const int n = e < Ne ? hn[e] : -1;
+        for (int t = j; t < kPsdDim * kPsdDim; t += kPsdGroup) {
+            const int r = t / kPsdDim, c = t % kPsdDim;
+            sc.A[t] = r < n && c < n ? hloc[144 * e + r * n + c] : T(0);
         }
         __syncwarp();
-        psd_warp_project(A, Vm, n, sCS[w], sPQ[w], sW[w], lane);
-        const int nv = n / 3, nb = nv * (nv + 1) / 2;
-        T* ho = hout + shell_block_off(e, Fm);
-        for (int t = lane; t < 9 * nb; t += 32) {
-            const int blk = t / 9, d = (t % 9) / 3, c = t % 3;
-            int a = 0, b = 0, kk = blk;
-            for (a = 0; a < nv; ++a) {
-                if (kk < nv - a) {
-                    b = a + kk;
-                    break;
-                }
-                kk -= nv - a;
+        psd_group_project(sc, n, j);
+        const int nv = e < Fm ? 3 : 4;
+        if (n >= 0)
+            for (int t = j; t < 9 * nv * (nv + 1) / 2; t += kPsdGroup) {
+                int a = 0, kk = t / 9;
+                while (kk >= nv - a) { kk -= nv - a; ++a; }
+                hout[shell_block_off(e, Fm) + t] =
+                    n > 0 ? psd_entry(sc, n, 3 * a + (t % 9) / 3, 3 * (a + kk) + t % 3) : T(0);
             }
-            ho[t] = A[(3 * a + d) * n + 3 * b + c];
-        }
         __syncwarp();
     }
 }
@@ -480,28 +443,21 @@ int shell_gradient(Arena& A, Work& W, const double* X, double w_h2, double* g, c
 // element blocks after the tets' (10 per tet): 6 per face, 10 per hinge
 template <class T>
 static int shell_hessian_t(Arena& A, Work& W, const double* X, double w_h2, T* base, cudaStream_t s) {
-    // PSD queue: local matrices (144 per element) | sizes | list | count
+    // local matrices (144 per element) | sizes
     const long Ne = A.Fm + A.Hn;
     const size_t o_n = ((sizeof(T) * 144 * (size_t)Ne) + 255) & ~size_t(255);
-    const size_t o_l = o_n + ((sizeof(int) * (size_t)Ne + 255) & ~size_t(255));
-    const size_t o_c = o_l + ((sizeof(int) * (size_t)Ne + 255) & ~size_t(255));
-    if (W[W_SHELL_PSD].ensure(o_c + 256)) return IDP_ERR_CUDA;
+    if (W[W_SHELL_PSD].ensure(o_n + sizeof(int) * (size_t)Ne)) return IDP_ERR_CUDA;
     char* pb = W[W_SHELL_PSD].as<char>();
     T* hloc = reinterpret_cast<T*>(pb);
     int* hn = reinterpret_cast<int*>(pb + o_n);
-    int* plist = reinterpret_cast<int*>(pb + o_l);
-    unsigned int* pcount = reinterpret_cast<unsigned int*>(pb + o_c);
-    IDP_CUDA_TRY(cudaMemsetAsync(pcount, 0, sizeof(unsigned int), s));
     if (A.Fm)
         (::idp::count_launch(), k_membrane_hess<T><<<grid_for(A.Fm, 64), 64, 0, s>>>(
-                                    A.Fm, A.finst, A.active, X, A.mface, A.mem, A.dbc_excl, w_h2, base, hloc, hn, plist,
-                                    pcount));
+                                    A.Fm, A.finst, A.active, X, A.mface, A.mem, A.dbc_excl, w_h2, hloc, hn));
     if (A.Hn)
         (::idp::count_launch(), k_bending_hess<T><<<grid_for(A.Hn, 64), 64, 0, s>>>(
-                                    A.Hn, A.Fm, A.hinst, A.active, X, A.hinge, A.hk, A.dbc_excl, w_h2, base, hloc, hn,
-                                    plist, pcount));
-    const int pgrid = (int)std::min<long>((Ne + kPsdWarps - 1) / kPsdWarps, 8L * 152);
-    (::idp::count_launch(), k_shell_psd_warp<T><<<pgrid, 32 * kPsdWarps, 0, s>>>(plist, pcount, hloc, hn, A.Fm, base));
+                                    A.Hn, A.Fm, A.hinst, A.active, X, A.hinge, A.hk, A.dbc_excl, w_h2, hloc, hn));
+    const int pgrid = (int)std::min<long>((Ne + kPsdPerCta - 1) / kPsdPerCta, 16L * 152);
+    (::idp::count_launch(), k_shell_psd<T><<<pgrid, kPsdThreads, 0, s>>>(Ne, hloc, hn, A.Fm, base));
     return cudaGetLastError() == cudaSuccess ? IDP_OK : IDP_ERR_CUDA;
 }
 
