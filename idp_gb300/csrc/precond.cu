@@ -15,12 +15,22 @@
 #include <numeric>
 #include <vector>
 #include <atomic>
+#include <cooperative_groups.h>
 #include "engine.hpp"
+
+namespace cg = cooperative_groups;
 
 namespace idp {
 
 namespace {
 
+// Row stride of a block's dense matrices: N = 3n rounded up to 4 values, so that
+// rows start on a 16-byte boundary.
+__host__ __device__ inline int block_ld(int N) { return (N + 3) & ~3; }
+
+// dense block of the system matrix for every cluster (K zeroed before):
+// a warp per row, lanes over the row's blocks (their columns differ), then over
+// the contact tail's; blockIdx.y slices of the rows
 template <class T>
 __global__ void k_cl_gather(int ncl, const int* __restrict__ off, const int* __restrict__ vert,
                             const int* __restrict__ vcl, const int* __restrict__ vloc,
@@ -28,177 +38,291 @@ __global__ void k_cl_gather(int ncl, const int* __restrict__ off, const int* __r
                             const int* __restrict__ colidx, const T* __restrict__ val, const int* __restrict__ trp,
                             const int* __restrict__ tcol, const T* __restrict__ tval,
                             const unsigned char* __restrict__ dbc, T* __restrict__ K) {
-    int c = blockIdx.x;
-    int n = off[c + 1] - off[c], N = 3 * n;
+    const int c = blockIdx.x;
+    const int n = off[c + 1] - off[c];
+    const int ld = block_ld(3 * n);
     T* Kc = K + doff[c];
-    for (long i = threadIdx.x; i < (long)N * N; i += blockDim.x) Kc[i] = T(0);
-    __syncthreads();
-    for (int li = threadIdx.x; li < n; li += blockDim.x) {
-        int v = vert[off[c] + li];
+    const int lane = threadIdx.x & 31, warps = blockDim.x >> 5;
+    for (int li = blockIdx.y * warps + (threadIdx.x >> 5); li < n; li += gridDim.y * warps) {
+        const int v = vert[off[c] + li];
+        T* row = Kc + 3L * li * ld;
         if (dbc[v]) {
-            for (int a = 0; a < 3; ++a) Kc[(long)(3 * li + a) * N + 3 * li + a] = T(1);
+            if (lane < 3) row[(long)lane * ld + 3 * li + lane] = T(1);
             continue;
         }
-        for (int k = rowptr[v]; k < rowptr[v + 1]; ++k) {
-            int col = colidx[k];
+        for (int k = rowptr[v] + lane; k < rowptr[v + 1]; k += 32) {
+            const int col = colidx[k];
             if (vcl[col] != c) continue;
-            int lj = vloc[col];
+            const int lj = 3 * vloc[col];
             for (int a = 0; a < 3; ++a)
-                for (int b = 0; b < 3; ++b) Kc[(long)(3 * li + a) * N + 3 * lj + b] += val[9 * (long)k + 3 * a + b];
+                for (int b = 0; b < 3; ++b) row[(long)a * ld + lj + b] = val[9 * (long)k + 3 * a + b];
         }
-        for (int k = trp[v]; k < trp[v + 1]; ++k) {
-            int col = tcol[k];
+        __syncwarp();
+        for (int k = trp[v] + lane; k < trp[v + 1]; k += 32) {
+            const int col = tcol[k];
             if (dbc[col] || vcl[col] != c) continue;
-            int lj = vloc[col];
+            const int lj = 3 * vloc[col];
             for (int a = 0; a < 3; ++a)
-                for (int b = 0; b < 3; ++b) Kc[(long)(3 * li + a) * N + 3 * lj + b] += tval[9 * (long)k + 3 * a + b];
+                for (int b = 0; b < 3; ++b) row[(long)a * ld + lj + b] += tval[9 * (long)k + 3 * a + b];
         }
     }
 }
 
-// Factor every block, one CTA per block, in 32-wide panels:
-//  Cholesky K_c = L L^T (right-looking, in place): the diagonal 32x32 tile is
-//  factored by one warp in shared memory, the panel below it is solved row by
-//  row (thread per row) into shared memory, and the trailing lower triangle
-//  takes the rank-32 update from the staged panel (padded rows, no bank
-//  conflicts);
-//  Y = L^{-1} by block rows: for rows i0..i0+31 every thread owns a column and
-//  keeps the 32 row sums in registers while streaming the column of the rows
-//  above, then solves with the diagonal tile.
-// The PCG applies K_c^{-1} = Y^T Y as z = Y^T (Y r). ok[c] = 0 when a pivot is
+// Factor every block, one thread-block cluster per block (8 CTAs above 96
+// rows, one CTA below), in 32-wide panels:
+//  Cholesky K = L L^T, right-looking. Every CTA factors the 32x32 diagonal
+//  tile and inverts the factor (one warp, rows in registers) and solves the
+//  whole panel below it (a thread per row) while it sits in shared memory, so
+//  the panel needs no exchange; the trailing lower triangle takes the rank-32
+//  update in 64x64 tiles, 4x4 values per thread, shared out over the cluster;
+//  one cluster barrier per panel. L's panels go to the upper triangle
+//  (transposed), the inverted diagonal tiles to Y.
+//  Y = L^{-1} by 32-wide columns, which do not depend on one another and are
+//  shared out over the cluster: a column stays in shared memory and its row
+//  tiles follow in order, Y_i = L_ii^{-1} (- sum_k L_ik Y_k), the sum's k split
+//  over four groups of 64 threads of 4x4 values each.
+// The PCG applies K^{-1} = Y^T Y as z = Y^T (Y r). ok[c] = 0 when a pivot is
 // not positive (the block then falls back to 3x3 inverses).
+// Bound by the chain of 18 panels (tile factor, panel, update, barrier) and the
+// FP32 or FP64 pipe. (One CTA per block with one output per lane and a column
+// of Y per thread took 3.4 ms a call on 20 pairs of bars of 200 to 6,000 tets,
+// a third of their step; with this and the shared-out applies of solver.cu the
+// step went from 175 to 93 ms.) Blocks of up to 96 rows, 3 panels, have too
+// little work between the barriers to share.
 constexpr int kInvThreads = 256;
 constexpr int kTB = 32;
 constexpr int kNMax = 3 * kClusterCap;
+constexpr int kInvClusterRows = 96;              // blocks of more rows take a cluster
+constexpr int kInvCluster = 8;
+constexpr int kPanLd = kNMax + 4;                // panel: [k][row]
+constexpr int kTileLd = kTB + 4;
+constexpr int kInvBuf = kTB * kPanLd;            // panel, or a column of Y ([row][32])
+constexpr int kInvStage = 128 * kTB;             // L rows of one pass, or the groups' partial sums
 
 template <class T>
-size_t invert_smem_bytes() {
-    const size_t pan = (size_t)kNMax * (kTB + 1), rows = (size_t)kTB * (kNMax + 1);
-    return sizeof(T) * ((pan > rows ? pan : rows) + (size_t)kTB * (kTB + 1)) + 64;
+struct alignas(16) Vec4 {
+    T x, y, z, w;
+};
+__device__ __forceinline__ Vec4<float> ldcg4(const float* p) {
+    const float4 v = __ldcg(reinterpret_cast<const float4*>(p));
+    return {v.x, v.y, v.z, v.w};
+}
+__device__ __forceinline__ Vec4<double> ldcg4(const double* p) {
+    const double2 a = __ldcg(reinterpret_cast<const double2*>(p)), b = __ldcg(reinterpret_cast<const double2*>(p) + 1);
+    return {a.x, a.y, b.x, b.y};
+}
+template <class T>
+__device__ __forceinline__ Vec4<T> lds4(const T* p) {
+    return *reinterpret_cast<const Vec4<T>*>(p);
+}
+template <class T>
+__device__ __forceinline__ void st4(T* p, const Vec4<T>& v) {
+    *reinterpret_cast<Vec4<T>*>(p) = v;
+}
+// acc (4x4) += a b^T
+template <class T>
+__device__ __forceinline__ void outer4(T (&acc)[4][4], const Vec4<T>& a, const Vec4<T>& b) {
+    const T av[4] = {a.x, a.y, a.z, a.w}, bv[4] = {b.x, b.y, b.z, b.w};
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+#pragma unroll
+        for (int j = 0; j < 4; ++j) acc[i][j] += av[i] * bv[j];
 }
 
 template <class T>
-__global__ void __launch_bounds__(kInvThreads) k_cl_invert(int ncl, const int* __restrict__ off,
+size_t invert_smem_bytes() {
+    return sizeof(T) * (kInvBuf + kInvStage + 3 * kTB * kTileLd);
+}
+
+// one warp: the kw x kw tile at A (row stride ld, lower triangle) into its
+// Cholesky factor (tile) and that factor's inverse (inv), both 32 x 32 padded
+// with the identity; false when a pivot is not positive
+template <class T>
+__device__ bool tile_factor(const T* A, int ld, int kw, T* tile, T* inv, int lane) {
+    T a[kTB];
+#pragma unroll
+    for (int q = 0; q < kTB; q += 4) {
+        Vec4<T> v = {T(0), T(0), T(0), T(0)};
+        if (lane < kw && q < kw) v = ldcg4(A + (long)lane * ld + q);
+        a[q] = v.x; a[q + 1] = v.y; a[q + 2] = v.z; a[q + 3] = v.w;
+    }
+#pragma unroll
+    for (int q = 0; q < kTB; ++q)
+        if (lane >= kw || q >= kw) a[q] = lane == q ? T(1) : T(0);
+    bool good = true;
+#pragma unroll
+    for (int j = 0; j < kTB; ++j) {
+        const T d = __shfl_sync(0xffffffffu, a[j], j);
+        good = good && d > T(0);
+        const T ljj = sqrt(d), r = T(1) / ljj;
+        a[j] = lane == j ? ljj : (lane > j ? a[j] * r : T(0));
+#pragma unroll
+        for (int q = j + 1; q < kTB; ++q) a[q] -= a[j] * __shfl_sync(0xffffffffu, a[j], q);
+    }
+#pragma unroll
+    for (int q = 0; q < kTB; ++q) tile[lane * kTileLd + q] = a[q];
+    __syncwarp();
+    // column `lane` of the inverse by forward substitution
+    T x[kTB];
+#pragma unroll
+    for (int r = 0; r < kTB; ++r) {
+        T s = r == lane ? T(1) : T(0);
+#pragma unroll
+        for (int t = 0; t < r; ++t) s -= tile[r * kTileLd + t] * x[t];
+        x[r] = s / tile[r * kTileLd + r];
+        inv[r * kTileLd + lane] = x[r];
+    }
+    __syncwarp();
+    return good;
+}
+
+template <class T>
+__global__ void __launch_bounds__(kInvThreads) k_cl_invert(const int* __restrict__ list, const int* __restrict__ off,
                                                            const long long* __restrict__ doff, T* __restrict__ K,
                                                            T* __restrict__ Ybuf, int* __restrict__ ok) {
     extern __shared__ __align__(16) unsigned char inv_smem[];
-    T* big = reinterpret_cast<T*>(inv_smem);                                  // panel or row tile
-    T* dsm = big + (kNMax * (kTB + 1) > kTB * (kNMax + 1) ? kNMax * (kTB + 1) : kTB * (kNMax + 1));  // TB x (TB+1)
+    T* buf = reinterpret_cast<T*>(inv_smem);
+    T* stage = buf + kInvBuf;
+    T* tile = stage + kInvStage;
+    T* inv = tile + kTB * kTileLd;
+    T* R = inv + kTB * kTileLd;
     __shared__ int fail;
-    const int c = blockIdx.x;
-    const int N = 3 * (off[c + 1] - off[c]);
+    cg::cluster_group cl = cg::this_cluster();
+    const int csize = (int)cl.num_blocks(), crank = (int)cl.block_rank();
+    const int c = list[blockIdx.x / csize];
+    const int N = 3 * (off[c + 1] - off[c]), ld = block_ld(N);
     T* L = K + doff[c];
     T* Y = Ybuf + doff[c];
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, nw = kInvThreads / 32;
-    if (tid == 0) fail = 0;
-    __syncthreads();
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     // ---- Cholesky
     for (int k0 = 0; k0 < N; k0 += kTB) {
-        const int kw = min(kTB, N - k0);
-        for (int e = tid; e < kw * kw; e += kInvThreads) {
-            const int r = e / kw, q = e % kw;
-            dsm[r * (kTB + 1) + q] = L[(long)(k0 + r) * N + k0 + q];
-        }
-        __syncthreads();
+        const int kw = min(kTB, N - k0), m0 = k0 + kw, m = N - m0, mt = (m + 63) / 64;
         if (warp == 0) {
-            for (int j = 0; j < kw; ++j) {
-                const T d = dsm[j * (kTB + 1) + j];
-                if (!(d > T(0))) {
-                    if (lane == 0) fail = 1;
-                    break;
+            const bool good = tile_factor(L + (long)k0 * ld + k0, ld, kw, tile, inv, lane);
+            if (lane == 0) fail = good ? 0 : 1;
+        } else {
+            // the panel below, [column][row], rows padded with zeros to the 64-row tiles
+            for (int ri = tid - 32; ri < mt * 64; ri += kInvThreads - 32)
+#pragma unroll
+                for (int q = 0; q < kTB; q += 4) {
+                    Vec4<T> v = {T(0), T(0), T(0), T(0)};
+                    if (ri < m && q < kw) v = ldcg4(L + (long)(m0 + ri) * ld + k0 + q);
+                    buf[q * kPanLd + ri] = v.x;
+                    buf[(q + 1) * kPanLd + ri] = v.y;
+                    buf[(q + 2) * kPanLd + ri] = v.z;
+                    buf[(q + 3) * kPanLd + ri] = v.w;
                 }
-                const T ljj = sqrt(d);
-                __syncwarp();
-                if (lane == j) dsm[j * (kTB + 1) + j] = ljj;
-                if (lane > j && lane < kw) dsm[lane * (kTB + 1) + j] /= ljj;
-                __syncwarp();
-                if (lane > j && lane < kw) {
-                    const T lij = dsm[lane * (kTB + 1) + j];
-                    for (int q = j + 1; q <= lane; ++q) dsm[lane * (kTB + 1) + q] -= lij * dsm[q * (kTB + 1) + j];
-                }
-                __syncwarp();
-            }
         }
         __syncthreads();
-        if (fail) {
-            if (tid == 0) ok[c] = 0;
+        if (fail) {  // the same in every CTA of the cluster: they factor the same tile
+            if (crank == 0 && tid == 0) ok[c] = 0;
             return;
         }
-        for (int e = tid; e < kw * kw; e += kInvThreads) {
-            const int r = e / kw, q = e % kw;
-            if (q <= r) L[(long)(k0 + r) * N + k0 + q] = dsm[r * (kTB + 1) + q];
-        }
-        // panel rows below: x L_kk^T = a, staged in big[(i - k0 - kw) * (kTB + 1) + q]
-        const int m0 = k0 + kw, m = N - m0;
+        if (crank == 0)
+            for (int e = tid; e < kw * kw; e += kInvThreads) {
+                const int r = e / kw, q = e % kw;
+                Y[(long)(k0 + r) * ld + k0 + q] = inv[r * kTileLd + q];
+            }
+        // panel rows x = a L_kk^{-T}, in place; this CTA's rows to L^T
         for (int ri = tid; ri < m; ri += kInvThreads) {
-            const long i = m0 + ri;
-            T x[kTB];
+            T a[kTB];
+#pragma unroll
+            for (int q = 0; q < kTB; ++q) a[q] = buf[q * kPanLd + ri];
+            const bool mine = (ri >> 5) % csize == crank;
 #pragma unroll
             for (int q = 0; q < kTB; ++q) {
-                if (q < kw) {
-                    T a = L[i * N + k0 + q];
-                    for (int t = 0; t < q; ++t) a -= x[t] * dsm[q * (kTB + 1) + t];
-                    x[q] = a / dsm[q * (kTB + 1) + q];
-                    big[ri * (kTB + 1) + q] = x[q];
-                    L[i * N + k0 + q] = x[q];
+                T x = 0;
+#pragma unroll
+                for (int t = 0; t <= q; t += 4) {  // the inverse is zero right of its diagonal
+                    const Vec4<T> w = lds4(inv + q * kTileLd + t);
+                    x += a[t] * w.x + a[t + 1] * w.y + a[t + 2] * w.z + a[t + 3] * w.w;
                 }
+                buf[q * kPanLd + ri] = x;
+                if (mine && q < kw) L[(long)(k0 + q) * ld + m0 + ri] = x;
             }
         }
         __syncthreads();
-        // trailing lower triangle: A[i][j] -= panel_i . panel_j
-        for (int ri = warp; ri < m; ri += nw) {
-            const T* pi = big + ri * (kTB + 1);
-            T* Ai = L + (long)(m0 + ri) * N + m0;
-            for (int rj = lane; rj <= ri; rj += 32) {
-                const T* pj = big + rj * (kTB + 1);
-                T acc = 0;
+        // trailing lower triangle, 64x64 tiles: A[i][j] -= panel_i . panel_j
+        const int tx = tid & 15, ty = tid >> 4;
+        for (int e = crank; e < mt * (mt + 1) / 2; e += csize) {
+            int ti = 0;
+            while ((ti + 1) * (ti + 2) / 2 <= e) ++ti;
+            const int tj = e - ti * (ti + 1) / 2;
+            const int ri = 64 * ti + 4 * ty, rj = 64 * tj + 4 * tx;
+            T acc[4][4] = {};
 #pragma unroll 8
-                for (int q = 0; q < kw; ++q) acc += pi[q] * pj[q];
-                Ai[rj] -= acc;
-            }
-        }
-        __syncthreads();
-    }
-    // ---- Y = L^{-1}, block row by block row
-    for (int i0 = 0; i0 < N; i0 += kTB) {
-        const int iw = min(kTB, N - i0);
-        const int ncol = i0 + iw;
-        // rows i0..i0+iw of L (columns < i0) and the diagonal tile
-        for (int e = tid; e < iw * ncol; e += kInvThreads) {
-            const int r = e / ncol, k = e % ncol;
-            const T v = L[(long)(i0 + r) * N + k];
-            if (k < i0) big[r * (kNMax + 1) + k] = v;
-            else dsm[r * (kTB + 1) + (k - i0)] = v;
-        }
-        __syncthreads();
-        for (int col = tid; col < ncol; col += kInvThreads) {
-            T acc[kTB];
+            for (int q = 0; q < kTB; ++q) outer4(acc, lds4(buf + q * kPanLd + ri), lds4(buf + q * kPanLd + rj));
+            if (rj < m)
 #pragma unroll
-            for (int r = 0; r < kTB; ++r) acc[r] = T(0);
-            for (int k = col; k < i0; ++k) {
-                const T ykc = Y[(long)k * N + col];
-#pragma unroll
-                for (int r = 0; r < kTB; ++r) acc[r] += big[r * (kNMax + 1) + k] * ykc;
-            }
-#pragma unroll
-            for (int r = 0; r < kTB; ++r) {
-                if (r < iw) {
-                    T v = (col == i0 + r ? T(1) : T(0)) - acc[r];
-                    for (int t = 0; t < r; ++t) v -= dsm[r * (kTB + 1) + t] * acc[t];
-                    v /= dsm[r * (kTB + 1) + r];
-                    acc[r] = v;  // acc[r] now holds y(i0 + r, col)
-                    Y[(long)(i0 + r) * N + col] = col <= i0 + r ? v : T(0);
+                for (int i = 0; i < 4; ++i) {
+                    if (ri + i >= m) continue;
+                    T* p = L + (long)(m0 + ri + i) * ld + m0 + rj;
+                    Vec4<T> v = ldcg4(p);
+                    v.x -= acc[i][0]; v.y -= acc[i][1]; v.z -= acc[i][2]; v.w -= acc[i][3];
+                    st4(p, v);
                 }
-            }
         }
-        // columns right of the tile stay zero (Y is lower triangular)
-        for (int e = tid; e < iw * (N - ncol); e += kInvThreads) {
-            const int r = e / (N - ncol), q = ncol + e % (N - ncol);
-            Y[(long)(i0 + r) * N + q] = T(0);
-        }
-        __syncthreads();
+        cl.sync();
     }
-    if (tid == 0) ok[c] = 1;
+    // ---- Y = L^{-1}, a 32-wide column of tiles at a time; the columns with the
+    // most rows go round first, then back (the cluster's shares even out)
+    const int nb = (N + kTB - 1) / kTB;
+    const int gq = tid >> 6, rx = tid & 7, ry = (tid >> 3) & 7;
+    for (int turn = 0; turn * csize < nb; ++turn) {
+        const int jb = turn * csize + ((turn & 1) ? csize - 1 - crank : crank);
+        if (jb >= nb) continue;
+        const int j0 = jb * kTB, jw = min(kTB, N - j0);
+        __syncthreads();
+        for (int e = tid; e < kTB * kTB; e += kInvThreads) {
+            const int r = e / kTB, q = e % kTB;
+            buf[e] = r < jw && q < jw ? __ldcg(Y + (long)(j0 + r) * ld + j0 + q) : T(0);
+        }
+        for (int i0 = j0 + kTB; i0 < N; i0 += kTB) {
+            const int iw = min(kTB, N - i0);
+            T acc[4][4] = {};
+            for (int k0 = j0; k0 < i0; k0 += 128) {
+                const int kn = min(128, i0 - k0);
+                __syncthreads();
+                for (int e = tid; e < kn * (kTB / 4); e += kInvThreads) {
+                    const int k = e / (kTB / 4), q = 4 * (e % (kTB / 4));
+                    Vec4<T> v = {T(0), T(0), T(0), T(0)};
+                    if (q < iw) v = ldcg4(L + (long)(k0 + k) * ld + i0 + q);
+                    if (q + 1 >= iw) v.y = T(0);
+                    if (q + 2 >= iw) v.z = T(0);
+                    if (q + 3 >= iw) v.w = T(0);
+                    st4(stage + k * kTB + q, v);
+                }
+                if (k0 == j0)
+                    for (int e = tid; e < kTB * kTB; e += kInvThreads) {
+                        const int r = e / kTB, q = e % kTB;
+                        inv[r * kTileLd + q] = r < iw && q < iw ? __ldcg(Y + (long)(i0 + r) * ld + i0 + q) : T(0);
+                    }
+                __syncthreads();
+#pragma unroll 4
+                for (int k = gq; k < kn; k += 4)
+                    outer4(acc, lds4(stage + k * kTB + 4 * ry), lds4(buf + (k0 - j0 + k) * kTB + 4 * rx));
+            }
+            __syncthreads();
+#pragma unroll
+            for (int i = 0; i < 4; ++i)
+                st4(stage + gq * kTB * kTB + (4 * ry + i) * kTB + 4 * rx, Vec4<T>{acc[i][0], acc[i][1], acc[i][2], acc[i][3]});
+            __syncthreads();
+            for (int e = tid; e < kTB * kTB; e += kInvThreads)
+                R[(e / kTB) * kTileLd + e % kTB] =
+                    -((stage[e] + stage[kTB * kTB + e]) + (stage[2 * kTB * kTB + e] + stage[3 * kTB * kTB + e]));
+            __syncthreads();
+            const int r = tid >> 3, q = 4 * (tid & 7);
+            Vec4<T> y = {T(0), T(0), T(0), T(0)};
+            for (int t = 0; t <= r; ++t) {
+                const T w = inv[r * kTileLd + t];
+                const Vec4<T> v = lds4(R + t * kTileLd + q);
+                y.x += w * v.x; y.y += w * v.y; y.z += w * v.z; y.w += w * v.w;
+            }
+            st4(buf + (i0 - j0 + r) * kTB + q, y);
+            if (r < iw) st4(Y + (long)(i0 + r) * ld + j0 + q, y);  // jw = 32 here
+        }
+    }
+    if (crank == 0 && tid == 0) ok[c] = 1;
 }
 
 struct DSU {
@@ -214,6 +338,44 @@ struct DSU {
         if (a != b) p[a < b ? b : a] = a < b ? a : b;
     }
 };
+
+template <class T>
+int factor_blocks(Arena& A, Work& W, const int* list, int nbig, int nfew, cudaStream_t s) {
+    Work::Clusters& cl = W.cl;
+    T* K = W[W_CL_DENSE].as<T>();
+    T* Y = K + cl.dense;
+    IDP_CUDA_TRY(cudaMemsetAsync(K, 0, sizeof(T) * (size_t)cl.dense, s));
+    (::idp::count_launch(), k_cl_gather<T><<<dim3(cl.n, 4), 256, 0, s>>>(
+                                cl.n, cl.off, cl.vert, cl.vcl, cl.vloc, cl.doff, A.rowptr, A.colidx,
+                                W[W_BSR_VAL].as<T>(), W[W_TAIL_ROWPTR].as<int>(), W[W_TAIL_COL].as<int>(),
+                                W[W_TAIL_VAL].as<T>(), A.dbc, K));
+    static std::atomic<bool> attr{false};  // one per instantiation
+    if (!attr.load()) {
+        IDP_CUDA_TRY(cudaFuncSetAttribute(k_cl_invert<T>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                          (int)invert_smem_bytes<T>()));
+        attr.store(true);
+    }
+    for (int part = 0; part < 2; ++part) {
+        const int n = part ? nfew : nbig, cs = part ? 1 : kInvCluster;
+        if (!n) continue;
+        cudaLaunchConfig_t cfg = {};
+        cfg.gridDim = dim3(n * cs);
+        cfg.blockDim = dim3(kInvThreads);
+        cfg.dynamicSmemBytes = invert_smem_bytes<T>();
+        cfg.stream = s;
+        cudaLaunchAttribute at[1];
+        at[0].id = cudaLaunchAttributeClusterDimension;
+        at[0].val.clusterDim.x = cs;
+        at[0].val.clusterDim.y = 1;
+        at[0].val.clusterDim.z = 1;
+        cfg.attrs = at;
+        cfg.numAttrs = 1;
+        ::idp::count_launch();
+        IDP_CUDA_TRY(cudaLaunchKernelEx(&cfg, k_cl_invert<T>, list + (part ? nbig : 0), (const int*)cl.off,
+                                        (const long long*)cl.doff, K, Y, (int*)cl.ok));
+    }
+    return cudaGetLastError() == cudaSuccess ? IDP_OK : IDP_ERR_CUDA;
+}
 
 }  // namespace
 
@@ -335,6 +497,7 @@ int build_contact_clusters(Arena& A, Work& W, const ContactSet& cs, bool fp64, c
     std::stable_sort(order.begin(), order.end(), [&](int a, int b) { return vinst_h[a] < vinst_h[b]; });
     std::vector<int> off(1, 0), vert, ioff(nI + 1, 0), vcl(A.V, -1), vloc(A.V, 0);
     std::vector<long long> doff(1, 0);
+    std::vector<int> big, few;  // blocks factored by a cluster, by one CTA
     int maxn = 0;
     for (int bi = 0; bi < (int)order.size(); ++bi) {
         auto& blk = blocks[order[bi]];
@@ -347,8 +510,9 @@ int build_contact_clusters(Arena& A, Work& W, const ContactSet& cs, bool fp64, c
         }
         vert.insert(vert.end(), vs.begin(), vs.end());
         off.push_back((int)vert.size());
-        long long N = 3LL * (long long)vs.size();
-        doff.push_back(doff.back() + N * N);
+        const int N = 3 * (int)vs.size();
+        doff.push_back(doff.back() + (long long)N * block_ld(N));
+        (N > kInvClusterRows ? big : few).push_back(bi);
         ioff[vinst_h[order[bi]] + 1]++;
         maxn = std::max(maxn, (int)vs.size());
     }
@@ -358,8 +522,8 @@ int build_contact_clusters(Arena& A, Work& W, const ContactSet& cs, bool fp64, c
     cl.nvert = (long)vert.size();
     cl.dense = doff.back();
     cl.max_n = maxn;
-    // int buffer layout: vcl[V] vloc[V] ioff[nI+1] off[ncl+1] vert[nvert] ok[ncl] | doff (8-byte aligned)
-    size_t ints = 2 * (size_t)A.V + (nI + 1) + (ncl + 1) + vert.size() + ncl + 8;
+    // int buffer layout: vcl[V] vloc[V] ioff[nI+1] off[ncl+1] vert[nvert] ok[ncl] list[ncl] | doff (8-byte aligned)
+    size_t ints = 2 * (size_t)A.V + (nI + 1) + (ncl + 1) + vert.size() + 2 * ncl + 8;
     size_t bytes = sizeof(int) * ints + sizeof(long long) * (ncl + 2) + 64;
     if (W[W_CL_INT].ensure(bytes)) return IDP_ERR_CUDA;
     base = W[W_CL_INT].as<int>();
@@ -370,7 +534,8 @@ int build_contact_clusters(Arena& A, Work& W, const ContactSet& cs, bool fp64, c
     cl.vert = cl.off + (ncl + 1);
     int* okp = cl.vert + vert.size();
     cl.ok = okp;
-    size_t used = (size_t)(okp + ncl - base);
+    int* list = okp + ncl;  // the cluster-factored blocks, then the others
+    size_t used = (size_t)(list + ncl - base);
     used = (used + 1) / 2 * 2;
     cl.doff = reinterpret_cast<long long*>(base + used);
     IDP_CUDA_TRY(cudaMemcpyAsync(cl.vcl, vcl.data(), sizeof(int) * A.V, cudaMemcpyHostToDevice, s));
@@ -384,38 +549,14 @@ int build_contact_clusters(Arena& A, Work& W, const ContactSet& cs, bool fp64, c
         IDP_CUDA_TRY(cudaStreamSynchronize(s));
         return IDP_OK;
     }
+    std::vector<int> order_l(big);
+    order_l.insert(order_l.end(), few.begin(), few.end());
+    IDP_CUDA_TRY(cudaMemcpyAsync(list, order_l.data(), sizeof(int) * ncl, cudaMemcpyHostToDevice, s));
+    // K | Y | t = Y r of the PCG's block applies
     size_t el = fp64 ? sizeof(double) : sizeof(float);
-    if (W[W_CL_DENSE].ensure(el * 2 * (size_t)(cl.dense + 1))) return IDP_ERR_CUDA;
-    const int* trp = W[W_TAIL_ROWPTR].as<int>();
-    const int* tcol = W[W_TAIL_COL].as<int>();
-    if (fp64) {
-        double* K = W[W_CL_DENSE].as<double>();
-        (::idp::count_launch(), k_cl_gather<double><<<ncl, 256, 0, s>>>(ncl, cl.off, cl.vert, cl.vcl, cl.vloc, cl.doff, A.rowptr, A.colidx,
-                                                  W[W_BSR_VAL].as<double>(), trp, tcol, W[W_TAIL_VAL].as<double>(),
-                                                  A.dbc, K));
-        static std::atomic<bool> attr_d{false};
-        if (!attr_d.load()) {
-            IDP_CUDA_TRY(cudaFuncSetAttribute(k_cl_invert<double>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                              (int)invert_smem_bytes<double>()));
-            attr_d.store(true);
-        }
-        (::idp::count_launch(), k_cl_invert<double><<<ncl, kInvThreads, invert_smem_bytes<double>(), s>>>(
-                                    ncl, cl.off, cl.doff, K, K + cl.dense, okp));
-    } else {
-        float* K = W[W_CL_DENSE].as<float>();
-        (::idp::count_launch(), k_cl_gather<float><<<ncl, 256, 0, s>>>(ncl, cl.off, cl.vert, cl.vcl, cl.vloc, cl.doff, A.rowptr, A.colidx,
-                                                 W[W_BSR_VAL].as<float>(), trp, tcol, W[W_TAIL_VAL].as<float>(), A.dbc,
-                                                 K));
-        static std::atomic<bool> attr_f{false};
-        if (!attr_f.load()) {
-            IDP_CUDA_TRY(cudaFuncSetAttribute(k_cl_invert<float>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                              (int)invert_smem_bytes<float>()));
-            attr_f.store(true);
-        }
-        (::idp::count_launch(), k_cl_invert<float><<<ncl, kInvThreads, invert_smem_bytes<float>(), s>>>(
-                                    ncl, cl.off, cl.doff, K, K + cl.dense, okp));
-    }
-    return cudaGetLastError() == cudaSuccess ? IDP_OK : IDP_ERR_CUDA;
+    if (W[W_CL_DENSE].ensure(el * (2 * (size_t)cl.dense + 3 * (size_t)cl.nvert + 16))) return IDP_ERR_CUDA;
+    return fp64 ? factor_blocks<double>(A, W, list, (int)big.size(), (int)few.size(), s)
+                : factor_blocks<float>(A, W, list, (int)big.size(), (int)few.size(), s);
 }
 
 }  // namespace idp

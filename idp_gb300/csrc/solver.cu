@@ -403,42 +403,33 @@ struct ClusterPC {
     const int* vert;       // block vertices
     const long long* doff; // dense offsets
     const int* ok;         // factorisation succeeded
-    const T* Kinv;         // dense inverses
+    const T* Kinv;         // inverse factors Y (row stride: 3n rounded up to 4)
+    T* t;                  // Y r of every block (3 values per block vertex)
 };
 
-// z = M^{-1} r on the rows of the blocks owned by this CTA (blocks c of the
-// instance with c % csize == crank): z = Y^T (Y r) with Y = L^{-1} the inverse
-// Cholesky factor of the block, or 3x3 inverses when the factorisation failed.
-// rc must hold 6 * kClusterCap values (r of the block, then Y r).
+// z = M^{-1} r on the rows of the instance's blocks, z = Y^T (Y r) with Y =
+// L^{-1} the inverse Cholesky factor of a block (3x3 inverses when the
+// factorisation failed), in two passes with a barrier of the instance's CTAs
+// between them. Every block is shared out over all of them (a block of 192
+// vertices is 1.3 MB of Y read twice: on one CTA it alone took longer than the
+// rest of an iteration).
+// Pass 1: t = Y r, rows of Y dealt in pairs to the warps of all CTAs (every
+// load of both rows issued before the sums). rc: N values of shared memory.
 template <class T>
-__device__ void apply_blocks(const ClusterPC<T>& pc, int inst, int crank, int csize, const T* __restrict__ dinv,
-                             const unsigned char* __restrict__ dbc, const T* __restrict__ r, T* __restrict__ z,
-                             T* __restrict__ p_init, T* rc) {
-    T* tc = rc + 3 * kClusterCap;  // second half of the caller's shared buffer
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
-    for (int c = pc.ioff[inst] + crank; c < pc.ioff[inst + 1]; c += csize) {
-        const int o = pc.off[c], n = pc.off[c + 1] - o, N = 3 * n;
-        if (!pc.ok[c]) {
-            for (int li = threadIdx.x; li < n; li += blockDim.x) {
-                int v = pc.vert[o + li];
-                T rv[3] = {__ldcg(r + 3 * v), __ldcg(r + 3 * v + 1), __ldcg(r + 3 * v + 2)}, zv[3];
-                precond(v, dinv, dbc, rv, zv);
-                for (int d = 0; d < 3; ++d) {
-                    z[3 * v + d] = zv[d];
-                    if (p_init) p_init[3 * v + d] = zv[d];
-                }
-            }
-            continue;
-        }
+__device__ void apply_blocks_1(const ClusterPC<T>& pc, int inst, int crank, int csize, const T* __restrict__ r, T* rc) {
+    const int lane = threadIdx.x & 31, nw = blockDim.x >> 5;
+    const int gw = (threadIdx.x >> 5) * csize + crank, gn = nw * csize;
+    for (int c = pc.ioff[inst]; c < pc.ioff[inst + 1]; ++c) {
+        const int o = pc.off[c], N = 3 * (pc.off[c + 1] - o), ld = (N + 3) & ~3;
+        if (!pc.ok[c] || 2 * crank >= N) continue;
+        __syncthreads();
         for (int a = threadIdx.x; a < N; a += blockDim.x) rc[a] = __ldcg(r + 3 * pc.vert[o + a / 3] + a % 3);
         __syncthreads();
         const T* Yc = pc.Kinv + pc.doff[c];
-        // t = Y r (Y lower triangular; rows by warps, two rows per warp, every
-        // load of both rows issued before the sums); t overwrites tc
         constexpr int kPer = (3 * kClusterCap + 31) / 32;
-        for (int a = 2 * warp; a < N; a += 2 * nw) {
-            const T* r0 = Yc + (long)a * N;
-            const T* r1 = r0 + N;
+        for (int a = 2 * gw; a < N; a += 2 * gn) {
+            const T* r0 = Yc + (long)a * ld;
+            const T* r1 = r0 + ld;
             const bool two = a + 1 < N;
             T acc0 = 0, acc1 = 0;
 #pragma unroll
@@ -455,23 +446,57 @@ __device__ void apply_blocks(const ClusterPC<T>& pc, int inst, int crank, int cs
                 acc1 += __shfl_down_sync(0xffffffffu, acc1, ofs);
             }
             if (lane == 0) {
-                tc[a] = acc0;
-                if (two) tc[a + 1] = acc1;
+                pc.t[3 * (long)o + a] = acc0;
+                if (two) pc.t[3 * (long)o + a + 1] = acc1;
             }
         }
-        __syncthreads();
-        // z = Y^T t: column b of Y against t, threads over b (row k of Y is
-        // read coalesced)
-        for (int b = threadIdx.x; b < N; b += blockDim.x) {
-            T acc = 0;
-#pragma unroll 4
-            for (int k = b; k < N; ++k) acc += __ldg(Yc + (long)k * N + b) * tc[k];
-            const int v = pc.vert[o + b / 3];
-            const T zz = dbc[v] ? T(0) : acc;
-            z[3 * v + b % 3] = zz;
-            if (p_init) p_init[3 * v + b % 3] = zz;
+    }
+}
+
+// Pass 2: z = Y^T t, 32 columns of Y at a time dealt to the CTAs, their rows
+// to the CTA's warps (coalesced), partial sums added in warp order. tc: 32
+// values per warp of shared memory. The vertices of a block without a factor
+// are dealt to the CTAs.
+template <class T>
+__device__ void apply_blocks_2(const ClusterPC<T>& pc, int inst, int crank, int csize, const T* __restrict__ dinv,
+                               const unsigned char* __restrict__ dbc, const T* __restrict__ r, T* __restrict__ z,
+                               T* __restrict__ p_init, T* tc) {
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
+    for (int c = pc.ioff[inst]; c < pc.ioff[inst + 1]; ++c) {
+        const int o = pc.off[c], n = pc.off[c + 1] - o, N = 3 * n, ld = (N + 3) & ~3;
+        if (!pc.ok[c]) {
+            for (int li = threadIdx.x * csize + crank; li < n; li += blockDim.x * csize) {
+                const int v = pc.vert[o + li];
+                T rv[3] = {__ldcg(r + 3 * v), __ldcg(r + 3 * v + 1), __ldcg(r + 3 * v + 2)}, zv[3];
+                precond(v, dinv, dbc, rv, zv);
+                for (int d = 0; d < 3; ++d) {
+                    z[3 * v + d] = zv[d];
+                    if (p_init) p_init[3 * v + d] = zv[d];
+                }
+            }
+            continue;
         }
-        __syncthreads();
+        const T* Yc = pc.Kinv + pc.doff[c];
+        const T* tv = pc.t + 3 * (long)o;
+        for (int g = crank; 32 * g < N; g += csize) {
+            const int b = 32 * g + lane;
+            T acc = 0;
+            if (b < N)
+#pragma unroll 4
+                for (int k = 32 * g + warp; k < N; k += nw)
+                    if (k >= b) acc += __ldg(Yc + (long)k * ld + b) * __ldcg(tv + k);
+            __syncthreads();  // the previous group's sums are read
+            tc[32 * warp + lane] = acc;
+            __syncthreads();
+            if (warp == 0 && b < N) {
+                T s = tc[lane];
+                for (int w = 1; w < nw; ++w) s += tc[32 * w + lane];
+                const int v = pc.vert[o + b / 3];
+                const T zz = dbc[v] ? T(0) : s;
+                z[3 * v + b % 3] = zz;
+                if (p_init) p_init[3 * v + b % 3] = zz;
+            }
+        }
     }
 }
 
@@ -485,7 +510,7 @@ __global__ void __launch_bounds__(CL_THREADS) k_pcg_cluster(
     int* __restrict__ iters_out) {
     __shared__ T wsh[2 * (CL_THREADS / 32)];
     __shared__ T slot[4][2];
-    __shared__ T rc[6 * kClusterCap];
+    __shared__ T rc[3 * kClusterCap];  // r of one block; or 32 partial sums per warp
     cg::cluster_group cl = cg::this_cluster();
     const int csize = (int)cl.num_blocks(), crank = (int)cl.block_rank();
     const int inst = inst_list[blockIdx.x / csize];
@@ -514,7 +539,9 @@ __global__ void __launch_bounds__(CL_THREADS) k_pcg_cluster(
     }
     if (has_blocks) {
         cl.sync();
-        apply_blocks(pc, inst, crank, csize, dinv, dbc, r, z, p, rc);
+        apply_blocks_1(pc, inst, crank, csize, r, rc);
+        cl.sync();
+        apply_blocks_2(pc, inst, crank, csize, dinv, dbc, r, z, p, rc);
         cl.sync();
     }
     T rz_l = 0;
@@ -561,7 +588,9 @@ __global__ void __launch_bounds__(CL_THREADS) k_pcg_cluster(
             }
             if (has_blocks) {
                 cl.sync();
-                apply_blocks(pc, inst, crank, csize, dinv, dbc, r, z, (T*)nullptr, rc);
+                apply_blocks_1(pc, inst, crank, csize, r, rc);
+                cl.sync();
+                apply_blocks_2(pc, inst, crank, csize, dinv, dbc, r, z, (T*)nullptr, rc);
                 cl.sync();
                 for (int v = v0 + threadIdx.x; v < v1; v += blockDim.x)
                     for (int d = 0; d < 3; ++d) rzn_l += r[3 * v + d] * __ldcg(z + 3 * v + d);
@@ -723,7 +752,7 @@ __global__ void __launch_bounds__(GP_THREADS, 3) k_pcg_grid(
     __shared__ T wsh[2 * (GP_THREADS / 32)];
     __shared__ T sh_t[kRed];
     __shared__ int sh_i[2];
-    __shared__ T rc[6 * kClusterCap];
+    __shared__ T rc[3 * kClusterCap];
     const GridCta me = plan[blockIdx.x];
     const int inst = me.inst, v0 = me.v0, v1 = me.v1, c0 = me.c0, nc = me.nc, rank = blockIdx.x - me.c0;
     const int nv = v1 - v0;
@@ -1043,7 +1072,9 @@ __global__ void __launch_bounds__(GP_THREADS, 3) k_pcg_grid(
     }
     if (has_blocks) {
         if (!barrier()) return;
-        apply_blocks(pc, inst, rank, nc, dinv, dbc, r, z, (T*)nullptr, rc);
+        apply_blocks_1(pc, inst, rank, nc, r, rc);
+        if (!barrier()) return;
+        apply_blocks_2(pc, inst, rank, nc, dinv, dbc, r, z, (T*)nullptr, rc);
         if (!barrier()) return;
         for (int lv = threadIdx.x; lv < nv; lv += GP_THREADS)
             for (int d = 0; d < 3; ++d) rz_l += r[3 * (v0 + lv) + d] * __ldcg(z + 3 * (v0 + lv) + d);
@@ -1151,7 +1182,9 @@ __global__ void __launch_bounds__(GP_THREADS, 3) k_pcg_grid(
             }
             if (has_blocks) {
                 if (!barrier()) return;
-                apply_blocks(pc, inst, rank, nc, dinv, dbc, r, z, (T*)nullptr, rc);
+                apply_blocks_1(pc, inst, rank, nc, r, rc);
+                if (!barrier()) return;
+                apply_blocks_2(pc, inst, rank, nc, dinv, dbc, r, z, (T*)nullptr, rc);
                 if (!barrier()) return;
                 for (int lv = threadIdx.x; lv < nv; lv += GP_THREADS)
                     for (int d = 0; d < 3; ++d) rzn_l += r[3 * (v0 + lv) + d] * __ldcg(z + 3 * (v0 + lv) + d);
@@ -1303,6 +1336,7 @@ static int pcg_inner(Arena& A, Work& W, const double* b, double rel_tol, int max
         pcb.doff = W.cl.doff;
         pcb.ok = W.cl.ok;
         pcb.Kinv = W.cl.n > 0 ? W[W_CL_DENSE].as<T>() + W.cl.dense : nullptr;
+        pcb.t = W.cl.n > 0 ? W[W_CL_DENSE].as<T>() + 2 * W.cl.dense : nullptr;
         W.timer.start(PhaseTimer::PCG, s);
         int base = 0;
         for (int k = 0; k < 5; ++k) {
@@ -1415,6 +1449,7 @@ static int pcg_inner(Arena& A, Work& W, const double* b, double rel_tol, int max
     pcb.doff = W.cl.doff;
     pcb.ok = W.cl.ok;
     pcb.Kinv = W.cl.n > 0 ? W[W_CL_DENSE].as<T>() + W.cl.dense : nullptr;
+    pcb.t = W.cl.n > 0 ? W[W_CL_DENSE].as<T>() + 2 * W.cl.dense : nullptr;
     W.timer.start(PhaseTimer::PCG, s);
     IDP_CUDA_TRY(cudaMemsetAsync(d_err, 0, sizeof(int), s));
     if (d_prof && !W.grid_prof_init) {
