@@ -41,14 +41,9 @@ __device__ bool chol_pd(const T* A, int n) {
 // itself (FP32 sums compensated, so that a zero eigenvalue beside a large one
 // does not come out as its rounding), and the projection is a sum of outer
 // products that takes the off-diagonals the sweeps left into account: a sum of
-// squares stays PSD to rounding, which A minus its negative part does not. In
-// FP32 eigenvalues are floored at eps / 4 of the largest: storing the matrix
-// rounds them by more than that either way, and the ones pushed below zero cost
-// definiteness under stiff contact (48 steps of folded bars, 40 Newton
-// iterations each: 60 thousand PCG iterations and 20 FP64 re-solves; 103
-// thousand and 54 without the floor, 63 thousand and 30 with the earlier
-// sweeps). A floor of eps is too much: its stiffness slows stiff contact until
-// the step-length test stops Newton early (energies 0.4 to 2 % too high).
+// squares stays PSD to rounding, which A minus its negative part does not. (No
+// floor under the eigenvalues: one of eps / 4 of the largest already leads mixed
+// solves with stiff contact to other minima than FP64 takes in 5 of 14 runs.)
 // Only columns move: no shared memory, no row updates and no separate
 // eigenvector matrix in the sweeps, which are bound by instruction issue
 // (FP32) or the FP64 pipe. 22,000 random 12x12 matrices: FP32 0.17 ms (3.4 ms
@@ -149,13 +144,7 @@ __device__ void psd_jacobi(PsdScratch<T>& sc, int j, bool mine) {
         y[i] = act ? av + ae : T(0);
         lam += g[i] * y[i];
     }
-    T floor = T(0);
-    if (sizeof(T) == 4) {
-        T most = act ? fabs(lam) : T(0);
-        for (int o = 8; o > 0; o >>= 1) most = fmax(most, __shfl_xor_sync(full, most, o));
-        floor = T(0.25 * 1.1920929e-7) * most;
-    }
-    const T sl = act && lam > floor ? sqrt(lam) : T(0);  // 0: not among the kept ones
+    const T sl = act && lam > T(0) ? sqrt(lam) : T(0);  // 0: not among the kept ones
     if (act)
 #pragma unroll
         for (int i = 0; i < N; ++i) sc.V[j * kPsdDim + i] = g[i];
@@ -164,7 +153,7 @@ __device__ void psd_jacobi(PsdScratch<T>& sc, int j, bool mine) {
     // off-diagonals m, what makes V^T (sum_j h_j h_j^T) V the projection of
     // lam + m (bounded by sqrt |m|, so that its square stays below m)
 #pragma unroll
-    for (int i = 0; i < N; ++i) g[i] *= sl > T(0) ? sl : sqrt(floor);
+    for (int i = 0; i < N; ++i) g[i] *= sl;
     for (int i = 0; i < N; ++i) {
         const T li = __shfl_sync(full, lam, base | i), sli = __shfl_sync(full, sl, base | i);
         T m = 0, v[N];
