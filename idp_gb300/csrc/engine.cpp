@@ -507,6 +507,8 @@ idp_ctx* idp_create(const idp_params* p, int* status) {
         return nullptr;
     }
     c->W.local_deg = c->P.pcg_local_degree;
+    c->W.sell_vper = c->P.pcg_grid_cta_vertices;
+    c->W.sell_f64 = c->P.mode == IDP_MODE_FP64;
     c->W.cl_cap = c->P.contact_block_vertices > 0 ? std::max(2, std::min(c->P.contact_block_vertices, kClusterCap))
                                                   : kClusterCap;
     int prio_lo = 0, prio_hi = 0;
@@ -561,6 +563,7 @@ int idp_reset(idp_ctx* c) {
     c->snap_kappa.clear();
     c->W.stats = idp_stats{};
     c->W.dense_ready[0] = c->W.dense_ready[1] = false;
+    c->W.sell.ready = false;
     return IDP_OK;
 }
 
@@ -938,6 +941,7 @@ int idp_commit(idp_ctx* c) {
     Arena& A = c->A;
     const int nI = (int)c->inst.size();
     A.nI = nI;
+    c->W.sell.ready = false;
     A.v_off.assign(nI + 1, 0);
     A.t_off.assign(nI + 1, 0);
     A.f_off.assign(nI + 1, 0);

@@ -258,8 +258,16 @@ enum WorkSlot {
     W_BH, W_BG, W_GENT_KEY, W_GENT_VAL, W_GENT_KEY2, W_GENT_VAL2, W_GENT_HEAD,
     W_TAIL_ROWPTR, W_TAIL_COL, W_TAIL_VAL, W_TAIL_KEYS,
     W_BSR_VAL, W_DIAG_INV, W_PCG_VEC, W_PCG_GRID, W_SPAN, W_CBASE, W_DENSE0, W_DENSE1, W_PCG_VEC64, W_CCD_TMP, W_CCD_ALPHA, W_MISC, W_MISC2,
-    W_CL_INT, W_CL_DENSE, W_CL_HOSTCONS, W_PSD, W_SHELL_GRAD, W_CCD_VOX, W_SHELL_PSD,
+    W_CL_INT, W_CL_DENSE, W_CL_HOSTCONS, W_PSD, W_SELL_CTA, W_SELL_SLOT, W_SELL_HALO, W_SELL_XCH, W_SELL_LIST, W_SHELL_GRAD, W_CCD_VOX, W_SHELL_PSD,
     W_NUM
+};
+// one CTA of the register-resident PCG (pcg_sell.cu): rows [v0, v0 + nv) of an
+// instance, CTA `rank` of its nc (the first is plan CTA c0)
+struct SellCta {
+    int inst, v0, nv, c0, nc, rank;
+    int slice0;       // first slice of its rows
+    int slot0, nsr;   // first slot row, slot rows (-1: did not fit)
+    int halo0, nh;    // halo list
 };
 struct Work {
     DBuf b[W_NUM];
@@ -269,6 +277,21 @@ struct Work {
     double* tol_inst = nullptr;              // per-instance PCG tolerance (device)
     long grid_min_v = 16384;                 // grid-wide PCG above this many vertices
     long grid_vper = 112;                    // vertices per CTA in the grid-wide PCG
+    long sell_vper = 0;                      // the same as the caller gave it (0: pcg_sell.cu's own rule)
+    bool sell_f64 = false;                   // its rule for FP64 contexts
+    // layout of pcg_sell.cu, made at the first solve after a commit
+    struct Sell {
+        bool ready = false;
+        int sms = 0;
+        std::vector<SellCta> cta;
+        std::vector<int> first;              // per instance: its first CTA, -1: left to the other kernels
+        SellCta* d_cta = nullptr;
+        int2* d_slice = nullptr;
+        unsigned short *d_prow = nullptr, *d_col = nullptr;
+        int *d_src = nullptr, *d_halo = nullptr;
+        size_t xch_bytes = 0;                // exchange words cleared so far
+        unsigned int tag = 0;                // first unused tag
+    } sell;
     int local_deg = 0;                       // degree of the grid PCG's CTA-local polynomial preconditioner
     int cl_cap = kClusterCap;                // vertices per dense contact block
     long long accd_maxit = 0;                // diagnostics (IDP_PROFILE)
@@ -285,6 +308,7 @@ struct Work {
         long long* doff = nullptr; // n+1: dense offsets
         int* ioff = nullptr;       // nI+1: clusters of each instance (clusters sorted by instance)
         int* ok = nullptr;         // n: factorisation succeeded
+        std::vector<int> ioff_h;   // host copy of ioff
         int max_n = 0;
     } cl;
     long cand_cap_pt = 0, cand_cap_ee = 0;   // candidate list capacities (grown on overflow)
@@ -397,6 +421,11 @@ int ccd_stepsize(Arena& A, Work& W, const double* X, const double* dir, double* 
 // solver.cu
 int assemble(Arena& A, Work& W, const ContactSet& cs, bool fp64, cudaStream_t s);
 int normal_flow_velocity(Arena& A, int sel, double step, double h, double* vel, cudaStream_t s);
+// pcg_sell.cu: PCG of instances without contact blocks
+int sell_plan(Arena& A, Work& W, cudaStream_t s);
+template <class T>
+int sell_solve(Arena& A, Work& W, const std::vector<int>& which, const double* b, T* x, double rel_tol, int max_iters,
+               int* d_iters, int* d_err, cudaStream_t s);
 int pcg_solve(Arena& A, Work& W, const ContactSet& cs, bool fp64, const double* rhs, double* sol,
               double rel_tol, int max_iters, std::vector<int>& iters_out, std::vector<double>& relres_out,
               cudaStream_t s, const double* tol_host = nullptr);

@@ -385,6 +385,7 @@ int build_contact_clusters(Arena& A, Work& W, const ContactSet& cs, bool fp64, c
     cl.nvert = 0;
     const long C = cs.C;
     const int nI = A.nI;
+    cl.ioff_h.assign(nI + 1, 0);
     if (W[W_CL_INT].ensure(sizeof(int) * (2 * A.V + 8 * (nI + 1) + 64))) return IDP_ERR_CUDA;
     int* base = W[W_CL_INT].as<int>();
     if (C <= 0) {
@@ -517,6 +518,7 @@ int build_contact_clusters(Arena& A, Work& W, const ContactSet& cs, bool fp64, c
         maxn = std::max(maxn, (int)vs.size());
     }
     for (int i = 0; i < nI; ++i) ioff[i + 1] += ioff[i];
+    cl.ioff_h = ioff;
     const int ncl = (int)order.size();
     cl.n = ncl;
     cl.nvert = (long)vert.size();

@@ -1301,10 +1301,24 @@ static int pcg_inner(Arena& A, Work& W, const double* b, double rel_tol, int max
     IDP_CUDA_TRY(cudaMemcpyAsync(act.data(), A.active, nI, cudaMemcpyDeviceToHost, s));
     IDP_CUDA_TRY(cudaStreamSynchronize(s));
     bool any_small = false, any_large = false;
+    // instances without contact blocks: pcg_sell.cu, unless they are too large
+    // for it or the CTA-local polynomial preconditioner is asked for
+    if (!W.sell.ready) {
+        const int rc = sell_plan(A, W, s);
+        if (rc) return rc;
+    }
+    std::vector<int> sells;
+    std::vector<unsigned char> by_sell(nI, 0);
     std::vector<int> by_size[5];  // cluster sizes 1, 2, 4, 8, 16
     for (int i = 0; i < nI; ++i) {
         if (!act[i]) continue;
         long vi = A.v_off[i + 1] - A.v_off[i];
+        const bool blocks = W.cl.ioff_h[i + 1] > W.cl.ioff_h[i];
+        if (!blocks && W.sell.first[i] >= 0 && (W.local_deg == 0 || vi <= W.grid_min_v)) {
+            sells.push_back(i);
+            by_sell[i] = 1;
+            continue;
+        }
         if (vi > W.grid_min_v) { large[i] = 1; any_large = true; continue; }
         small[i] = 1;
         any_small = true;
@@ -1319,6 +1333,37 @@ static int pcg_inner(Arena& A, Work& W, const double* b, double rel_tol, int max
     int* d_list = W[W_MISC2].as<int>();
     int* d_iters = d_list + nI + 32;
     iters.assign(nI, 0);
+    auto account = [&](const std::vector<unsigned char>& which) {
+        for (int i = 0; i < nI; ++i)
+            if (which[i]) {
+                W.stats.pcg_iters += iters[i];
+                if ((int)W.pcg_bytes_per_iter.size() == nI)
+                    W.stats.pcg_bytes += (double)iters[i] * W.pcg_bytes_per_iter[i] * (sizeof(T) / 4.0);
+            }
+    };
+    if (!sells.empty()) {
+        int* d_bad = d_iters + nI + 16;
+        IDP_CUDA_TRY(cudaMemsetAsync(d_bad, 0, sizeof(int), s));
+        W.timer.start(PhaseTimer::PCG, s);
+        const int rc = sell_solve<T>(A, W, sells, b, x, rel_tol, max_iters, d_iters, d_bad, s);
+        W.timer.stop(s);
+        if (rc) return rc;
+        std::vector<int> hit(nI + 17);
+        IDP_CUDA_TRY(cudaMemcpyAsync(hit.data(), d_iters, sizeof(int) * (nI + 17), cudaMemcpyDeviceToHost, s));
+        IDP_CUDA_TRY(cudaStreamSynchronize(s));
+        int most = 0;
+        for (int i : sells) most = std::max(most, iters[i] = hit[i]);
+        W.sell.tag += (unsigned int)most + 4;  // the tags this solve used
+        if (hit[nI + 16]) {  // a poll ran out (never expected): its tags are not reused
+            W.sell.xch_bytes = 0;
+            return IDP_ERR_CUDA;
+        }
+        account(by_sell);
+        if (!any_small && !any_large) {
+            *xout = x;
+            return IDP_OK;
+        }
+    }
     if (any_small) {
         std::vector<int> flat;
         for (int k = 0; k < 5; ++k) flat.insert(flat.end(), by_size[k].begin(), by_size[k].end());
@@ -1370,14 +1415,6 @@ static int pcg_inner(Arena& A, Work& W, const double* b, double rel_tol, int max
         for (int i = 0; i < nI; ++i)
             if (small[i]) iters[i] = hit[i];
     }
-    auto account = [&](const std::vector<unsigned char>& which) {
-        for (int i = 0; i < nI; ++i)
-            if (which[i]) {
-                W.stats.pcg_iters += iters[i];
-                if ((int)W.pcg_bytes_per_iter.size() == nI)
-                    W.stats.pcg_bytes += (double)iters[i] * W.pcg_bytes_per_iter[i] * (sizeof(T) / 4.0);
-            }
-    };
     account(small);
     if (!any_large) {
         *xout = x;

@@ -55,10 +55,16 @@ typedef struct idp_params {
     int pcg_max_iters;    /* PCG iteration cap per refinement sweep                 */
     double thickness;     /* IPC offset (`thickness` argument, IPC.h:53,757)        */
     int device;           /* CUDA device ordinal                                    */
-    int pcg_grid_min_vertices; /* instances above this many vertices solve with the
-                             grid-wide PCG (all SMs), the others with one thread-block
-                             cluster each; 0 = default (16384)                        */
-    int pcg_grid_cta_vertices; /* vertices per CTA in the grid-wide PCG; 0 = default (112) */
+    int pcg_grid_min_vertices; /* instances with contact constraints above this many
+                             vertices solve with the grid-wide PCG (all SMs), the
+                             others with one thread-block cluster each; 0 = default
+                             (16384). Instances without constraints solve with
+                             persistent CTAs (at most one per SM), whatever their
+                             size, up to 384 vertices per SM                         */
+    int pcg_grid_cta_vertices; /* vertices per CTA above pcg_grid_min_vertices (at
+                             least what one CTA per SM has to take); 0 = default:
+                             112 in the grid-wide PCG, 64 (FP64: 40) in the
+                             persistent CTAs                                          */
     int contact_block_vertices; /* largest group of contact-coupled vertices the
                              preconditioner inverts as one dense block (2..192);
                              0 = default (192)                                        */
