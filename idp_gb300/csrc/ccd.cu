@@ -20,6 +20,7 @@
 #include <algorithm>
 #include "engine.hpp"
 #include "grid.cuh"
+#include "far.cuh"
 #include "geom.cuh"
 #include "prims.cuh"
 
@@ -41,28 +42,28 @@ __global__ void k_edge_len(long nE, const int2* __restrict__ e, const double* __
     len[i] = sqrt(sqn(ld3(X, v.x) - ld3(X, v.y)));
 }
 
-__global__ void k_abs_dir(long nN, const int* __restrict__ nodes, const double* __restrict__ dir, double* __restrict__ out) {
-    long i = (long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= nN) return;
-    int v = nodes[i];
-    out[3 * i] = fabs(dir[3 * v]);
-    out[3 * i + 1] = fabs(dir[3 * v + 1]);
-    out[3 * i + 2] = fabs(dir[3 * v + 2]);
-}
+// component i of an instance's |dir| sequence: the three components of its
+// surface nodes in order
+struct AbsDir {
+    const int* nodes;
+    const double* dir;
+    __device__ double operator()(long i) const { return fabs(dir[3L * nodes[i / 3] + i % 3]); }
+};
 
 // first level of the fixed-order estimate of sum |dir| (a span cap can only
 // apply when this estimate comes near 1), one CTA per 2048-item tile of every
 // instance's |dir| segment
 __global__ void k_span_tiles(const SpanTile* __restrict__ tiles, const unsigned char* __restrict__ active,
-                             const double* __restrict__ absdir, double* __restrict__ out) {
+                             const int* __restrict__ nodes, const double* __restrict__ dir,
+                             double* __restrict__ out) {
     __shared__ double a[256];
     const SpanTile t = tiles[blockIdx.x];
     if (!active[t.inst]) return;
-    const double* in = absdir + t.start;
+    const AbsDir in = {nodes + t.start / 3, dir};
     double s = 0.0;
     for (int r = 0; r < 8; ++r) {
         long i = (long)t.k * 2048 + r * 256 + threadIdx.x;
-        if (i < t.m) s += in[i];
+        if (i < t.m) s += in(i);
     }
     a[threadIdx.x] = s;
     __syncthreads();
@@ -130,17 +131,17 @@ __device__ double cta_eigen_sum(const double* __restrict__ x, long n, double (*b
     return res;
 }
 
-// x[0] + x[1] + ... + x[n-1] added left to right into one accumulator (the
+// x(0) + x(1) + ... + x(n-1) added left to right into one accumulator (the
 // reference's serial loop), the items staged through shared memory by the
 // whole CTA while thread 0 adds the previous tile. Every thread must call
 // it; thread 0 receives the result.
-__device__ double cta_serial_sum(const double* __restrict__ x, long n, double (*buf)[kStageTile]) {
+__device__ double cta_serial_sum(const AbsDir x, long n, double (*buf)[kStageTile]) {
     const int tid = threadIdx.x;
     double acc = 0.0;
     for (long base = 0, k = 0; base < n; base += kStageTile, ++k) {
         double* t = buf[k & 1];
         const long m = min((long)kStageTile, n - base);
-        for (long i = tid; i < m; i += blockDim.x) t[i] = x[base + i];
+        for (long i = tid; i < m; i += blockDim.x) t[i] = x(base + i);
         __syncthreads();
         if (tid == 0) {
 #pragma unroll 8
@@ -206,12 +207,13 @@ __global__ void k_mean_edge(int nI, const int* __restrict__ se_off, const double
 __global__ void k_span_cap(int nI, const unsigned char* __restrict__ active, const int* __restrict__ se_off,
                            const int* __restrict__ sn_off, const int* __restrict__ tile_off,
                            const double* __restrict__ tsum, const double* __restrict__ len,
-                           const double* __restrict__ absdir, double* __restrict__ scratch,
+                           const int* __restrict__ nodes, const double* __restrict__ dir, double* __restrict__ scratch,
                            double* __restrict__ alpha, double* __restrict__ voxel_size,
-                           const double* __restrict__ voxel_pre) {
+                           const double* __restrict__ voxel_pre, unsigned long long* __restrict__ bb) {
     __shared__ double buf[2][kStageTile];
     __shared__ double s_vsz, s_est;
     int i = blockIdx.x;
+    if (threadIdx.x < 6) bb[6 * i + threadIdx.x] = threadIdx.x < 3 ? 0xffffffffffffffffull : 0ull;  // empty box
     if (!active[i]) return;
     const long e0 = se_off[i], ne = se_off[i + 1] - se_off[i];
     const long n0 = sn_off[i], nn = sn_off[i + 1] - sn_off[i];
@@ -230,7 +232,7 @@ __global__ void k_span_cap(int nI, const unsigned char* __restrict__ active, con
     double a = alpha[i];
     const double bound = 1.0 - ((double)(3 * nn) + 32.0) * 2.3e-16;
     if (!(s_est < bound)) {
-        double pSize = cta_serial_sum(absdir + 3 * n0, 3 * nn, buf);
+        double pSize = cta_serial_sum(AbsDir{nodes + n0, dir}, 3 * nn, buf);
         if (threadIdx.x == 0) {
             pSize /= cnt;
             const double spanSize = a * pSize / vsz;
@@ -243,10 +245,13 @@ __global__ void k_span_cap(int nI, const unsigned char* __restrict__ active, con
     }
 }
 
+// swept bounding box of every instance; FP32 positions of its surface vertices
+// relative to its first one, and FP32 displacements
 __global__ void k_ccd_bbox(long nN, const int* __restrict__ nodes, const int* __restrict__ ninst,
                            const unsigned char* __restrict__ active, const double* __restrict__ X,
                            const double* __restrict__ dir, const double* __restrict__ alpha,
-                           unsigned long long* __restrict__ bb) {
+                           const int* __restrict__ sn_off, unsigned long long* __restrict__ bb,
+                           float4* __restrict__ Xf, float4* __restrict__ df) {
     long s = (long)blockIdx.x * blockDim.x + threadIdx.x;
     const int inst = s < nN ? ninst[s] : 0;
     const int inst_first = ninst[(long)blockIdx.x * blockDim.x];
@@ -254,6 +259,9 @@ __global__ void k_ccd_bbox(long nN, const int* __restrict__ nodes, const int* __
     unsigned long long lo[3] = {0, 0, 0}, hi[3] = {0, 0, 0};
     if (valid) {
         int v = nodes[s];
+        const F3 f = tof(ld3(X, v) - ld3(X, nodes[sn_off[inst]])), g = tof(ld3(dir, v));
+        Xf[v] = make_float4(f.x, f.y, f.z, 0.0f);
+        df[v] = make_float4(g.x, g.y, g.z, 0.0f);
         double a = alpha[inst];
         double p[3] = {X[3 * v], X[3 * v + 1], X[3 * v + 2]};
         double q[3] = {X[3 * v] + a * dir[3 * v], X[3 * v + 1] + a * dir[3 * v + 1], X[3 * v + 2] + a * dir[3 * v + 2]};
@@ -265,26 +273,18 @@ __global__ void k_ccd_bbox(long nN, const int* __restrict__ nodes, const int* __
     bbox_block_update(valid, inst, inst_first, lo, hi, bb);
 }
 
-__global__ void k_bb_init(int nI, unsigned long long* bb) {
-    int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= 6 * nI) return;
-    bb[i] = (i % 6) < 3 ? 0xffffffffffffffffull : 0ull;
-}
-
-// SPATIAL_HASH.h:502-519
-__global__ void k_ccd_grid(int nI, const unsigned char* __restrict__ active, const unsigned long long* __restrict__ bb,
-                           const double* __restrict__ thick, const double* __restrict__ voxel_size,
-                           GridP* __restrict__ gp) {
-    int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= nI) return;
+// voxel grid of one instance (SPATIAL_HASH.h:502-519)
+__device__ GridP ccd_grid(int i, const unsigned char* __restrict__ active, const unsigned long long* __restrict__ bb,
+                          const double* __restrict__ thick, const double* __restrict__ voxel_size) {
     GridP g;
+    g.coarse = 1;
+    g.ext = 0.0f;
     if (!active[i]) {
         for (int d = 0; d < 3; ++d) { g.lo[d] = 0; g.n[d] = 1; }
         g.inv = 1;
         g.s1 = 2;
         g.s2 = 4;
-        gp[i] = g;
-        return;
+        return g;
     }
     double ht = thick[i] / 2;
     double lo[3], range[3];
@@ -319,49 +319,8 @@ __global__ void k_ccd_grid(int nI, const unsigned char* __restrict__ active, con
     g.inv = inv;
     g.s1 = (long)vc[0] + 1;
     g.s2 = g.s1 * ((long)vc[1] + 1);
-    gp[i] = g;
-}
-
-// swept voxel box of every surface node (SPATIAL_HASH.h:525-533)
-__global__ void k_node_box(long nN, const int* __restrict__ nodes, const int* __restrict__ ninst,
-                           const unsigned char* __restrict__ active, const double* __restrict__ X,
-                           const double* __restrict__ dir, const double* __restrict__ alpha,
-                           const double* __restrict__ thick, const GridP* __restrict__ gp, BoxI* __restrict__ nbox) {
-    long s = (long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (s >= nN) return;
-    int inst = ninst[s];
-    BoxI b;
-    if (!active[inst]) {
-        for (int d = 0; d < 3; ++d) { b.lo[d] = 1; b.hi[d] = 0; }
-        nbox[s] = b;
-        return;
-    }
-    GridP g = gp[inst];
-    int v = nodes[s];
-    double a = alpha[inst], ht = thick[inst] / 2;
-    for (int d = 0; d < 3; ++d) {
-        double p = X[3 * v + d], q = X[3 * v + d] + a * dir[3 * v + d];
-        double mn = fmin(p, q) - ht, mx = fmax(p, q) + ht;
-        b.lo[d] = (int)floor((mn - g.lo[d]) * g.inv);
-        b.hi[d] = (int)floor((mx - g.lo[d]) * g.inv);
-    }
-    nbox[s] = b;
-}
-
-template <int K>
-__global__ void k_prim_box_from_nodes(long n, const int* __restrict__ verts, const int* __restrict__ v2s,
-                                      const BoxI* __restrict__ nbox, BoxI* __restrict__ out) {
-    long i = (long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    BoxI b = nbox[v2s[verts[K * i]]];
-    for (int k = 1; k < K; ++k) {
-        BoxI c = nbox[v2s[verts[K * i + k]]];
-        for (int d = 0; d < 3; ++d) {
-            b.lo[d] = min(b.lo[d], c.lo[d]);
-            b.hi[d] = max(b.hi[d], c.hi[d]);
-        }
-    }
-    out[i] = b;
+    g.ext = (float)fmax(range[0], fmax(range[1], range[2]));
+    return g;
 }
 
 struct CCand {
@@ -374,27 +333,11 @@ struct CCand {
 // overlap) is applied to every pair it returns
 constexpr double kCcdCellBudget = 4194304.0;
 
-// coarse boxes of the triangles, edges and nodes (stored in that order),
-// clamped to the coarse grid [0, n]: the clamp is monotone, so every pair of
-// overlapping boxes still overlaps, and all query and table cells exist
-__global__ void k_coarse_boxes(long pt, long pe, long pn, long nt, long ne, long nn, const int* __restrict__ tinst,
-                               const int* __restrict__ einst, const int* __restrict__ ninst,
-                               const GridP* __restrict__ gc, const BoxI* __restrict__ in, BoxI* __restrict__ out) {
-    // segments are padded to pt, pe, pn boxes (at least one each); padding
-    // boxes are left empty
-    long i = (long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= pt + pe + pn) return;
-    int inst = -1;
-    if (i < pt) { if (i < nt) inst = tinst[i]; }
-    else if (i < pt + pe) { if (i - pt < ne) inst = einst[i - pt]; }
-    else if (i - pt - pe < nn) inst = ninst[i - pt - pe];
-    BoxI b = in[i], c;
-    if (inst < 0) {
-        for (int d = 0; d < 3; ++d) { c.lo[d] = 1; c.hi[d] = 0; }
-        out[i] = c;
-        return;
-    }
-    const GridP g = gc[inst];
+// a voxel box in coarse cells, clamped to the coarse grid [0, n]: the clamp is
+// monotone, so every pair of overlapping boxes still overlaps, and all query
+// and table cells exist
+__device__ __forceinline__ BoxI coarse_box(const BoxI& b, const GridP& g) {
+    BoxI c;
     for (int d = 0; d < 3; ++d) {
         if (b.lo[d] > b.hi[d]) {  // empty box (inactive instance) stays empty
             c.lo[d] = 1;
@@ -406,22 +349,99 @@ __global__ void k_coarse_boxes(long pt, long pe, long pn, long nt, long ne, long
         c.lo[d] = clampi(lo, 0, g.n[d]);
         c.hi[d] = clampi(hi, 0, g.n[d]);
     }
-    out[i] = c;
+    return c;
 }
 
-__global__ void k_coarse_grid(int nI, const GridP* __restrict__ gp, GridP* __restrict__ gc) {
-    int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= nI) return;
-    GridP g = gp[i];
-    int c = 1;
-    while (c < (1 << 20) && ((double)(g.n[0] / c + 2) * (double)(g.n[1] / c + 2) * (double)(g.n[2] / c + 2)) >
-                                kCcdCellBudget)
-        c *= 2;
-    g.coarse = c;
-    for (int d = 0; d < 3; ++d) g.n[d] = g.n[d] / c + 1;
-    g.s1 = (long)g.n[0] + 1;
-    g.s2 = g.s1 * ((long)g.n[1] + 1);
-    gc[i] = g;
+// voxel grids gp and coarse grids gc of every instance, the step sizes' start
+// values and, when cbase is given, the coarse grids' cell bases (one CTA)
+__global__ void k_ccd_grids(int nI, const unsigned char* __restrict__ active, const unsigned long long* __restrict__ bb,
+                            const double* __restrict__ thick, const double* __restrict__ voxel_size,
+                            GridP* __restrict__ gp, GridP* __restrict__ gc, double* __restrict__ amin,
+                            int* __restrict__ flags, uint32_t* __restrict__ cbase,
+                            unsigned long long* __restrict__ total, unsigned long long cap,
+                            unsigned int* __restrict__ flag) {
+    for (int i = threadIdx.x; i < nI; i += blockDim.x) {
+        GridP g = ccd_grid(i, active, bb, thick, voxel_size);
+        gp[i] = g;
+        int c = 1;
+        while (c < (1 << 20) && ((double)(g.n[0] / c + 2) * (double)(g.n[1] / c + 2) * (double)(g.n[2] / c + 2)) >
+                                    kCcdCellBudget)
+            c *= 2;
+        g.coarse = c;
+        for (int d = 0; d < 3; ++d) g.n[d] = g.n[d] / c + 1;
+        g.s1 = (long)g.n[0] + 1;
+        g.s2 = g.s1 * ((long)g.n[1] + 1);
+        gc[i] = g;
+        amin[i] = 1e300;
+        flags[i] = 0;
+    }
+    if (!cbase) return;
+    __syncthreads();
+    cta_cell_bases(nI, gc, cbase, total, cap, flag);
+}
+
+// swept voxel box of every surface node (SPATIAL_HASH.h:525-533) and its coarse box
+__global__ void k_node_box(long nN, const int* __restrict__ nodes, const int* __restrict__ ninst,
+                           const unsigned char* __restrict__ active, const double* __restrict__ X,
+                           const double* __restrict__ dir, const double* __restrict__ alpha,
+                           const double* __restrict__ thick, const GridP* __restrict__ gp,
+                           const GridP* __restrict__ gc, BoxI* __restrict__ nbox, BoxI* __restrict__ nboxc) {
+    long s = (long)blockIdx.x * blockDim.x + threadIdx.x;
+    if (s >= nN) return;
+    int inst = ninst[s];
+    BoxI b;
+    if (!active[inst]) {
+        for (int d = 0; d < 3; ++d) { b.lo[d] = 1; b.hi[d] = 0; }
+    } else {
+        GridP g = gp[inst];
+        int v = nodes[s];
+        double a = alpha[inst], ht = thick[inst] / 2;
+        for (int d = 0; d < 3; ++d) {
+            double p = X[3 * v + d], q = X[3 * v + d] + a * dir[3 * v + d];
+            double mn = fmin(p, q) - ht, mx = fmax(p, q) + ht;
+            b.lo[d] = (int)floor((mn - g.lo[d]) * g.inv);
+            b.hi[d] = (int)floor((mx - g.lo[d]) * g.inv);
+        }
+    }
+    nbox[s] = b;
+    nboxc[s] = coarse_box(b, gc[inst]);
+}
+
+// boxes of the triangles [0, nt) and edges [nt, nt + ne) from their nodes'
+// boxes, their coarse boxes, and the coarse cells counted in the table of each
+// kind (ccount null: boxes only)
+__global__ void k_prim_boxes_from_nodes(long nt, long ne, const int* __restrict__ tris, const int2* __restrict__ edges,
+                                        const int* __restrict__ tinst, const int* __restrict__ einst,
+                                        const unsigned char* __restrict__ active, const int* __restrict__ v2s,
+                                        const BoxI* __restrict__ nbox, const GridP* __restrict__ gc,
+                                        BoxI* __restrict__ tbox, BoxI* __restrict__ ebox, BoxI* __restrict__ tboxc,
+                                        BoxI* __restrict__ eboxc, const uint32_t* __restrict__ cbase, uint32_t cap,
+                                        uint32_t* __restrict__ ccount) {
+    const long i = (long)blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= nt + ne) return;
+    const bool tri = i < nt;
+    int v[3];
+    if (tri) {
+        for (int k = 0; k < 3; ++k) v[k] = tris[3 * i + k];
+    } else {
+        const int2 e = edges[i - nt];
+        v[0] = e.x;
+        v[1] = v[2] = e.y;
+    }
+    BoxI b = nbox[v2s[v[0]]];
+    for (int k = 1; k < (tri ? 3 : 2); ++k) {
+        const BoxI c = nbox[v2s[v[k]]];
+        for (int d = 0; d < 3; ++d) {
+            b.lo[d] = min(b.lo[d], c.lo[d]);
+            b.hi[d] = max(b.hi[d], c.hi[d]);
+        }
+    }
+    const int inst = tri ? tinst[i] : einst[i - nt];
+    const GridP g = gc[inst];
+    const BoxI c = coarse_box(b, g);
+    if (tri) { tbox[i] = b; tboxc[i] = c; }
+    else { ebox[i - nt] = b; eboxc[i - nt] = c; }
+    if (ccount && active[inst]) count_cells(c, g, cbase[inst], cap, ccount + (tri ? 0 : (size_t)cap + 1));
 }
 
 __device__ __forceinline__ bool boxes_overlap(const BoxI& a, const BoxI& b) {
@@ -437,20 +457,38 @@ __device__ __forceinline__ bool swept_far(const double* lo_a, const double* hi_a
     return false;
 }
 
+// A pair further apart than this cannot lower the step size: the first
+// conservative advance of its ACCD, 0.9 (d - thickness) / |relative motion|,
+// already exceeds the step size alpha it starts from, so the loop ends there
+// without a hit (with 5 % in hand; the motion's bound carries its rounding).
+__device__ __forceinline__ float ccd_reach(const F3* d, int split, float alpha, float th, float ext) {
+    const F3 mov = 0.25f * (((d[0] + d[1]) + d[2]) + d[3]);
+    float ma = 0.0f, mb = 0.0f, mag = 0.0f;
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+        const float m = sqn(d[k] - mov);
+        if (k < split) ma = fmaxf(ma, m);
+        else mb = fmaxf(mb, m);
+        mag += fabsf(d[k].x) + fabsf(d[k].y) + fabsf(d[k].z);
+    }
+    const float motion = (sqrtf(ma) + sqrtf(mb)) * 1.00001f + 1e-6f * mag;
+    return alpha * motion * (1.0f / (0.9f * 0.95f)) + th + kFarMargin * ext;
+}
+
 // one lane group per surface node: triangles whose voxel boxes overlap the node's
 // swept voxel box (Query_Point_For_Primitives, SPATIAL_HASH.h:624-647), then
 // the exclusions and swept-AABB test of IPC.h:1980-2006
-__global__ void k_ccd_query_pt(long nN, const int* __restrict__ nodes, const int* __restrict__ ninst,
-                               const unsigned char* __restrict__ active, const double* __restrict__ X,
-                               const double* __restrict__ dir, const unsigned char* __restrict__ dbc,
-                               const int* __restrict__ tris, const BoxI* __restrict__ nbox,
-                               const BoxI* __restrict__ tbox, const BoxI* __restrict__ nboxc,
-                               const BoxI* __restrict__ tboxc, const GridP* __restrict__ gp,
-                               const double* __restrict__ thick, CellHash cells,
-                               const uint32_t* __restrict__ cstart, const uint32_t* __restrict__ entries,
-                               CCand* __restrict__ out, unsigned int* counter, long cap) {
-    long s = ((long)blockIdx.x * blockDim.x + threadIdx.x) / kCcdQueryLanes;
-    if (s >= nN) return;
+__device__ __forceinline__ void ccd_query_pt(long s, const int* __restrict__ nodes, const int* __restrict__ ninst,
+                                             const unsigned char* __restrict__ active, const double* __restrict__ X,
+                                             const double* __restrict__ dir, const float4* __restrict__ Xf,
+                                             const float4* __restrict__ df, const double* __restrict__ alpha,
+                                             const unsigned char* __restrict__ dbc, const int* __restrict__ tris,
+                                             const BoxI* __restrict__ nbox, const BoxI* __restrict__ tbox,
+                                             const BoxI* __restrict__ nboxc, const BoxI* __restrict__ tboxc,
+                                             const GridP* __restrict__ gp, const double* __restrict__ thick,
+                                             const CellHash& cells, const uint32_t* __restrict__ cstart,
+                                             const uint32_t* __restrict__ entries, CCand* __restrict__ out,
+                                             unsigned int* counter, long cap) {
     int inst = ninst[s];
     if (!active[inst]) return;
     int vI = nodes[s];
@@ -462,6 +500,8 @@ __global__ void k_ccd_query_pt(long nN, const int* __restrict__ nodes, const int
         plo[d] = fmin(p, pe);
         phi[d] = fmax(p, pe);
     }
+    const F3 pf = ldf(Xf, vI), pd = ldf(df, vI);
+    const float al = (float)alpha[inst] * 1.000001f;
     const BoxI qc = nboxc[s], qx = nbox[s];
     const bool pdbc = dbc[vI] != 0;
     group_walk_emit<kCcdQueryLanes>(qc, inst, g, cells, cstart, entries, out, counter, cap,
@@ -470,6 +510,10 @@ __global__ void k_ccd_query_pt(long nN, const int* __restrict__ nodes, const int
                        if (!is_first_shared(qc, tboxc[f], cx, cy, cz) || !boxes_overlap(qx, tbox[f])) return false;
                        int t0 = tris[3 * f], t1 = tris[3 * f + 1], t2 = tris[3 * f + 2];
                        if (vI == t0 || vI == t1 || vI == t2) return false;
+                       const F3 mv[4] = {pd, ldf(df, t0), ldf(df, t1), ldf(df, t2)};
+                       if (al > 0.0f && far_point_triangle(pf, ldf(Xf, t0), ldf(Xf, t1), ldf(Xf, t2),
+                                                           ccd_reach(mv, 1, al, (float)th, g.ext)))
+                           return false;
                        if (pdbc && dbc[t0] && dbc[t1] && dbc[t2]) return false;
                        double tlo[3], thi[3];
                        const int tv[3] = {t0, t1, t2};
@@ -491,16 +535,15 @@ __global__ void k_ccd_query_pt(long nN, const int* __restrict__ nodes, const int
 
 // one lane group per surface edge: edges eJ > eI with overlapping voxel boxes
 // (SPATIAL_HASH.h:650-662), exclusions and swept-AABB test of IPC.h:2193-2230
-__global__ void k_ccd_query_ee(long nE, const int2* __restrict__ edges, const int* __restrict__ einst,
-                               const unsigned char* __restrict__ active, const double* __restrict__ X,
-                               const double* __restrict__ dir, const unsigned char* __restrict__ dbc,
-                               const BoxI* __restrict__ ebox, const BoxI* __restrict__ eboxc,
-                               const GridP* __restrict__ gp, const double* __restrict__ thick,
-                               CellHash cells, const uint32_t* __restrict__ cstart,
-                               const uint32_t* __restrict__ entries, CCand* __restrict__ out, unsigned int* counter,
-                               long cap) {
-    long eI = ((long)blockIdx.x * blockDim.x + threadIdx.x) / kCcdQueryLanes;
-    if (eI >= nE) return;
+__device__ __forceinline__ void ccd_query_ee(long eI, const int2* __restrict__ edges, const int* __restrict__ einst,
+                                             const unsigned char* __restrict__ active, const double* __restrict__ X,
+                                             const double* __restrict__ dir, const float4* __restrict__ Xf,
+                                             const float4* __restrict__ df, const double* __restrict__ alpha,
+                                             const unsigned char* __restrict__ dbc, const BoxI* __restrict__ ebox,
+                                             const BoxI* __restrict__ eboxc, const GridP* __restrict__ gp,
+                                             const double* __restrict__ thick, const CellHash& cells,
+                                             const uint32_t* __restrict__ cstart, const uint32_t* __restrict__ entries,
+                                             CCand* __restrict__ out, unsigned int* counter, long cap) {
     int inst = einst[eI];
     if (!active[inst]) return;
     int2 mi = edges[eI];
@@ -518,6 +561,8 @@ __global__ void k_ccd_query_ee(long nE, const int2* __restrict__ edges, const in
         alo[d] = mn;
         ahi[d] = mx;
     }
+    const F3 f0 = ldf(Xf, mi.x), f1 = ldf(Xf, mi.y), d0 = ldf(df, mi.x), d1 = ldf(df, mi.y);
+    const float al = (float)alpha[inst] * 1.000001f;
     const BoxI qc = eboxc[eI], qx = ebox[eI];
     const bool adbc = dbc[mi.x] && dbc[mi.y];
     group_walk_emit<kCcdQueryLanes>(qc, inst, g, cells, cstart, entries, out, counter, cap,
@@ -527,6 +572,10 @@ __global__ void k_ccd_query_ee(long nE, const int2* __restrict__ edges, const in
                            return false;
                        int2 mj = edges[eJ];
                        if (mi.x == mj.x || mi.x == mj.y || mi.y == mj.x || mi.y == mj.y) return false;
+                       const F3 mv[4] = {d0, d1, ldf(df, mj.x), ldf(df, mj.y)};
+                       if (al > 0.0f && far_segments(f0, f1, ldf(Xf, mj.x), ldf(Xf, mj.y),
+                                                     ccd_reach(mv, 2, al, (float)th, g.ext)))
+                           return false;
                        if (adbc && dbc[mj.x] && dbc[mj.y]) return false;
                        double blo[3], bhi[3];
                        const int bv[2] = {mj.x, mj.y};
@@ -544,6 +593,32 @@ __global__ void k_ccd_query_ee(long nE, const int2* __restrict__ edges, const in
                        c = {(int)eI, eJ};
                        return true;
                    });
+}
+
+// both queries in one launch: the first bpt CTAs take the nodes, the others
+// the edges
+__global__ void k_ccd_query(unsigned int bpt, long nN, const int* __restrict__ nodes, const int* __restrict__ ninst,
+                            long nE, const int2* __restrict__ edges, const int* __restrict__ einst,
+                            const unsigned char* __restrict__ active, const double* __restrict__ X,
+                            const double* __restrict__ dir, const float4* __restrict__ Xf,
+                            const float4* __restrict__ df, const double* __restrict__ alpha,
+                            const unsigned char* __restrict__ dbc, const int* __restrict__ tris,
+                            const BoxI* __restrict__ nbox, const BoxI* __restrict__ tbox, const BoxI* __restrict__ ebox,
+                            const BoxI* __restrict__ nboxc, const BoxI* __restrict__ tboxc,
+                            const BoxI* __restrict__ eboxc, const GridP* __restrict__ gp,
+                            const double* __restrict__ thick, CellHash tcells, const uint32_t* __restrict__ tstart,
+                            const uint32_t* __restrict__ tentries, CellHash ecells,
+                            const uint32_t* __restrict__ estart, const uint32_t* __restrict__ eentries,
+                            CCand* __restrict__ out, unsigned int* counter, long cap_pt, long cap_ee) {
+    const bool pt = blockIdx.x < bpt;
+    const long q = ((long)(blockIdx.x - (pt ? 0u : bpt)) * blockDim.x + threadIdx.x) / kCcdQueryLanes;
+    if (q >= (pt ? nN : nE)) return;  // the whole group leaves together
+    if (pt)
+        ccd_query_pt(q, nodes, ninst, active, X, dir, Xf, df, alpha, dbc, tris, nbox, tbox, nboxc, tboxc, gp, thick,
+                     tcells, tstart, tentries, out, counter, cap_pt);
+    else
+        ccd_query_ee(q, edges, einst, active, X, dir, Xf, df, alpha, dbc, ebox, eboxc, gp, thick, ecells, estart,
+                     eentries, out + cap_pt, counter + 1, cap_ee);
 }
 
 // ---- ACCD (CCD.h:279-328, 330-395)
@@ -679,16 +754,12 @@ __global__ void k_accd(const unsigned int* __restrict__ counts, long cap_pt, lon
         accd_one(k, npt, cand_pt, cand_ee, nodes, ninst, tris, edges, einst, X, dir, thick, alpha_cap, alpha_min, flags);
 }
 
-__global__ void k_alpha_final(int nI, const unsigned char* __restrict__ active, const double* __restrict__ amin,
-                              double* __restrict__ alpha) {
+// step sizes into amin (alpha is kept for the case that the build is redone)
+__global__ void k_alpha_final(int nI, const unsigned char* __restrict__ active, const double* __restrict__ alpha,
+                              double* __restrict__ amin) {
     int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= nI || !active[i]) return;
-    alpha[i] = fmin(alpha[i], amin[i]);
-}
-
-__global__ void k_fill(int n, double v, double* a) {
-    int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < n) a[i] = v;
+    if (i >= nI) return;
+    amin[i] = active[i] ? fmin(alpha[i], amin[i]) : alpha[i];
 }
 
 }  // namespace
@@ -709,35 +780,33 @@ const double* ccd_voxel_sizes(Arena& A, Work& W) {
 }
 
 int ccd_stepsize(Arena& A, Work& W, const double* X, const double* dir, double* alpha, int* flags, cudaStream_t s,
-                 const double* voxel_pre) {
+                 const double* voxel_pre, double* host_alpha, int* host_flags) {
     const int nI = A.nI;
     long Se = A.Se > 0 ? A.Se : 1, Sn = A.Sn > 0 ? A.Sn : 1;
-    // scratch layout (doubles): len[Se] | absdir[3Sn] | sum scratch | voxel[nI] | amin[nI]
+    // scratch layout (doubles): len[Se] | sum scratch | voxel[nI] | amin[nI]
     long nsum = 2 * (A.Se + 3 * A.Sn) / 1024 + 16 * (long)nI + 64;
-    if (W[W_CCD_TMP].ensure(sizeof(double) * (Se + 3 * Sn + nsum + 2 * nI + 8))) return IDP_ERR_CUDA;
+    if (W[W_CCD_TMP].ensure(sizeof(double) * (Se + nsum + 2 * nI + 8))) return IDP_ERR_CUDA;
     double* len = W[W_CCD_TMP].as<double>();
-    double* absdir = len + Se;
-    double* sumsc = absdir + 3 * Sn;
+    double* sumsc = len + Se;
     double* vsz = sumsc + nsum;
     double* amin = vsz + nI;
-    const int* d_se_off = A.d_se_off;
-    const int* d_sn_off = A.d_sn_off;
-    if (A.Se && !voxel_pre) (::idp::count_launch(), k_edge_len<<<grid_for(A.Se), kBlock, 0, s>>>(A.Se, A.sedge, X, len));
-    if (A.Sn) (::idp::count_launch(), k_abs_dir<<<grid_for(A.Sn), kBlock, 0, s>>>(A.Sn, A.snode, dir, absdir));
-    if (W[W_SPAN].ensure(sizeof(double) * (A.n_span_tiles + 1))) return IDP_ERR_CUDA;
-    double* tsum = W[W_SPAN].as<double>();
-    if (A.n_span_tiles > 0)
-        (::idp::count_launch(), k_span_tiles<<<A.n_span_tiles, 256, 0, s>>>(A.span_tiles, A.active, absdir, tsum));
-    (::idp::count_launch(), k_span_cap<<<nI, 256, 0, s>>>(nI, A.active, d_se_off, d_sn_off, A.span_tile_off, tsum,
-                                                          len, absdir, sumsc, alpha, vsz, voxel_pre));
-    // grid
-    if (W[W_BBOX].ensure(sizeof(unsigned long long) * 6 * nI) || W[W_GRIDP].ensure(sizeof(GridP) * nI))
+    if (W[W_SPAN].ensure(sizeof(double) * (A.n_span_tiles + 1)) ||
+        W[W_BBOX].ensure(sizeof(unsigned long long) * 6 * nI) || W[W_GRIDP].ensure(sizeof(GridP) * nI) ||
+        W[W_XF].ensure(sizeof(float4) * (A.V + 1)) || W[W_DF].ensure(sizeof(float4) * (A.V + 1)))
         return IDP_ERR_CUDA;
     unsigned long long* bb = W[W_BBOX].as<unsigned long long>();
     GridP* gp = W[W_GRIDP].as<GridP>();
-    (::idp::count_launch(), k_bb_init<<<grid_for(6 * nI), kBlock, 0, s>>>(nI, bb));
-    if (A.Sn) (::idp::count_launch(), k_ccd_bbox<<<grid_for(A.Sn), kBlock, 0, s>>>(A.Sn, A.snode, A.sn_inst, A.active, X, dir, alpha, bb));
-    (::idp::count_launch(), k_ccd_grid<<<grid_for(nI), kBlock, 0, s>>>(nI, A.active, bb, A.thickness, vsz, gp));
+    float4 *Xf = W[W_XF].as<float4>(), *df = W[W_DF].as<float4>();
+    double* tsum = W[W_SPAN].as<double>();
+    if (A.Se && !voxel_pre) (::idp::count_launch(), k_edge_len<<<grid_for(A.Se), kBlock, 0, s>>>(A.Se, A.sedge, X, len));
+    if (A.n_span_tiles > 0)
+        (::idp::count_launch(), k_span_tiles<<<A.n_span_tiles, 256, 0, s>>>(A.span_tiles, A.active, A.snode, dir, tsum));
+    (::idp::count_launch(), k_span_cap<<<nI, 256, 0, s>>>(nI, A.active, A.d_se_off, A.d_sn_off, A.span_tile_off, tsum,
+                                                          len, A.snode, dir, sumsc, alpha, vsz, voxel_pre, bb));
+    // grid
+    if (A.Sn)
+        (::idp::count_launch(), k_ccd_bbox<<<grid_for(A.Sn), kBlock, 0, s>>>(A.Sn, A.snode, A.sn_inst, A.active, X, dir,
+                                                                             alpha, A.d_sn_off, bb, Xf, df));
     long St = A.St > 0 ? A.St : 1;
     if (W[W_BOX_A].ensure(sizeof(BoxI) * 2 * (St + Se + Sn)) || W[W_BOX_B].ensure(sizeof(GridP) * (nI + 1)))
         return IDP_ERR_CUDA;
@@ -748,50 +817,54 @@ int ccd_stepsize(Arena& A, Work& W, const double* X, const double* dir, double* 
     BoxI* eboxc = tboxc + St;
     BoxI* nboxc = eboxc + Se;
     GridP* gc = W[W_BOX_B].as<GridP>();
-    if (A.Sn)
-        (::idp::count_launch(), k_node_box<<<grid_for(A.Sn), kBlock, 0, s>>>(A.Sn, A.snode, A.sn_inst, A.active, X, dir, alpha, A.thickness, gp,
-                                                     nbox));
-    // triangle / edge boxes from node boxes (v2s: vertex -> surface node)
-    if (A.St)
-        (::idp::count_launch(), k_prim_box_from_nodes<3><<<grid_for(A.St), kBlock, 0, s>>>(A.St, A.stri, A.v2s, nbox, tbox));
-    if (A.Se)
-        (::idp::count_launch(), k_prim_box_from_nodes<2><<<grid_for(A.Se), kBlock, 0, s>>>(A.Se, reinterpret_cast<const int*>(A.sedge), A.v2s,
-                                                                   nbox, ebox));
-    (::idp::count_launch(), k_coarse_grid<<<grid_for(nI), kBlock, 0, s>>>(nI, gp, gc));
-    (::idp::count_launch(), k_coarse_boxes<<<grid_for(St + Se + Sn), kBlock, 0, s>>>(
-                                St, Se, Sn, A.St, A.Se, A.Sn, A.st_inst, A.se_inst, A.sn_inst, gc, tbox, tboxc));
     // grids, candidates (PT in [0, cap_pt), EE in [cap_pt, cap_pt + cap_ee))
     // and ACCD without a host round trip; one synchronisation at the end reads
-    // the candidate counts and the grids' overflow flag (ccount[2]), and only
-    // a build that fitted publishes its step sizes
+    // the candidate counts, the grids' overflow flag (ccount[2]) and the
+    // results, and only a build that fitted publishes its step sizes
     uint32_t* hp = W.pinned();
-    if (!hp) return IDP_ERR_CUDA;
+    double* hres = W.pinned_doubles(2 * (long)nI);
+    if (!hp || !hres) return IDP_ERR_CUDA;
+    int* hflags = reinterpret_cast<int*>(hres + nI);
     if (W[W_CAND_CNT].ensure(64)) return IDP_ERR_CUDA;
     unsigned int* ccount = W[W_CAND_CNT].as<unsigned int>();
     long cap_pt = std::max<long>(W.ccd_cap_pt, 4 * A.Sn + 1024);
     long cap_ee = std::max<long>(W.ccd_cap_ee, 4 * A.Se + 1024);
     for (int attempt = 0; attempt < 8; ++attempt) {
         BoxGrid gt, ge;
+        GridTables t;
         IDP_CUDA_TRY(cudaMemsetAsync(ccount, 0, 3 * sizeof(unsigned int), s));
-        int rc = grids_build(W, 1, tboxc, A.St, A.st_inst, eboxc, A.Se, A.se_inst, A.active, gc, nI, ccount + 2, gt, ge,
-                             s);
+        int rc = grids_tables(W, 1, nI, t, s);
+        if (rc) return rc;
+        (::idp::count_launch(), k_ccd_grids<<<1, kBlock, 0, s>>>(nI, A.active, bb, A.thickness, vsz, gp, gc, amin, flags,
+                                                                 t.cbase, t.total, t.cap, ccount + 2));
+        if (A.Sn)
+            (::idp::count_launch(), k_node_box<<<grid_for(A.Sn), kBlock, 0, s>>>(A.Sn, A.snode, A.sn_inst, A.active, X,
+                                                                                 dir, alpha, A.thickness, gp, gc, nbox,
+                                                                                 nboxc));
+        // triangle / edge boxes from node boxes (v2s: vertex -> surface node)
+        if (A.St + A.Se)
+            (::idp::count_launch(), k_prim_boxes_from_nodes<<<grid_for(A.St + A.Se), kBlock, 0, s>>>(
+                                        A.St, A.Se, A.stri, A.sedge, A.st_inst, A.se_inst, A.active, A.v2s, nbox, gc,
+                                        tbox, ebox, tboxc, eboxc, t.cbase, t.cap, t.ccount));
+        rc = grids_build(W, 1, tboxc, A.St, A.st_inst, eboxc, A.Se, A.se_inst, A.active, gc, nI, ccount + 2, gt, ge, s,
+                         t.ccount != nullptr);
         if (rc) return rc;
         if (W[W_CAND].ensure(sizeof(CCand) * (cap_pt + cap_ee))) return IDP_ERR_CUDA;
         CCand* cand = W[W_CAND].as<CCand>();
-        if (A.Sn)
-            (::idp::count_launch(), k_ccd_query_pt<<<grid_for(kCcdQueryLanes * A.Sn), kBlock, 0, s>>>(A.Sn, A.snode, A.sn_inst, A.active, X, dir, A.dbc_excl, A.stri,
-                                                             nbox, tbox, nboxc, tboxc, gc, A.thickness, gt.cells, gt.cell_start,
-                                                             gt.entries, cand, ccount, cap_pt));
-        if (A.Se)
-            (::idp::count_launch(), k_ccd_query_ee<<<grid_for(kCcdQueryLanes * A.Se), kBlock, 0, s>>>(A.Se, A.sedge, A.se_inst, A.active, X, dir, A.dbc_excl, ebox, eboxc, gc,
-                                                             A.thickness, ge.cells, ge.cell_start,
-                                                             ge.entries, cand + cap_pt, ccount + 1, cap_ee));
-        (::idp::count_launch(), k_fill<<<grid_for(nI), kBlock, 0, s>>>(nI, 1e300, amin));
-        IDP_CUDA_TRY(cudaMemsetAsync(flags, 0, sizeof(int) * nI, s));
+        const int bpt = A.Sn ? grid_for(kCcdQueryLanes * A.Sn) : 0, bee = A.Se ? grid_for(kCcdQueryLanes * A.Se) : 0;
+        if (bpt + bee)
+            (::idp::count_launch(), k_ccd_query<<<bpt + bee, kBlock, 0, s>>>(
+                                        (unsigned int)bpt, A.Sn, A.snode, A.sn_inst, A.Se, A.sedge, A.se_inst, A.active,
+                                        X, dir, Xf, df, alpha, A.dbc_excl, A.stri, nbox, tbox, ebox, nboxc, tboxc, eboxc,
+                                        gc, A.thickness, gt.cells, gt.cell_start, gt.entries, ge.cells, ge.cell_start,
+                                        ge.entries, cand, ccount, cap_pt, cap_ee));
         (::idp::count_launch(), k_accd<<<kAccdBlocks, 128, 0, s>>>(ccount, cap_pt, cap_ee, cand, cand + cap_pt, A.snode,
                                                                     A.sn_inst, A.stri, A.sedge, A.se_inst, X, dir,
                                                                     A.thickness, alpha, amin, flags));
+        (::idp::count_launch(), k_alpha_final<<<grid_for(nI), kBlock, 0, s>>>(nI, A.active, alpha, amin));
         IDP_CUDA_TRY(cudaMemcpyAsync(hp + 2, ccount, 3 * sizeof(unsigned int), cudaMemcpyDeviceToHost, s));
+        if (host_alpha) IDP_CUDA_TRY(cudaMemcpyAsync(hres, amin, sizeof(double) * nI, cudaMemcpyDeviceToHost, s));
+        if (host_flags) IDP_CUDA_TRY(cudaMemcpyAsync(hflags, flags, sizeof(int) * nI, cudaMemcpyDeviceToHost, s));
         IDP_CUDA_TRY(cudaStreamSynchronize(s));
         const long npt = hp[2], nee = hp[3];
         if (grids_overflowed(W, 1, hp[4])) continue;
@@ -802,7 +875,9 @@ int ccd_stepsize(Arena& A, Work& W, const double* X, const double* dir, double* 
             W.ccd_cap_ee = cap_ee;
             continue;
         }
-        (::idp::count_launch(), k_alpha_final<<<grid_for(nI), kBlock, 0, s>>>(nI, A.active, amin, alpha));
+        IDP_CUDA_TRY(cudaMemcpyAsync(alpha, amin, sizeof(double) * nI, cudaMemcpyDeviceToDevice, s));
+        if (host_alpha) std::copy(hres, hres + nI, host_alpha);
+        if (host_flags) std::copy(hflags, hflags + nI, host_flags);
         if (std::getenv("IDP_PROFILE")) {
             unsigned long long st[4] = {0, 0, 0, 0};
             void* sym = nullptr;
@@ -817,7 +892,7 @@ int ccd_stepsize(Arena& A, Work& W, const double* X, const double* dir, double* 
         }
         return cudaGetLastError() == cudaSuccess ? IDP_OK : IDP_ERR_CUDA;
     }
-        return IDP_ERR_CAPACITY;
+    return IDP_ERR_CAPACITY;
 }
 
 }  // namespace idp

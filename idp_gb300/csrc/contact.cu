@@ -5,10 +5,12 @@
 //      origin = min surface-node position), triangles and edges binned into
 //      the cells their integer boxes cover, (instance, cell) radix-sorted;
 //   2. point-triangle and edge-edge queries walk their +-dHat box, report each
-//      candidate once (lowest shared cell) after the reference's exclusions and
-//      AABB test (CCD.h:149-185), compacted warp-cooperatively;
-//   3. narrow phase: FP64 distance type + squared distance, d < dHat^2, and the
-//      sign-tagged int4 encoding of IPC.h:202-250 / 434-554;
+//      candidate once (lowest shared cell) after the reference's exclusions,
+//      unless a conservative FP32 bound shows the pair beyond dHat (far.cuh),
+//      compacted warp-cooperatively;
+//   3. narrow phase: AABB test (CCD.h:149-185), FP64 distance type + squared
+//      distance, d < dHat^2, and the sign-tagged int4 encoding of
+//      IPC.h:202-250 / 434-554;
 //   4. records sorted by (instance, c0, c1, c2, c3); duplicate regular PP/PE
 //      records merged with multiplicity -count in slot 3 (IPC.h:599-654).
 // The grid is only a conservative filter; membership is decided by the same
@@ -16,6 +18,7 @@
 // size. The output order is the sort order, independent of thread timing.
 #include "engine.hpp"
 #include "grid.cuh"
+#include "far.cuh"
 #include "geom.cuh"
 #include "predicates.cuh"
 #include "prims.cuh"
@@ -26,16 +29,21 @@ using namespace geo;
 
 namespace {
 
+// bounding box of every instance, and the FP32 positions of its surface
+// vertices relative to its first one
 __global__ void k_bbox(long n, const int* __restrict__ nodes, const int* __restrict__ ninst,
                        const unsigned char* __restrict__ active, const double* __restrict__ X,
-                       unsigned long long* __restrict__ bb) {
+                       const int* __restrict__ sn_off, unsigned long long* __restrict__ bb, float4* __restrict__ Xf) {
     long i = (long)blockIdx.x * blockDim.x + threadIdx.x;
     const int inst = i < n ? ninst[i] : 0;
     const int inst_first = ninst[(long)blockIdx.x * blockDim.x];
     const bool valid = i < n && active[inst];
     unsigned long long lo[3] = {0, 0, 0}, hi[3] = {0, 0, 0};
     if (valid) {
-        D3 p = ld3(X, nodes[i]);
+        const int v = nodes[i];
+        D3 p = ld3(X, v);
+        const F3 f = tof(p - ld3(X, nodes[sn_off[inst]]));
+        Xf[v] = make_float4(f.x, f.y, f.z, 0.0f);
         lo[0] = hi[0] = ord_enc(p.x);
         lo[1] = hi[1] = ord_enc(p.y);
         lo[2] = hi[2] = ord_enc(p.z);
@@ -49,12 +57,10 @@ __global__ void k_bbox_init(int nI, unsigned long long* bb) {
     bb[i] = (i % 6) < 3 ? 0xffffffffffffffffull : 0ull;
 }
 
-// grid parameters of the constraint-set grid
-__global__ void k_grid_params(int nI, const unsigned long long* __restrict__ bb, const double* __restrict__ cell,
-                              const double* __restrict__ dHat2, const double* __restrict__ thick,
-                              const unsigned char* __restrict__ active, GridP* __restrict__ gp) {
-    int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= nI) return;
+// grid parameters of the constraint-set grid of one instance
+__device__ GridP grid_params(int i, const unsigned long long* __restrict__ bb, const double* __restrict__ cell,
+                             const double* __restrict__ dHat2, const double* __restrict__ thick,
+                             const unsigned char* __restrict__ active) {
     GridP g;
     double r = sqrt(dHat2[i]) + thick[i];
     double h = cell[i];
@@ -76,7 +82,22 @@ __global__ void k_grid_params(int nI, const unsigned long long* __restrict__ bb,
     for (int d = 0; d < 3; ++d) g.n[d] = (int)floor(ext[d] * g.inv) + 1;
     g.s1 = (long)g.n[0] + 1;
     g.s2 = g.s1 * ((long)g.n[1] + 1);
-    gp[i] = g;
+    g.coarse = 1;
+    g.ext = (float)fmax(ext[0], fmax(ext[1], ext[2]));
+    return g;
+}
+
+// grid parameters of every instance and, when cbase is given, the cell bases
+// (one CTA: a launch of its own took longer than the work)
+__global__ void k_grid_params(int nI, const unsigned long long* __restrict__ bb, const double* __restrict__ cell,
+                              const double* __restrict__ dHat2, const double* __restrict__ thick,
+                              const unsigned char* __restrict__ active, GridP* __restrict__ gp,
+                              uint32_t* __restrict__ cbase, unsigned long long* __restrict__ total,
+                              unsigned long long cap, unsigned int* __restrict__ flag) {
+    for (int i = threadIdx.x; i < nI; i += blockDim.x) gp[i] = grid_params(i, bb, cell, dHat2, thick, active);
+    if (!cbase) return;
+    __syncthreads();
+    cta_cell_bases(nI, gp, cbase, total, cap, flag);
 }
 
 __device__ __forceinline__ void vox3(const GridP& g, D3 p, int o[3]) {
@@ -86,19 +107,9 @@ __device__ __forceinline__ void vox3(const GridP& g, D3 p, int o[3]) {
 }
 
 template <int K>
-__global__ void k_prim_boxes(long n, const int* __restrict__ verts, const int* __restrict__ pinst,
-                             const unsigned char* __restrict__ active, const double* __restrict__ X,
-                             const GridP* __restrict__ gp, BoxI* __restrict__ boxes) {
-    long i = (long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    int inst = pinst[i];
+__device__ __forceinline__ BoxI prim_box(const int* __restrict__ verts, long i, const double* __restrict__ X,
+                                         const GridP& g) {
     BoxI b;
-    if (!active[inst]) {
-        for (int d = 0; d < 3; ++d) { b.lo[d] = 1; b.hi[d] = 0; }
-        boxes[i] = b;
-        return;
-    }
-    GridP g = gp[inst];
     int o[3];
     vox3(g, ld3(X, verts[K * i]), o);
     for (int d = 0; d < 3; ++d) b.lo[d] = b.hi[d] = o[d];
@@ -109,7 +120,30 @@ __global__ void k_prim_boxes(long n, const int* __restrict__ verts, const int* _
             b.hi[d] = max(b.hi[d], o[d]);
         }
     }
-    boxes[i] = b;
+    return b;
+}
+
+// integer boxes of the surface triangles [0, nt) and edges [nt, nt + ne), and
+// their cells counted in the table of each kind (ccount null: boxes only)
+__global__ void k_prim_boxes(long nt, long ne, const int* __restrict__ tris, const int* __restrict__ edges,
+                             const int* __restrict__ tinst, const int* __restrict__ einst,
+                             const unsigned char* __restrict__ active, const double* __restrict__ X,
+                             const GridP* __restrict__ gp, BoxI* __restrict__ tbox, BoxI* __restrict__ ebox,
+                             const uint32_t* __restrict__ cbase, uint32_t cap, uint32_t* __restrict__ ccount) {
+    const long i = (long)blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= nt + ne) return;
+    const bool tri = i < nt;
+    const int inst = tri ? tinst[i] : einst[i - nt];
+    BoxI b;
+    if (!active[inst]) {
+        for (int d = 0; d < 3; ++d) { b.lo[d] = 1; b.hi[d] = 0; }
+    } else {
+        const GridP g = gp[inst];
+        b = tri ? prim_box<3>(tris, i, X, g) : prim_box<2>(edges, i - nt, X, g);
+        if (ccount) count_cells(b, g, cbase[inst], cap, ccount + (tri ? 0 : (size_t)cap + 1));
+    }
+    if (tri) tbox[i] = b;
+    else ebox[i - nt] = b;
 }
 
 // ---- generic grid build
@@ -182,17 +216,7 @@ __global__ void k_dense_count2(long nt, long ne, const BoxI* __restrict__ tbox, 
     BoxI b;
     int inst, grid;
     if (!dense2_box(i, nt, tbox, tinst, ebox, einst, active, b, inst, grid)) return;
-    const GridP g = gp[inst];
-    const uint32_t c0 = cbase[inst];
-    uint32_t* cnt = ccount + (size_t)grid * (cap + 1);
-    const int zl = max(b.lo[2], 0), zh = min(b.hi[2], g.n[2]), yl = max(b.lo[1], 0), yh = min(b.hi[1], g.n[1]);
-    const int xl = max(b.lo[0], 0), xh = min(b.hi[0], g.n[0]);
-    for (int z = zl; z <= zh; ++z)
-        for (int y = yl; y <= yh; ++y)
-            for (int x = xl; x <= xh; ++x) {
-                const uint32_t c = c0 + (uint32_t)((long)x + (long)y * g.s1 + (long)z * g.s2);
-                if (c < cap) atomicAdd(cnt + c, 1u);
-            }
+    count_cells(b, gp[inst], cbase[inst], cap, ccount + (size_t)grid * (cap + 1));
 }
 
 __global__ void k_dense_fill2(long nt, long ne, const BoxI* __restrict__ tbox, const int* __restrict__ tinst,
@@ -300,16 +324,14 @@ struct Cand {
 };
 
 // one lane group per surface node: triangles within the +-dHat box (IPC.h:158-196)
-__global__ void k_query_pt(long nN, const int* __restrict__ nodes, const int* __restrict__ ninst,
-                           const unsigned char* __restrict__ active, const double* __restrict__ X,
-                           const unsigned char* __restrict__ dbc, const int* __restrict__ tris,
-                           const BoxI* __restrict__ tbox, const GridP* __restrict__ gp,
-                           const double* __restrict__ dHat2, const double* __restrict__ thick,
-                           CellHash cells, const uint32_t* __restrict__ cstart,
-                           const uint32_t* __restrict__ entries, Cand* __restrict__ out, unsigned int* counter,
-                           long cap) {
-    long s = ((long)blockIdx.x * blockDim.x + threadIdx.x) / kQueryLanes;
-    if (s >= nN) return;  // the whole group leaves together
+__device__ __forceinline__ void query_pt(long s, const int* __restrict__ nodes, const int* __restrict__ ninst,
+                                         const unsigned char* __restrict__ active, const double* __restrict__ X,
+                                         const float4* __restrict__ Xf, const unsigned char* __restrict__ dbc,
+                                         const int* __restrict__ tris, const BoxI* __restrict__ tbox,
+                                         const GridP* __restrict__ gp, const double* __restrict__ dHat2,
+                                         const double* __restrict__ thick, const CellHash& cells,
+                                         const uint32_t* __restrict__ cstart, const uint32_t* __restrict__ entries,
+                                         Cand* __restrict__ out, unsigned int* counter, long cap) {
     int inst = ninst[s];
     if (!active[inst]) return;
     int vI = nodes[s];
@@ -322,7 +344,8 @@ __global__ void k_query_pt(long nN, const int* __restrict__ nodes, const int* __
     vox3(g, mk3(p.x + rq, p.y + rq, p.z + rq), hi);
     BoxI qb;
     for (int d = 0; d < 3; ++d) { qb.lo[d] = lo[d]; qb.hi[d] = hi[d]; }
-    const double pp[3] = {p.x, p.y, p.z};
+    const F3 pf = ldf(Xf, vI);
+    const float lim = (float)r * 1.000001f + kFarMargin * g.ext;
     const bool pdbc = dbc[vI] != 0;
     group_walk_emit<kQueryLanes>(qb, inst, g, cells, cstart, entries, out, counter, cap,
                    [&](uint32_t ent, int cx, int cy, int cz, Cand& c) -> bool {
@@ -330,27 +353,22 @@ __global__ void k_query_pt(long nN, const int* __restrict__ nodes, const int* __
                        if (!is_first_shared(qb, tbox[f], cx, cy, cz)) return false;
                        int t0 = tris[3 * f], t1 = tris[3 * f + 1], t2 = tris[3 * f + 2];
                        if (vI == t0 || vI == t1 || vI == t2) return false;
+                       if (far_point_triangle(pf, ldf(Xf, t0), ldf(Xf, t1), ldf(Xf, t2), lim)) return false;
                        if (pdbc && dbc[t0] && dbc[t1] && dbc[t2]) return false;
-                       D3 a = ld3(X, t0), b = ld3(X, t1), cc = ld3(X, t2);
-                       double mx[3] = {fmax(fmax(a.x, b.x), cc.x), fmax(fmax(a.y, b.y), cc.y), fmax(fmax(a.z, b.z), cc.z)};
-                       double mn[3] = {fmin(fmin(a.x, b.x), cc.x), fmin(fmin(a.y, b.y), cc.y), fmin(fmin(a.z, b.z), cc.z)};
-                       for (int d = 0; d < 3; ++d)
-                           if (pp[d] - mx[d] > r || mn[d] - pp[d] > r) return false;
                        c = {(int)s, f};
                        return true;
                    });
 }
 
 // one lane group per surface edge: edges eJ > eI within the +-dHat box (IPC.h:371-420)
-__global__ void k_query_ee(long nE, const int2* __restrict__ edges, const int* __restrict__ einst,
-                           const unsigned char* __restrict__ active, const double* __restrict__ X,
-                           const unsigned char* __restrict__ dbc, const BoxI* __restrict__ ebox,
-                           const GridP* __restrict__ gp, const double* __restrict__ dHat2,
-                           const double* __restrict__ thick, CellHash cells,
-                           const uint32_t* __restrict__ cstart, const uint32_t* __restrict__ entries,
-                           Cand* __restrict__ out, unsigned int* counter, long cap) {
-    long eI = ((long)blockIdx.x * blockDim.x + threadIdx.x) / kQueryLanes;
-    if (eI >= nE) return;
+__device__ __forceinline__ void query_ee(long eI, const int2* __restrict__ edges, const int* __restrict__ einst,
+                                         const unsigned char* __restrict__ active, const double* __restrict__ X,
+                                         const float4* __restrict__ Xf, const unsigned char* __restrict__ dbc,
+                                         const BoxI* __restrict__ ebox, const GridP* __restrict__ gp,
+                                         const double* __restrict__ dHat2, const double* __restrict__ thick,
+                                         const CellHash& cells, const uint32_t* __restrict__ cstart,
+                                         const uint32_t* __restrict__ entries, Cand* __restrict__ out,
+                                         unsigned int* counter, long cap) {
     int inst = einst[eI];
     if (!active[inst]) return;
     int2 mi = edges[eI];
@@ -363,8 +381,8 @@ __global__ void k_query_ee(long nE, const int2* __restrict__ edges, const int* _
     vox3(g, mk3(fmax(a0.x, a1.x) + rq, fmax(a0.y, a1.y) + rq, fmax(a0.z, a1.z) + rq), hi);
     BoxI qb;
     for (int d = 0; d < 3; ++d) { qb.lo[d] = lo[d]; qb.hi[d] = hi[d]; }
-    const double amax[3] = {fmax(a0.x, a1.x), fmax(a0.y, a1.y), fmax(a0.z, a1.z)};
-    const double amin[3] = {fmin(a0.x, a1.x), fmin(a0.y, a1.y), fmin(a0.z, a1.z)};
+    const F3 f0 = ldf(Xf, mi.x), f1 = ldf(Xf, mi.y);
+    const float lim = (float)r * 1.000001f + kFarMargin * g.ext;
     const bool adbc = dbc[mi.x] && dbc[mi.y];
     group_walk_emit<kQueryLanes>(qb, inst, g, cells, cstart, entries, out, counter, cap,
                    [&](uint32_t ent, int cx, int cy, int cz, Cand& c) -> bool {
@@ -372,15 +390,36 @@ __global__ void k_query_ee(long nE, const int2* __restrict__ edges, const int* _
                        if (eJ <= eI || !is_first_shared(qb, ebox[eJ], cx, cy, cz)) return false;
                        int2 mj = edges[eJ];
                        if (mi.x == mj.x || mi.x == mj.y || mi.y == mj.x || mi.y == mj.y) return false;
+                       if (far_segments(f0, f1, ldf(Xf, mj.x), ldf(Xf, mj.y), lim)) return false;
                        if (adbc && dbc[mj.x] && dbc[mj.y]) return false;
-                       D3 b0 = ld3(X, mj.x), b1 = ld3(X, mj.y);
-                       double bmax[3] = {fmax(b0.x, b1.x), fmax(b0.y, b1.y), fmax(b0.z, b1.z)};
-                       double bmin[3] = {fmin(b0.x, b1.x), fmin(b0.y, b1.y), fmin(b0.z, b1.z)};
-                       for (int d = 0; d < 3; ++d)
-                           if (amin[d] - bmax[d] > r || bmin[d] - amax[d] > r) return false;
                        c = {(int)eI, eJ};
                        return true;
                    });
+}
+
+// both queries in one launch: the first bpt CTAs take the nodes, the others
+// the edges. Bound by latency (chains of dependent L2 loads per table row); the
+// FP32 bound keeps nearly every pair beyond d-hat out of the FP64 phase (on a
+// surface without contact, all of them).
+__global__ void k_query(unsigned int bpt, long nN, const int* __restrict__ nodes, const int* __restrict__ ninst,
+                        long nE, const int2* __restrict__ edges, const int* __restrict__ einst,
+                        const unsigned char* __restrict__ active, const double* __restrict__ X,
+                        const float4* __restrict__ Xf, const unsigned char* __restrict__ dbc,
+                        const int* __restrict__ tris, const BoxI* __restrict__ tbox, const BoxI* __restrict__ ebox,
+                        const GridP* __restrict__ gp, const double* __restrict__ dHat2,
+                        const double* __restrict__ thick, CellHash tcells, const uint32_t* __restrict__ tstart,
+                        const uint32_t* __restrict__ tentries, CellHash ecells, const uint32_t* __restrict__ estart,
+                        const uint32_t* __restrict__ eentries, Cand* __restrict__ out, unsigned int* counter,
+                        long cap_pt, long cap_ee) {
+    const bool pt = blockIdx.x < bpt;
+    const long q = ((long)(blockIdx.x - (pt ? 0u : bpt)) * blockDim.x + threadIdx.x) / kQueryLanes;
+    if (q >= (pt ? nN : nE)) return;  // the whole group leaves together
+    if (pt)
+        query_pt(q, nodes, ninst, active, X, Xf, dbc, tris, tbox, gp, dHat2, thick, tcells, tstart, tentries, out,
+                 counter, cap_pt);
+    else
+        query_ee(q, edges, einst, active, X, Xf, dbc, ebox, gp, dHat2, thick, ecells, estart, eentries, out + cap_pt,
+                 counter + 1, cap_ee);
 }
 
 // ---- narrow phase
@@ -389,85 +428,110 @@ struct Rec {
     int inst;
 };
 
-__global__ void k_narrow_pt(long K, const Cand* __restrict__ cand, const int* __restrict__ nodes,
-                            const int* __restrict__ ninst, const int* __restrict__ tris,
-                            const double* __restrict__ X, const double* __restrict__ dHat2,
-                            const double* __restrict__ thick, Rec* __restrict__ out, unsigned int* counter,
-                            long cap) {
-    long k = (long)blockIdx.x * blockDim.x + threadIdx.x;
-    bool emit = false;
-    Rec rec;
-    rec.c = make_int4(0, 0, 0, 0);
-    rec.inst = 0;
-    if (k < K) {
-        Cand cd = cand[k];
-        int vI = nodes[cd.a], inst = ninst[cd.a];
-        int t0 = tris[3 * cd.b], t1 = tris[3 * cd.b + 1], t2 = tris[3 * cd.b + 2];
-        D3 p = ld3(X, vI), a = ld3(X, t0), b = ld3(X, t1), c = ld3(X, t2);
-        double r = sqrt(dHat2[inst]) + thick[inst];
-        double r2 = r * r;
-        double d;
-        int4 cc;
-        switch (type_PT(p, a, b, c)) {
-            case 0: d = d_PP(p, a); cc = make_int4(-vI - 1, t0, -1, -1); break;
-            case 1: d = d_PP(p, b); cc = make_int4(-vI - 1, t1, -1, -1); break;
-            case 2: d = d_PP(p, c); cc = make_int4(-vI - 1, t2, -1, -1); break;
-            case 3: d = d_PE(p, a, b); cc = make_int4(-vI - 1, t0, t1, -1); break;
-            case 4: d = d_PE(p, b, c); cc = make_int4(-vI - 1, t1, t2, -1); break;
-            case 5: d = d_PE(p, c, a); cc = make_int4(-vI - 1, t2, t0, -1); break;
-            default: d = d_PT(p, a, b, c); cc = make_int4(-vI - 1, t0, t1, t2); break;
-        }
-        if (d < r2) {
-            emit = true;
-            rec.c = cc;
-            rec.inst = inst;
-        }
+__device__ __forceinline__ bool narrow_pt(Cand cd, const int* __restrict__ nodes, const int* __restrict__ ninst,
+                                          const int* __restrict__ tris, const double* __restrict__ X,
+                                          const double* __restrict__ dHat2, const double* __restrict__ thick, Rec& rec) {
+    int vI = nodes[cd.a], inst = ninst[cd.a];
+    int t0 = tris[3 * cd.b], t1 = tris[3 * cd.b + 1], t2 = tris[3 * cd.b + 2];
+    D3 p = ld3(X, vI), a = ld3(X, t0), b = ld3(X, t1), c = ld3(X, t2);
+    double r = sqrt(dHat2[inst]) + thick[inst];
+    const double pp[3] = {p.x, p.y, p.z};
+    double mx[3] = {fmax(fmax(a.x, b.x), c.x), fmax(fmax(a.y, b.y), c.y), fmax(fmax(a.z, b.z), c.z)};
+    double mn[3] = {fmin(fmin(a.x, b.x), c.x), fmin(fmin(a.y, b.y), c.y), fmin(fmin(a.z, b.z), c.z)};
+    for (int d = 0; d < 3; ++d)
+        if (pp[d] - mx[d] > r || mn[d] - pp[d] > r) return false;
+    double r2 = r * r;
+    double d;
+    int4 cc;
+    switch (type_PT(p, a, b, c)) {
+        case 0: d = d_PP(p, a); cc = make_int4(-vI - 1, t0, -1, -1); break;
+        case 1: d = d_PP(p, b); cc = make_int4(-vI - 1, t1, -1, -1); break;
+        case 2: d = d_PP(p, c); cc = make_int4(-vI - 1, t2, -1, -1); break;
+        case 3: d = d_PE(p, a, b); cc = make_int4(-vI - 1, t0, t1, -1); break;
+        case 4: d = d_PE(p, b, c); cc = make_int4(-vI - 1, t1, t2, -1); break;
+        case 5: d = d_PE(p, c, a); cc = make_int4(-vI - 1, t2, t0, -1); break;
+        default: d = d_PT(p, a, b, c); cc = make_int4(-vI - 1, t0, t1, t2); break;
     }
-    group_emit<32>(emit, rec, out, counter, cap);
+    rec.c = cc;
+    rec.inst = inst;
+    return d < r2;
 }
 
-__global__ void k_narrow_ee(long K, const Cand* __restrict__ cand, const int2* __restrict__ edges,
-                            const int* __restrict__ einst, const double* __restrict__ X,
-                            const double* __restrict__ X0, const double* __restrict__ dHat2,
-                            const double* __restrict__ thick, Rec* __restrict__ out, unsigned int* counter,
-                            long cap) {
-    long k = (long)blockIdx.x * blockDim.x + threadIdx.x;
-    bool emit = false;
-    Rec rec;
-    rec.c = make_int4(0, 0, 0, 0);
-    rec.inst = 0;
-    if (k < K) {
-        Cand cd = cand[k];
-        int2 mi = edges[cd.a], mj = edges[cd.b];
-        int inst = einst[cd.a];
-        int a0 = mi.x, a1 = mi.y, b0 = mj.x, b1 = mj.y;
-        D3 ea0 = ld3(X, a0), ea1 = ld3(X, a1), eb0 = ld3(X, b0), eb1 = ld3(X, b1);
-        double r = sqrt(dHat2[inst]) + thick[inst];
-        double r2 = r * r;
-        double cn = ee_cross_norm2(ea0, ea1, eb0, eb1);
-        double eps_x = mollifier_threshold(ld3(X0, a0), ld3(X0, a1), ld3(X0, b0), ld3(X0, b1));
-        bool mol = cn < eps_x;
-        double d;
-        int4 c;
-        switch (type_EE(ea0, ea1, eb0, eb1)) {
-            case 0: d = d_PP(ea0, eb0); c = mol ? make_int4(a0, b0, -a1 - 1, -b1 - 1) : make_int4(-a0 - 1, b0, -1, -1); break;
-            case 1: d = d_PP(ea0, eb1); c = mol ? make_int4(a0, b1, -a1 - 1, -b0 - 1) : make_int4(-a0 - 1, b1, -1, -1); break;
-            case 2: d = d_PE(ea0, eb0, eb1); c = mol ? make_int4(a0, b0, b1, -a1 - 1) : make_int4(-a0 - 1, b0, b1, -1); break;
-            case 3: d = d_PP(ea1, eb0); c = mol ? make_int4(a1, b0, -a0 - 1, -b1 - 1) : make_int4(-a1 - 1, b0, -1, -1); break;
-            case 4: d = d_PP(ea1, eb1); c = mol ? make_int4(a1, b1, -a0 - 1, -b0 - 1) : make_int4(-a1 - 1, b1, -1, -1); break;
-            case 5: d = d_PE(ea1, eb0, eb1); c = mol ? make_int4(a1, b0, b1, -a0 - 1) : make_int4(-a1 - 1, b0, b1, -1); break;
-            case 6: d = d_PE(eb0, ea0, ea1); c = mol ? make_int4(b0, a0, a1, -b1 - 1) : make_int4(-b0 - 1, a0, a1, -1); break;
-            case 7: d = d_PE(eb1, ea0, ea1); c = mol ? make_int4(b1, a0, a1, -b0 - 1) : make_int4(-b1 - 1, a0, a1, -1); break;
-            default: d = d_EE(ea0, ea1, eb0, eb1); c = mol ? make_int4(a0, a1, -b0 - 1, b1) : make_int4(a0, a1, b0, b1); break;
-        }
-        if (d < r2) {
-            emit = true;
-            rec.c = c;
-            rec.inst = inst;
-        }
+__device__ __forceinline__ bool narrow_ee(Cand cd, const int2* __restrict__ edges, const int* __restrict__ einst,
+                                          const double* __restrict__ X, const double* __restrict__ X0,
+                                          const double* __restrict__ dHat2, const double* __restrict__ thick, Rec& rec) {
+    int2 mi = edges[cd.a], mj = edges[cd.b];
+    int inst = einst[cd.a];
+    int a0 = mi.x, a1 = mi.y, b0 = mj.x, b1 = mj.y;
+    D3 ea0 = ld3(X, a0), ea1 = ld3(X, a1), eb0 = ld3(X, b0), eb1 = ld3(X, b1);
+    double r = sqrt(dHat2[inst]) + thick[inst];
+    const double amax[3] = {fmax(ea0.x, ea1.x), fmax(ea0.y, ea1.y), fmax(ea0.z, ea1.z)};
+    const double amin[3] = {fmin(ea0.x, ea1.x), fmin(ea0.y, ea1.y), fmin(ea0.z, ea1.z)};
+    const double bmax[3] = {fmax(eb0.x, eb1.x), fmax(eb0.y, eb1.y), fmax(eb0.z, eb1.z)};
+    const double bmin[3] = {fmin(eb0.x, eb1.x), fmin(eb0.y, eb1.y), fmin(eb0.z, eb1.z)};
+    for (int d = 0; d < 3; ++d)
+        if (amin[d] - bmax[d] > r || bmin[d] - amax[d] > r) return false;
+    double r2 = r * r;
+    const int type = type_EE(ea0, ea1, eb0, eb1);
+    double d;
+    switch (type) {
+        case 0: d = d_PP(ea0, eb0); break;
+        case 1: d = d_PP(ea0, eb1); break;
+        case 2: d = d_PE(ea0, eb0, eb1); break;
+        case 3: d = d_PP(ea1, eb0); break;
+        case 4: d = d_PP(ea1, eb1); break;
+        case 5: d = d_PE(ea1, eb0, eb1); break;
+        case 6: d = d_PE(eb0, ea0, ea1); break;
+        case 7: d = d_PE(eb1, ea0, ea1); break;
+        default: d = d_EE(ea0, ea1, eb0, eb1); break;
     }
-    group_emit<32>(emit, rec, out, counter, cap);
+    if (!(d < r2)) return false;
+    double cn = ee_cross_norm2(ea0, ea1, eb0, eb1);
+    double eps_x = mollifier_threshold(ld3(X0, a0), ld3(X0, a1), ld3(X0, b0), ld3(X0, b1));
+    bool mol = cn < eps_x;
+    int4 c;
+    switch (type) {
+        case 0: c = mol ? make_int4(a0, b0, -a1 - 1, -b1 - 1) : make_int4(-a0 - 1, b0, -1, -1); break;
+        case 1: c = mol ? make_int4(a0, b1, -a1 - 1, -b0 - 1) : make_int4(-a0 - 1, b1, -1, -1); break;
+        case 2: c = mol ? make_int4(a0, b0, b1, -a1 - 1) : make_int4(-a0 - 1, b0, b1, -1); break;
+        case 3: c = mol ? make_int4(a1, b0, -a0 - 1, -b1 - 1) : make_int4(-a1 - 1, b0, -1, -1); break;
+        case 4: c = mol ? make_int4(a1, b1, -a0 - 1, -b0 - 1) : make_int4(-a1 - 1, b1, -1, -1); break;
+        case 5: c = mol ? make_int4(a1, b0, b1, -a0 - 1) : make_int4(-a1 - 1, b0, b1, -1); break;
+        case 6: c = mol ? make_int4(b0, a0, a1, -b1 - 1) : make_int4(-b0 - 1, a0, a1, -1); break;
+        case 7: c = mol ? make_int4(b1, a0, a1, -b0 - 1) : make_int4(-b1 - 1, a0, a1, -1); break;
+        default: c = mol ? make_int4(a0, a1, -b0 - 1, b1) : make_int4(a0, a1, b0, b1); break;
+    }
+    rec.c = c;
+    rec.inst = inst;
+    return true;
 }
+
+// the candidates of both lists; their numbers come from the device (clamped to
+// the capacities: an overflowing build is redone by the caller), so no host
+// round trip lies between the queries and this
+__global__ void k_narrow(const unsigned int* __restrict__ counts, long cap_pt, long cap_ee, const Cand* __restrict__ cand,
+                         const int* __restrict__ nodes, const int* __restrict__ ninst, const int* __restrict__ tris,
+                         const int2* __restrict__ edges, const int* __restrict__ einst, const double* __restrict__ X,
+                         const double* __restrict__ X0, const double* __restrict__ dHat2,
+                         const double* __restrict__ thick, Rec* __restrict__ out, unsigned int* counter, long cap) {
+    const long npt = min((long)counts[0], cap_pt), nee = min((long)counts[1], cap_ee);
+    // each list in whole warps, so that a warp takes one kind
+    const long wpt = (npt + 31) & ~31L, total = wpt + nee;
+    for (long k0 = (long)blockIdx.x * blockDim.x; k0 < total; k0 += (long)gridDim.x * blockDim.x) {
+        const long k = k0 + threadIdx.x;
+        Rec rec;
+        rec.c = make_int4(0, 0, 0, 0);
+        rec.inst = 0;
+        bool emit = false;
+        if (k < wpt) {
+            if (k < npt) emit = narrow_pt(cand[k], nodes, ninst, tris, X, dHat2, thick, rec);
+        } else if (k < total) {
+            emit = narrow_ee(cand[cap_pt + k - wpt], edges, einst, X, X0, dHat2, thick, rec);
+        }
+        group_emit<32>(emit, rec, out, counter, cap);
+    }
+}
+constexpr int kNarrowBlocks = 4 * 152;
 
 // ---- sort + merge
 __global__ void k_rec_keys(long n, const Rec* __restrict__ recs, int b, int off, uint64_t* __restrict__ klo,
@@ -706,7 +770,7 @@ bool grids_overflowed(Work& W, int set, unsigned int flag) {
 
 int grids_build(Work& W, int set, const BoxI* tbox, long nt, const int* tinst, const BoxI* ebox, long ne,
                 const int* einst, const unsigned char* active, const GridP* gp, int nI, unsigned int* d_flag,
-                BoxGrid& gt, BoxGrid& ge, cudaStream_t s) {
+                BoxGrid& gt, BoxGrid& ge, cudaStream_t s, bool counted) {
     if (W[W_CBASE].ensure(sizeof(uint32_t) * (nI + 1) + 64)) return IDP_ERR_CUDA;
     uint32_t* cbase = W[W_CBASE].as<uint32_t>();
     unsigned long long* d_total = reinterpret_cast<unsigned long long*>(W[W_CBASE].as<char>() +
@@ -723,10 +787,12 @@ int grids_build(Work& W, int set, const BoxI* tbox, long nt, const int* tinst, c
             return IDP_ERR_CUDA;
         uint32_t* ccount = tab.as<uint32_t>();
         uint32_t* cstart = ccount + slots + 1;
-        (::idp::count_launch(), k_cell_bases<<<1, 1, 0, s>>>(nI, gp, cbase, d_total, cap, d_flag));
-        IDP_CUDA_TRY(cudaMemsetAsync(ccount, 0, sizeof(uint32_t) * slots, s));
         const long n = nt + ne;
-        if (n > 0)
+        if (!counted) {
+            (::idp::count_launch(), k_cell_bases<<<1, 1, 0, s>>>(nI, gp, cbase, d_total, cap, d_flag));
+            IDP_CUDA_TRY(cudaMemsetAsync(ccount, 0, sizeof(uint32_t) * slots, s));
+        }
+        if (n > 0 && !counted)
             (::idp::count_launch(), k_dense_count2<<<grid_for(n), kBlock, 0, s>>>(nt, ne, tbox, tinst, ebox, einst, active,
                                                                                   gp, cbase, (uint32_t)cap, ccount));
         if (scan_exclusive(ccount, cstart, (long)slots, cstart + slots, W[W_SCRATCH].p, s) != cudaSuccess)
@@ -769,37 +835,60 @@ int grids_build(Work& W, int set, const BoxI* tbox, long nt, const int* tinst, c
     return IDP_OK;
 }
 
+int grids_tables(Work& W, int set, int nI, GridTables& t, cudaStream_t s) {
+    t = GridTables();
+    if (!W.dense_ready[set]) return IDP_OK;
+    const size_t slots = 2 * (size_t)(W.dense_cells_cap[set] + 1);
+    DBuf& tab = W[set ? W_DENSE1 : W_DENSE0];
+    if (W[W_CBASE].ensure(sizeof(uint32_t) * (nI + 1) + 64) || tab.ensure(sizeof(uint32_t) * (2 * slots + 2)))
+        return IDP_ERR_CUDA;
+    t.ccount = tab.as<uint32_t>();
+    t.cbase = W[W_CBASE].as<uint32_t>();
+    t.total = reinterpret_cast<unsigned long long*>(W[W_CBASE].as<char>() +
+                                                    ((sizeof(uint32_t) * (nI + 1) + 15) & ~size_t(15)));
+    t.cap = (uint32_t)W.dense_cells_cap[set];
+    IDP_CUDA_TRY(cudaMemsetAsync(t.ccount, 0, sizeof(uint32_t) * slots, s));
+    return IDP_OK;
+}
+
 // per-instance grid over the surface at X and the integer boxes of every
-// surface triangle and edge in it
-static int surface_boxes(Arena& A, Work& W, const double* X, GridP*& gp, BoxI*& tbox, BoxI*& ebox, cudaStream_t s) {
+// surface triangle and edge in it; when the tables' capacities are known the
+// cells are counted on the way (counted, d_flag as in grids_build). The FP32
+// positions go to W_XF.
+static int surface_boxes(Arena& A, Work& W, const double* X, GridP*& gp, BoxI*& tbox, BoxI*& ebox,
+                         unsigned int* d_flag, bool& counted, cudaStream_t s) {
     const int nI = A.nI;
     if (W[W_BBOX].ensure(sizeof(unsigned long long) * 6 * nI) || W[W_GRIDP].ensure(sizeof(GridP) * nI))
         return IDP_ERR_CUDA;
     unsigned long long* bb = W[W_BBOX].as<unsigned long long>();
     gp = W[W_GRIDP].as<GridP>();
+    GridTables t;
+    if (int r = grids_tables(W, 0, nI, t, s)) return r;
+    counted = t.ccount != nullptr;
+    if (W[W_XF].ensure(sizeof(float4) * (A.V + 1))) return IDP_ERR_CUDA;
+    float4* Xf = W[W_XF].as<float4>();
     (::idp::count_launch(), k_bbox_init<<<grid_for(6 * nI), kBlock, 0, s>>>(nI, bb));
-    if (A.Sn) (::idp::count_launch(), k_bbox<<<grid_for(A.Sn), kBlock, 0, s>>>(A.Sn, A.snode, A.sn_inst, A.active, X, bb));
-    (::idp::count_launch(), k_grid_params<<<grid_for(nI), kBlock, 0, s>>>(nI, bb, A.cell, A.dHat2, A.thickness, A.active, gp));
+    if (A.Sn)
+        (::idp::count_launch(), k_bbox<<<grid_for(A.Sn), kBlock, 0, s>>>(A.Sn, A.snode, A.sn_inst, A.active, X, A.d_sn_off,
+                                                                         bb, Xf));
+    (::idp::count_launch(), k_grid_params<<<1, kBlock, 0, s>>>(nI, bb, A.cell, A.dHat2, A.thickness, A.active, gp, t.cbase,
+                                                               t.total, t.cap, d_flag));
     long St = A.St > 0 ? A.St : 1, Se = A.Se > 0 ? A.Se : 1;
     if (W[W_BOX_A].ensure(sizeof(BoxI) * St) || W[W_BOX_B].ensure(sizeof(BoxI) * Se)) return IDP_ERR_CUDA;
     tbox = W[W_BOX_A].as<BoxI>();
     ebox = W[W_BOX_B].as<BoxI>();
-    if (A.St) (::idp::count_launch(), k_prim_boxes<3><<<grid_for(A.St), kBlock, 0, s>>>(A.St, A.stri, A.st_inst, A.active, X, gp, tbox));
-    if (A.Se)
-        (::idp::count_launch(), k_prim_boxes<2><<<grid_for(A.Se), kBlock, 0, s>>>(A.Se, reinterpret_cast<const int*>(A.sedge), A.se_inst,
-                                                           A.active, X, gp, ebox));
+    if (A.St + A.Se)
+        (::idp::count_launch(), k_prim_boxes<<<grid_for(A.St + A.Se), kBlock, 0, s>>>(
+                                    A.St, A.Se, A.stri, reinterpret_cast<const int*>(A.sedge), A.st_inst, A.se_inst,
+                                    A.active, X, gp, tbox, ebox, t.cbase, t.cap, t.ccount));
     return IDP_OK;
 }
 
 int build_constraint_set(Arena& A, Work& W, const double* X, ContactSet& cs, cudaStream_t s) {
     const int nI = A.nI;
-    // 1-2. per-instance grid parameters, triangle and edge boxes
-    GridP* gp = nullptr;
-    BoxI *tbox = nullptr, *ebox = nullptr;
-    if (int r = surface_boxes(A, W, X, gp, tbox, ebox, s)) return r;
-    // 3. grids and candidates: PT in [0, cap_pt), EE in [cap_pt, cap_pt +
-    // cap_ee); one host round trip reads both counts and the grids' overflow
-    // flag (ccount[2])
+    // grids, candidates (PT in [0, cap_pt), EE in [cap_pt, cap_pt + cap_ee)) and
+    // records; one host round trip reads the candidate counts, the grids'
+    // overflow flag (ccount[2]) and the number of records (ccount[3])
     uint32_t* hp = W.pinned();
     if (!hp) return IDP_ERR_CUDA;
     if (W[W_CAND_CNT].ensure(64)) return IDP_ERR_CUDA;
@@ -808,22 +897,33 @@ int build_constraint_set(Arena& A, Work& W, const double* X, ContactSet& cs, cud
     long cap_ee = std::max<long>(W.cand_cap_ee, 2 * A.Se + 512);
     int rc = IDP_OK;
     for (int attempt = 0; attempt < 6; ++attempt) {
+        // 1-2. per-instance grid parameters, triangle and edge boxes
+        GridP* gp = nullptr;
+        BoxI *tbox = nullptr, *ebox = nullptr;
+        bool counted = false;
+        IDP_CUDA_TRY(cudaMemsetAsync(ccount, 0, 4 * sizeof(unsigned int), s));
+        if ((rc = surface_boxes(A, W, X, gp, tbox, ebox, ccount + 2, counted, s))) return rc;
         BoxGrid gt, ge;
-        IDP_CUDA_TRY(cudaMemsetAsync(ccount, 0, 3 * sizeof(unsigned int), s));
         if ((rc = grids_build(W, 0, tbox, A.St, A.st_inst, ebox, A.Se, A.se_inst, A.active, gp, nI, ccount + 2, gt, ge,
-                              s)))
+                              s, counted)))
             return rc;
-        if (W[W_CAND].ensure(sizeof(Cand) * (cap_pt + cap_ee))) return IDP_ERR_CUDA;
+        const long rcap = cap_pt + cap_ee;
+        if (W[W_CAND].ensure(sizeof(Cand) * rcap) || W[W_CONS_TMP].ensure(sizeof(Rec) * rcap)) return IDP_ERR_CUDA;
         Cand* cand = W[W_CAND].as<Cand>();
-        if (A.Sn)
-            (::idp::count_launch(), k_query_pt<<<grid_for(kQueryLanes * A.Sn), kBlock, 0, s>>>(A.Sn, A.snode, A.sn_inst, A.active, X, A.dbc_excl, A.stri, tbox, gp,
-                                                         A.dHat2, A.thickness, gt.cells, gt.cell_start,
-                                                         gt.entries, cand, ccount, cap_pt));
-        if (A.Se)
-            (::idp::count_launch(), k_query_ee<<<grid_for(kQueryLanes * A.Se), kBlock, 0, s>>>(A.Se, A.sedge, A.se_inst, A.active, X, A.dbc_excl, ebox, gp, A.dHat2,
-                                                         A.thickness, ge.cells, ge.cell_start, ge.entries,
-                                                         cand + cap_pt, ccount + 1, cap_ee));
-        IDP_CUDA_TRY(cudaMemcpyAsync(hp + 2, ccount, 3 * sizeof(unsigned int), cudaMemcpyDeviceToHost, s));
+        Rec* recs = W[W_CONS_TMP].as<Rec>();
+        const int bpt = A.Sn ? grid_for(kQueryLanes * A.Sn) : 0, bee = A.Se ? grid_for(kQueryLanes * A.Se) : 0;
+        if (bpt + bee) {
+            (::idp::count_launch(), k_query<<<bpt + bee, kBlock, 0, s>>>(
+                                        (unsigned int)bpt, A.Sn, A.snode, A.sn_inst, A.Se, A.sedge, A.se_inst, A.active,
+                                        X, W[W_XF].as<float4>(), A.dbc_excl, A.stri, tbox, ebox, gp, A.dHat2,
+                                        A.thickness, gt.cells, gt.cell_start, gt.entries, ge.cells, ge.cell_start,
+                                        ge.entries, cand, ccount, cap_pt, cap_ee));
+            // 3. narrow phase
+            (::idp::count_launch(), k_narrow<<<kNarrowBlocks, 128, 0, s>>>(
+                                        ccount, cap_pt, cap_ee, cand, A.snode, A.sn_inst, A.stri, A.sedge, A.se_inst, X,
+                                        A.X0, A.dHat2, A.thickness, recs, ccount + 3, rcap));
+        }
+        IDP_CUDA_TRY(cudaMemcpyAsync(hp + 2, ccount, 4 * sizeof(unsigned int), cudaMemcpyDeviceToHost, s));
         IDP_CUDA_TRY(cudaStreamSynchronize(s));
         const long npt = hp[2], nee = hp[3];
         if (grids_overflowed(W, 0, hp[4])) continue;
@@ -834,7 +934,8 @@ int build_constraint_set(Arena& A, Work& W, const double* X, ContactSet& cs, cud
             W.cand_cap_ee = cap_ee;
             continue;
         }
-        if (npt + nee == 0) {
+        const unsigned int nrec = hp[5];
+        if (nrec == 0) {
             cs.C = 0;
             cs.off.assign(nI + 1, 0);
             if (W[W_CONS_OFF].ensure(sizeof(int) * (nI + 1)) || W[W_CONS].ensure(sizeof(int4)) ||
@@ -845,23 +946,6 @@ int build_constraint_set(Arena& A, Work& W, const double* X, ContactSet& cs, cud
             return IDP_OK;
         }
         {
-            // 4. narrow phase
-            long rcap = (long)(W[W_CONS_TMP].bytes / sizeof(Rec));
-            if (rcap < npt + nee + 1) {
-                rcap = npt + nee + 1;
-                if (W[W_CONS_TMP].ensure(sizeof(Rec) * rcap)) return IDP_ERR_CUDA;
-            }
-            Rec* recs = W[W_CONS_TMP].as<Rec>();
-            IDP_CUDA_TRY(cudaMemsetAsync(ccount, 0, sizeof(unsigned int), s));
-            if (npt)
-                (::idp::count_launch(), k_narrow_pt<<<grid_for(npt), kBlock, 0, s>>>(npt, cand, A.snode, A.sn_inst, A.stri, X, A.dHat2, A.thickness,
-                                                             recs, ccount, rcap));
-            if (nee)
-                (::idp::count_launch(), k_narrow_ee<<<grid_for(nee), kBlock, 0, s>>>(nee, cand + cap_pt, A.sedge, A.se_inst, X, A.X0, A.dHat2,
-                                                             A.thickness, recs, ccount, rcap));
-            unsigned int nrec = 0;
-            IDP_CUDA_TRY(cudaMemcpyAsync(&nrec, ccount, sizeof(unsigned int), cudaMemcpyDeviceToHost, s));
-            IDP_CUDA_TRY(cudaStreamSynchronize(s));
             long n = nrec;
             // 5. sort by (inst, c0, c1, c2, c3) and merge PP/PE duplicates
             long na = n > 0 ? n : 1;
@@ -919,19 +1003,20 @@ int build_constraint_set(Arena& A, Work& W, const double* X, ContactSet& cs, cud
 int edge_tri_intersections(Arena& A, Work& W, const double* X, unsigned int* inst_count, const int2** pairs,
                            long* npairs, cudaStream_t s) {
     const int nI = A.nI;
-    GridP* gp = nullptr;
-    BoxI *tbox = nullptr, *ebox = nullptr;
-    if (int r = surface_boxes(A, W, X, gp, tbox, ebox, s)) return r;
     uint32_t* hp = W.pinned();
     if (!hp || W[W_CAND_CNT].ensure(64)) return IDP_ERR_CUDA;
     unsigned int* ccount = W[W_CAND_CNT].as<unsigned int>();
     long cap = std::max<long>(W.isect_cap, 1024);
     for (int attempt = 0; attempt < 6; ++attempt) {
+        GridP* gp = nullptr;
+        BoxI *tbox = nullptr, *ebox = nullptr;
         BoxGrid gt, ge;
+        bool counted = false;
         IDP_CUDA_TRY(cudaMemsetAsync(ccount, 0, 3 * sizeof(unsigned int), s));
         IDP_CUDA_TRY(cudaMemsetAsync(inst_count, 0, sizeof(unsigned int) * nI, s));
+        if (int r = surface_boxes(A, W, X, gp, tbox, ebox, ccount + 2, counted, s)) return r;
         if (int r = grids_build(W, 0, tbox, A.St, A.st_inst, ebox, A.Se, A.se_inst, A.active, gp, nI, ccount + 2, gt,
-                                ge, s))
+                                ge, s, counted))
             return r;
         if (W[W_CAND].ensure(sizeof(Cand) * cap)) return IDP_ERR_CUDA;
         Cand* out = W[W_CAND].as<Cand>();

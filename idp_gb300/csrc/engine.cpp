@@ -1727,13 +1727,11 @@ int step_iterate(idp_ctx* c, int max_iters, idp_result* results, int* n_active) 
         if ((rc = set_mask(c, mask))) return rc;
         IDP_CUDA_TRY(cudaMemcpyAsync(A.alpha, alpha.data(), sizeof(double) * nI, cudaMemcpyHostToDevice, s));
         W.timer.start(PhaseTimer::CCD, s);
-        rc = ccd_stepsize(A, W, A.Xprev, A.dir, A.alpha, isc(c, SI_CCDF), s, ccd_voxel_sizes(A, W));
+        hi.resize(nI);
+        rc = ccd_stepsize(A, W, A.Xprev, A.dir, A.alpha, isc(c, SI_CCDF), s, ccd_voxel_sizes(A, W), alpha.data(),
+                          hi.data());
         W.timer.stop(s);
         if (rc) return rc;
-        hi.resize(nI);
-        IDP_CUDA_TRY(cudaMemcpyAsync(alpha.data(), A.alpha, sizeof(double) * nI, cudaMemcpyDeviceToHost, s));
-        IDP_CUDA_TRY(cudaMemcpyAsync(hi.data(), isc(c, SI_CCDF), sizeof(int) * nI, cudaMemcpyDeviceToHost, s));
-        IDP_CUDA_TRY(cudaStreamSynchronize(s));
         std::vector<double> feasible = alpha;
         for (int i = 0; i < nI; ++i) {
             if (!mask[i]) continue;
@@ -2279,10 +2277,10 @@ int idp_ccd_stepsize(idp_ctx* c, int i, const double* X, const double* dir, doub
     if ((rc = upload3(c, i, dir, c->A.dir))) return rc;
     std::vector<double> a(c->A.nI, *alpha);
     IDP_CUDA_TRY(cudaMemcpyAsync(c->A.alpha, a.data(), sizeof(double) * c->A.nI, cudaMemcpyHostToDevice, c->s));
-    if ((rc = ccd_stepsize(c->A, c->W, c->A.Xprev, c->A.dir, c->A.alpha, isc(c, SI_CCDF), c->s))) return rc;
-    std::vector<int> fl;
-    fetch(c, c->A.alpha, a);
-    fetch(c, isc(c, SI_CCDF), fl);
+    std::vector<int> fl(c->A.nI);
+    if ((rc = ccd_stepsize(c->A, c->W, c->A.Xprev, c->A.dir, c->A.alpha, isc(c, SI_CCDF), c->s, nullptr, a.data(),
+                           fl.data())))
+        return rc;
     *alpha = a[i];
     if (fl[i] & 2) return IDP_ERR_ZERO_STEP;
     if (fl[i] & 1) return IDP_WARN_ITER_CAP;

@@ -250,7 +250,7 @@ enum WorkSlot {
     W_SCRATCH, W_SCRATCH2, W_TET_GRAD, W_TET_HESS, W_CHUNK_SUM, W_INST_SUM, W_FLAGS,
     // grids (two slots: 0 and 1), 6 buffers each
     W_GRID0, W_GRID0_END = W_GRID0 + 6, W_GRID1 = W_GRID0_END, W_GRID1_END = W_GRID1 + 6,
-    W_BOX_A, W_BOX_B, W_GRIDP, W_BBOX,
+    W_BOX_A, W_BOX_B, W_GRIDP, W_BBOX, W_XF, W_DF,
     W_CAND, W_CAND_CNT,
     W_CONS, W_CONS_INST, W_CONS_KEY_HI, W_CONS_KEY_LO, W_CONS_PERM, W_CONS_PERM2, W_CONS_TMP, W_CONS_TMP_INST,
     W_CONS_HEAD, W_CONS_OFF, W_CONS_CNT, W_DIST2,
@@ -416,7 +416,8 @@ int barrier_hessian(Arena& A, Work& W, const double* X, const ContactSet& cs, bo
 int ccd_voxel_size(Arena& A, Work& W, const double* X, cudaStream_t s);
 const double* ccd_voxel_sizes(Arena& A, Work& W);
 int ccd_stepsize(Arena& A, Work& W, const double* X, const double* dir, double* alpha /*device nI*/, int* flags,
-                 cudaStream_t s, const double* voxel_pre = nullptr);
+                 cudaStream_t s, const double* voxel_pre = nullptr, double* host_alpha = nullptr,
+                 int* host_flags = nullptr);  // host copies of the results (nI values), read with the call's own sync
 
 // solver.cu
 int assemble(Arena& A, Work& W, const ContactSet& cs, bool fp64, cudaStream_t s);

@@ -19,6 +19,7 @@ struct GridP {
     double inv;
     int n[3];      // cells per axis (indices clamped to [0, n])
     int coarse;    // CCD candidate grid: reference voxels per cell along each axis
+    float ext;     // largest extent of the instance (bounds the coordinates of its FP32 positions)
     long s1, s2;   // linear strides: cell = x + y*s1 + z*s2
 };
 
@@ -88,6 +89,46 @@ __device__ __forceinline__ uint64_t cell_key(int inst, const GridP& g, int x, in
     return ((uint64_t)inst << 32) | (uint64_t)((long)x + (long)y * g.s1 + (long)z * g.s2);
 }
 
+
+// first cell of every instance of the grids gp[0..nI) (prefix of the cell
+// counts), the total and, beyond cap, bit 0 of *flag; one CTA, after its own
+// threads wrote gp
+__device__ inline void cta_cell_bases(int nI, const GridP* gp, uint32_t* cbase, unsigned long long* total,
+                               unsigned long long cap, unsigned int* flag) {
+    __shared__ unsigned long long cnt[kBlock];
+    __shared__ unsigned long long acc;
+    if (threadIdx.x == 0) acc = 0;
+    __syncthreads();
+    for (int i0 = 0; i0 < nI; i0 += kBlock) {
+        const int i = i0 + threadIdx.x;
+        if (threadIdx.x < kBlock)
+            cnt[threadIdx.x] = i < nI ? (unsigned long long)gp[i].s2 * (unsigned long long)(gp[i].n[2] + 1) : 0ull;
+        __syncthreads();
+        if (threadIdx.x == 0)
+            for (int k = 0; k < kBlock && i0 + k < nI; ++k) {
+                cbase[i0 + k] = (uint32_t)(acc < 0xffffffffull ? acc : 0xffffffffull);
+                acc += cnt[k];
+            }
+        __syncthreads();
+    }
+    if (threadIdx.x == 0) {
+        cbase[nI] = (uint32_t)(acc < 0xffffffffull ? acc : 0xffffffffull);
+        *total = acc;
+        if (acc > cap) atomicOr(flag, 1u);
+    }
+}
+
+// boxes are built inside [0, n]; the clamp only guards the table bounds
+__device__ __forceinline__ void count_cells(const BoxI& b, const GridP& g, uint32_t c0, uint32_t cap, uint32_t* cnt) {
+    const int zl = max(b.lo[2], 0), zh = min(b.hi[2], g.n[2]), yl = max(b.lo[1], 0), yh = min(b.hi[1], g.n[1]);
+    const int xl = max(b.lo[0], 0), xh = min(b.hi[0], g.n[0]);
+    for (int z = zl; z <= zh; ++z)
+        for (int y = yl; y <= yh; ++y)
+            for (int x = xl; x <= xh; ++x) {
+                const uint32_t c = c0 + (uint32_t)((long)x + (long)y * g.s1 + (long)z * g.s2);
+                if (c < cap) atomicAdd(cnt + c, 1u);
+            }
+}
 
 // open-addressing hash from (instance, cell) key to the cell's index in the
 // sorted cell table (linear probing, table at most half full)
@@ -184,6 +225,34 @@ __device__ __forceinline__ void group_walk_emit(const BoxI& qb, int inst, const 
                                                 const uint32_t* __restrict__ entries, V* __restrict__ out,
                                                 unsigned int* counter, long cap, Test&& test) {
     const int gl = threadIdx.x & (G - 1);
+    if (cells.dense) {
+        // a run of cells along x is a run of the table, hence of the entries: one
+        // pass per (y, z) instead of one per cell (a pass is a chain of four
+        // dependent loads; most cells hold fewer entries than the group has lanes)
+        const int x0 = max(qb.lo[0], 0), x1 = min(qb.hi[0], g.n[0]);
+        const int y0 = max(qb.lo[1], 0), y1 = min(qb.hi[1], g.n[1]), z0 = max(qb.lo[2], 0), z1 = min(qb.hi[2], g.n[2]);
+        if (x0 > x1) return;
+        const uint32_t c_inst = cells.cbase[inst];
+        for (int z = z0; z <= z1; ++z)
+            for (int y = y0; y <= y1; ++y) {
+                const uint32_t c0 = c_inst + (uint32_t)((long)x0 + (long)y * g.s1 + (long)z * g.s2);
+                if (c0 >= cells.cap) continue;
+                const uint32_t c1 = min(c0 + (uint32_t)(x1 - x0), cells.cap - 1);
+                const uint32_t e0 = cstart[c0], e1 = min(cstart[c1 + 1], cells.ent_cap);
+                for (uint32_t base = e0; base < e1; base += G) {
+                    const uint32_t e = base + gl;
+                    V v;
+                    bool emit = false;
+                    if (e < e1) {
+                        uint32_t c = c0;
+                        while (c < c1 && e >= cstart[c + 1]) ++c;
+                        emit = test(entries[e], x0 + (int)(c - c0), y, z, v);
+                    }
+                    group_emit<G>(emit, v, out, counter, cap);
+                }
+            }
+        return;
+    }
     for (int z = qb.lo[2]; z <= qb.hi[2]; ++z)
         for (int y = qb.lo[1]; y <= qb.hi[1]; ++y)
             for (int x = qb.lo[0]; x <= qb.hi[0]; ++x) {
@@ -225,9 +294,20 @@ int box_grid_finish(Work& W, int slot, const BoxI* boxes, const int* inst, const
 // *d_flag (bit 0: more cells, bit 1: more entries than the capacities) what
 // did not fit, and the caller, at its next synchronisation, calls
 // grids_overflowed and rebuilds when it returns true.
+// counted: the caller's kernels already made the cell bases and counted the boxes
+// into grids_tables' counters (only when that returned true).
 int grids_build(Work& W, int set, const BoxI* tbox, long nt, const int* tinst, const BoxI* ebox, long ne,
                 const int* einst, const unsigned char* active, const GridP* gp, int nI, unsigned int* d_flag,
-                BoxGrid& gt, BoxGrid& ge, cudaStream_t s);
+                BoxGrid& gt, BoxGrid& ge, cudaStream_t s, bool counted = false);
+// tables of a set whose capacities are known (see grids_build), their counters
+// cleared; false: the set has not been built yet, or not as a dense table
+struct GridTables {
+    uint32_t* ccount = nullptr;
+    uint32_t* cbase = nullptr;
+    unsigned long long* total = nullptr;
+    uint32_t cap = 0;
+};
+int grids_tables(Work& W, int set, int nI, GridTables& t, cudaStream_t s);
 bool grids_overflowed(Work& W, int set, unsigned int flag);
 // first cell of every instance of a grid and the total cell count (written
 // to *h_cells, pinned host memory, valid after the stream is synchronised)
