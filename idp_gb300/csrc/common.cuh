@@ -39,7 +39,7 @@ struct Chunk {
     int begin;
     int end;
 };
-constexpr int kChunk = 1024;
+constexpr int kChunk = 256;  // one element per thread: small meshes still fill several CTAs
 // vertices per dense contact-cluster block of the preconditioner (576 x 576)
 constexpr int kClusterCap = 192;
 

@@ -7,6 +7,7 @@
 #include <string>
 #include <chrono>
 #include "common.cuh"
+#include "reduce.cuh"
 #include "../../include/idp_gb300.h"
 
 namespace idp {
@@ -250,7 +251,7 @@ enum WorkSlot {
     W_SCRATCH, W_SCRATCH2, W_TET_GRAD, W_TET_HESS, W_CHUNK_SUM, W_INST_SUM, W_FLAGS,
     // grids (two slots: 0 and 1), 6 buffers each
     W_GRID0, W_GRID0_END = W_GRID0 + 6, W_GRID1 = W_GRID0_END, W_GRID1_END = W_GRID1 + 6,
-    W_BOX_A, W_BOX_B, W_GRIDP, W_BBOX, W_XF, W_DF,
+    W_BOX_A, W_BOX_B, W_GRIDP, W_BBOX, W_XF, W_DF, W_SUMCNT,
     W_CAND, W_CAND_CNT,
     W_CONS, W_CONS_INST, W_CONS_KEY_HI, W_CONS_KEY_LO, W_CONS_PERM, W_CONS_PERM2, W_CONS_TMP, W_CONS_TMP_INST,
     W_CONS_HEAD, W_CONS_OFF, W_CONS_CNT, W_DIST2,
@@ -321,6 +322,7 @@ struct Work {
     long dense_ent_cap[2] = {0, 0};
     unsigned long long grid_prof[5] = {0, 0, 0, 0, 0};  // grid PCG phase ns (IDP_PROFILE)
     bool grid_prof_init = false;
+    int sum_counters = 0;                    // counters of W_SUMCNT cleared so far
     uint32_t* hpin = nullptr;                // 64 words of pinned host memory for batched readbacks
     uint32_t* pinned() {
         if (!hpin && cudaMallocHost(reinterpret_cast<void**>(&hpin), 64 * sizeof(uint32_t)) != cudaSuccess)
@@ -447,8 +449,9 @@ int dbc_classify(Arena& A, const double* X, double* dir, int* moving, cudaStream
 int dbc_snap(Arena& A, double* X, cudaStream_t s);
 int dbc_sums(Arena& A, Work& W, const double* X, double* inst_w, double* inst_d, cudaStream_t s);
 int dbc_gradient(Arena& A, const double* X, double* g, cudaStream_t s);
-int chunk_reduce(Arena& A, Work& W, const Chunk* chunks, int nchunks, const double* chunk_vals, double* inst_out,
-                 cudaStream_t s);
+// arguments of a per-instance sum over the chunks coff (per CTAs each) into out
+int inst_sum_args(Arena& A, Work& W, const int* coff, int nchunks, int per, double* out, bool accumulate, InstSum& r,
+                  cudaStream_t s);
 int chunk_reduce_off(Arena& A, const int* coff, const double* part, double* out, bool accumulate, cudaStream_t s);
 int grad_gather_tet(Arena& A, Work& W, const double* X, double* g, cudaStream_t s);
 int hessian_apply(Arena& A, Work& W, bool fp64, const double* x, double* y, cudaStream_t s);

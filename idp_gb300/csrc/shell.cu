@@ -13,19 +13,6 @@
 namespace idp {
 namespace {
 
-__device__ double block_sum_flow(double v) {
-    __shared__ double sh[kBlock];
-    sh[threadIdx.x] = v;
-    __syncthreads();
-    for (int st = kBlock / 2; st > 0; st >>= 1) {
-        if (threadIdx.x < st) sh[threadIdx.x] += sh[threadIdx.x + st];
-        __syncthreads();
-    }
-    double r = sh[0];
-    __syncthreads();
-    return r;
-}
-
 __device__ __forceinline__ double sq3(const double* a, const double* b) {
     const double d0 = a[0] - b[0], d1 = a[1] - b[1], d2 = a[2] - b[2];
     return d0 * d0 + d1 * d1 + d2 * d2;
@@ -34,7 +21,7 @@ __device__ __forceinline__ double sq3(const double* a, const double* b) {
 // one CTA per chunk of faces of one instance; fixed tree per chunk
 __global__ void k_flow_energy(const Chunk* __restrict__ chunks, const unsigned char* __restrict__ active,
                               const double* __restrict__ X, const int* __restrict__ face,
-                              const double* __restrict__ fvol, double h, double* __restrict__ part) {
+                              const double* __restrict__ fvol, double h, InstSum sum) {
     const Chunk c = chunks[blockIdx.x];
     double acc = 0.0;
     if (active[c.inst])
@@ -44,8 +31,7 @@ __global__ void k_flow_energy(const Chunk* __restrict__ chunks, const unsigned c
             const double* x2 = X + 3L * face[3L * f + 2];
             acc += h / 12.0 * fvol[f] * (sq3(x0, x1) + sq3(x1, x2) + sq3(x2, x0));
         }
-    const double s = block_sum_flow(acc);
-    if (threadIdx.x == 0) part[blockIdx.x] = s;
+    inst_sum(sum, c.inst, acc);
 }
 
 // per vertex: its incident faces in ascending order
@@ -78,12 +64,11 @@ __global__ void k_flow_gradient(long V, const int* __restrict__ vinst, const uns
 
 int flow_energy(Arena& A, Work& W, const double* X, double* inst_E, cudaStream_t s) {
     if (A.F == 0) return IDP_OK;
-    if (W[W_CHUNK_SUM].ensure(sizeof(double) * (A.n_face_chunks + A.n_tet_chunks + A.n_vert_chunks + 2)))
-        return IDP_ERR_CUDA;
-    double* part = W[W_CHUNK_SUM].as<double>();
+    InstSum r;
+    if (int rc = inst_sum_args(A, W, A.face_chunk_off, A.n_face_chunks, 1, inst_E, true, r, s)) return rc;
     (::idp::count_launch(),
-     k_flow_energy<<<A.n_face_chunks, kBlock, 0, s>>>(A.face_chunks, A.active, X, A.face, A.fvol, A.h, part));
-    return chunk_reduce_off(A, A.face_chunk_off, part, inst_E, true, s);
+     k_flow_energy<<<A.n_face_chunks, kBlock, 0, s>>>(A.face_chunks, A.active, X, A.face, A.fvol, A.h, r));
+    return cudaGetLastError() == cudaSuccess ? IDP_OK : IDP_ERR_CUDA;
 }
 
 int flow_gradient(Arena& A, const double* X, double* g, cudaStream_t s) {

@@ -34,19 +34,6 @@ __device__ __forceinline__ D3s crs(D3s a, D3s b) {
 }
 __device__ __forceinline__ double comp(D3s a, int i) { return i == 0 ? a.x : (i == 1 ? a.y : a.z); }
 
-__device__ double block_sum_shell(double v) {
-    __shared__ double sh[kBlock];
-    sh[threadIdx.x] = v;
-    __syncthreads();
-    for (int st = kBlock / 2; st > 0; st >>= 1) {
-        if (threadIdx.x < st) sh[threadIdx.x] += sh[threadIdx.x + st];
-        __syncthreads();
-    }
-    double r = sh[0];
-    __syncthreads();
-    return r;
-}
-
 // ---- membrane of one face; mem = (IB^-1 00, 01, 11, det IB^-1, vol, lam, mu)
 __device__ double membrane_face(D3s x1, D3s x2, D3s x3, const double* m, double w, double* g, double* H) {
     const D3s e01 = sub(x2, x1), e02 = sub(x3, x1);
@@ -243,7 +230,7 @@ __device__ __forceinline__ bool all_fixed(const unsigned char* dbc, const int* v
 __global__ void k_membrane_energy(const Chunk* __restrict__ chunks, const unsigned char* __restrict__ active,
                                   const double* __restrict__ X, const int* __restrict__ mface,
                                   const double* __restrict__ mem, const unsigned char* __restrict__ dbc, double w,
-                                  double* __restrict__ part) {
+                                  InstSum sum) {
     const Chunk c = chunks[blockIdx.x];
     double acc = 0.0;
     if (active[c.inst])
@@ -252,14 +239,13 @@ __global__ void k_membrane_energy(const Chunk* __restrict__ chunks, const unsign
             if (all_fixed(dbc, t, 3)) continue;
             acc += membrane_face(ld(X, t[0]), ld(X, t[1]), ld(X, t[2]), mem + 7L * f, w, nullptr, nullptr);
         }
-    const double s = block_sum_shell(acc);
-    if (threadIdx.x == 0) part[blockIdx.x] = s;
+    inst_sum(sum, c.inst, acc);
 }
 
 __global__ void k_bending_energy(const Chunk* __restrict__ chunks, const unsigned char* __restrict__ active,
                                  const double* __restrict__ X, const int4* __restrict__ hinge,
                                  const double* __restrict__ hk, const unsigned char* __restrict__ dbc, double w,
-                                 double* __restrict__ part) {
+                                 InstSum sum) {
     const Chunk c = chunks[blockIdx.x];
     double acc = 0.0;
     if (active[c.inst])
@@ -269,8 +255,7 @@ __global__ void k_bending_energy(const Chunk* __restrict__ chunks, const unsigne
             if (all_fixed(dbc, v, 4)) continue;
             acc += bending_hinge(ld(X, v[0]), ld(X, v[1]), ld(X, v[2]), ld(X, v[3]), hk + 2L * i, w, nullptr, nullptr);
         }
-    const double s = block_sum_shell(acc);
-    if (threadIdx.x == 0) part[blockIdx.x] = s;
+    inst_sum(sum, c.inst, acc);
 }
 
 // element gradients: face f at slots 3f..3f+2, hinge i at 3 Fm + 4i ..
@@ -406,23 +391,18 @@ __global__ void __launch_bounds__(kPsdThreads) k_shell_psd(long Ne, const T* __r
 
 int shell_energy(Arena& A, Work& W, const double* X, double w_h2, double* inst_E, cudaStream_t s) {
     if (A.Fm == 0 && A.Hn == 0) return IDP_OK;
-    if (W[W_CHUNK_SUM].ensure(sizeof(double) *
-                              (A.n_mface_chunks + A.n_hinge_chunks + A.n_face_chunks + A.n_tet_chunks + A.n_vert_chunks + 2)))
-        return IDP_ERR_CUDA;
-    double* part = W[W_CHUNK_SUM].as<double>();
-    int rc = IDP_OK;
+    InstSum r;
     if (A.Fm) {
+        if (int rc = inst_sum_args(A, W, A.mface_chunk_off, A.n_mface_chunks, 1, inst_E, true, r, s)) return rc;
         (::idp::count_launch(), k_membrane_energy<<<A.n_mface_chunks, kBlock, 0, s>>>(A.mface_chunks, A.active, X, A.mface,
-                                                                                      A.mem, A.dbc_excl, w_h2, part));
-        rc = chunk_reduce_off(A, A.mface_chunk_off, part, inst_E, true, s);
-        if (rc) return rc;
+                                                                                      A.mem, A.dbc_excl, w_h2, r));
     }
     if (A.Hn) {
+        if (int rc = inst_sum_args(A, W, A.hinge_chunk_off, A.n_hinge_chunks, 1, inst_E, true, r, s)) return rc;
         (::idp::count_launch(), k_bending_energy<<<A.n_hinge_chunks, kBlock, 0, s>>>(A.hinge_chunks, A.active, X, A.hinge,
-                                                                                     A.hk, A.dbc_excl, w_h2, part));
-        rc = chunk_reduce_off(A, A.hinge_chunk_off, part, inst_E, true, s);
+                                                                                     A.hk, A.dbc_excl, w_h2, r));
     }
-    return rc;
+    return cudaGetLastError() == cudaSuccess ? IDP_OK : IDP_ERR_CUDA;
 }
 
 int shell_gradient(Arena& A, Work& W, const double* X, double w_h2, double* g, cudaStream_t s) {

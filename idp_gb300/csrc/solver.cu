@@ -120,85 +120,92 @@ __global__ void k_diag_inv(long V, const int* __restrict__ diagblk, const T* __r
     for (int q = 0; q < 9; ++q) dinv[9 * v + q] = o[q];
 }
 
-// y = A x for the rows of instances with run[inst] != 0; optional partial
-// dot products p.y per vertex chunk
-template <class T, class TX, class TY>
-__device__ __forceinline__ void spmv_row(long v, const int* __restrict__ rowptr, const int* __restrict__ colidx,
-                                         const T* __restrict__ val, const int* __restrict__ trp,
-                                         const int* __restrict__ tcol, const T* __restrict__ tval,
-                                         const unsigned char* __restrict__ dbc, const TX* __restrict__ x, TY y[3]) {
-    if (dbc[v]) {
-        y[0] = (TY)x[3 * v]; y[1] = (TY)x[3 * v + 1]; y[2] = (TY)x[3 * v + 2];
-        return;
-    }
-    TY a0 = 0, a1 = 0, a2 = 0;
-    for (int k = rowptr[v]; k < rowptr[v + 1]; ++k) {
-        int c = colidx[k];
-        const T* m = val + 9 * (long)k;
-        TY x0 = (TY)x[3 * c], x1 = (TY)x[3 * c + 1], x2 = (TY)x[3 * c + 2];
-        a0 += (TY)m[0] * x0 + (TY)m[1] * x1 + (TY)m[2] * x2;
-        a1 += (TY)m[3] * x0 + (TY)m[4] * x1 + (TY)m[5] * x2;
-        a2 += (TY)m[6] * x0 + (TY)m[7] * x1 + (TY)m[8] * x2;
-    }
-    for (int k = trp[v]; k < trp[v + 1]; ++k) {
-        int c = tcol[k];
-        if (dbc[c]) continue;
-        const T* m = tval + 9 * (long)k;
-        TY x0 = (TY)x[3 * c], x1 = (TY)x[3 * c + 1], x2 = (TY)x[3 * c + 2];
-        a0 += (TY)m[0] * x0 + (TY)m[1] * x1 + (TY)m[2] * x2;
-        a1 += (TY)m[3] * x0 + (TY)m[4] * x1 + (TY)m[5] * x2;
-        a2 += (TY)m[6] * x0 + (TY)m[7] * x1 + (TY)m[8] * x2;
-    }
-    y[0] = a0; y[1] = a1; y[2] = a2;
-}
-
-__device__ double cta_sum(double v) {
-    __shared__ double sh[kBlock];
-    sh[threadIdx.x] = v;
-    __syncthreads();
-    for (int st = kBlock / 2; st > 0; st >>= 1) {
-        if (threadIdx.x < st) sh[threadIdx.x] += sh[threadIdx.x + st];
-        __syncthreads();
-    }
-    double r = sh[0];
-    __syncthreads();
-    return r;
-}
-
-// FP64 residual res = b - A x64 (FP32/FP64 matrix, FP64 accumulation), one
-// thread per block row in small CTAs (the FP64 pipe, not memory, limits it);
-// the squared norm is reduced afterwards per vertex chunk
+// Row v of A x in FP64 (FP32 or FP64 matrix) by 8 lanes: lane l takes blocks
+// l, l + 8, ... of the row and of its contact tail; every lane gets the sums.
+// (A thread per row was a chain of up to 19 dependent gathers: 35 us for 160
+// vertices, 52 us for 49,863.) All lanes of the warp call this together.
 template <class T>
-__global__ void k_residual64(long V, const int* __restrict__ vinst, const unsigned char* __restrict__ active,
+__device__ __forceinline__ void row8_f64(bool on, long v, int l, const int* __restrict__ rowptr,
+                                         const int* __restrict__ colidx, const T* __restrict__ val,
+                                         const int* __restrict__ trp, const int* __restrict__ tcol,
+                                         const T* __restrict__ tval, const unsigned char* __restrict__ dbc,
+                                         const double* __restrict__ x, double y[3]) {
+    double a0 = 0, a1 = 0, a2 = 0;
+    if (on) {
+        const int k1 = rowptr[v + 1];
+#pragma unroll 2
+        for (int k = rowptr[v] + l; k < k1; k += 8) {
+            const double* xv = x + 3L * colidx[k];
+            const T* m = val + 9L * k;
+            const double x0 = xv[0], x1 = xv[1], x2 = xv[2];
+            a0 += (double)m[0] * x0 + (double)m[1] * x1 + (double)m[2] * x2;
+            a1 += (double)m[3] * x0 + (double)m[4] * x1 + (double)m[5] * x2;
+            a2 += (double)m[6] * x0 + (double)m[7] * x1 + (double)m[8] * x2;
+        }
+        const int t1 = trp[v + 1];
+        for (int k = trp[v] + l; k < t1; k += 8) {
+            const int c = tcol[k];
+            if (dbc[c]) continue;
+            const double* xv = x + 3L * c;
+            const T* m = tval + 9L * k;
+            const double x0 = xv[0], x1 = xv[1], x2 = xv[2];
+            a0 += (double)m[0] * x0 + (double)m[1] * x1 + (double)m[2] * x2;
+            a1 += (double)m[3] * x0 + (double)m[4] * x1 + (double)m[5] * x2;
+            a2 += (double)m[6] * x0 + (double)m[7] * x1 + (double)m[8] * x2;
+        }
+    }
+    for (int o = 4; o > 0; o >>= 1) {
+        a0 += __shfl_xor_sync(0xffffffffu, a0, o);
+        a1 += __shfl_xor_sync(0xffffffffu, a1, o);
+        a2 += __shfl_xor_sync(0xffffffffu, a2, o);
+    }
+    y[0] = a0;
+    y[1] = a1;
+    y[2] = a2;
+}
+
+// CTAs per vertex chunk of the residual: 32 rows each
+constexpr int kResPer = kChunk / 32;
+
+// FP64 residual res = b - A x (FP64 accumulation) and |res|^2 per instance
+template <class T>
+__global__ void k_residual64(const Chunk* __restrict__ chunks, const unsigned char* __restrict__ active,
                              const int* __restrict__ rowptr, const int* __restrict__ colidx, const T* __restrict__ val,
                              const int* __restrict__ trp, const int* __restrict__ tcol, const T* __restrict__ tval,
                              const unsigned char* __restrict__ dbc, const double* __restrict__ b,
-                             const double* __restrict__ x, double* __restrict__ res) {
-    long v = (long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (v >= V || !active[vinst[v]]) return;
+                             const double* __restrict__ x, double* __restrict__ res, InstSum sum) {
+    const Chunk c = chunks[blockIdx.x / kResPer];
+    const int l = threadIdx.x & 7;
+    const long v = c.begin + 32 * (blockIdx.x % kResPer) + (threadIdx.x >> 3);
+    const bool on = active[c.inst] && v < c.end;
+    const bool fixed = on && dbc[v];
     double y[3];
-    spmv_row<T, double, double>(v, rowptr, colidx, val, trp, tcol, tval, dbc, x, y);
-#pragma unroll
-    for (int d = 0; d < 3; ++d) res[3 * v + d] = dbc[v] ? 0.0 : b[3 * v + d] - y[d];
+    row8_f64<T>(on && !fixed, v, l, rowptr, colidx, val, trp, tcol, tval, dbc, x, y);
+    double acc = 0;
+    if (on && l < 3) {
+        const double r = fixed ? 0.0 : b[3 * v + l] - (l == 0 ? y[0] : (l == 1 ? y[1] : y[2]));
+        res[3 * v + l] = r;
+        acc = r * r;
+    }
+    inst_sum(sum, c.inst, acc);
 }
 
-__global__ void k_norm2_chunks(const Chunk* __restrict__ chunks, const unsigned char* __restrict__ active,
-                               const double* __restrict__ a, double* __restrict__ part) {
-    Chunk c = chunks[blockIdx.x];
+// start of the refinement: x = 0 (only the active instances': a later solve of
+// some instances, the FP64 fallback, must not disturb the others' directions),
+// so res = b without a product
+__global__ void k_refine_start(const Chunk* __restrict__ chunks, const unsigned char* __restrict__ active,
+                               const unsigned char* __restrict__ dbc, const double* __restrict__ b,
+                               double* __restrict__ x, double* __restrict__ res, InstSum sum) {
+    const Chunk c = chunks[blockIdx.x];
     double acc = 0;
     if (active[c.inst])
-        for (int k = 3 * c.begin + threadIdx.x; k < 3 * c.end; k += blockDim.x) acc += a[k] * a[k];
-    double s = cta_sum(acc);
-    if (threadIdx.x == 0) part[blockIdx.x] = s;
-}
-
-__global__ void k_zero_masked(long V, const int* __restrict__ vinst, const unsigned char* __restrict__ active,
-                              double* __restrict__ x) {
-    long v = (long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (v >= V || !active[vinst[v]]) return;
-    x[3 * v] = 0.0;
-    x[3 * v + 1] = 0.0;
-    x[3 * v + 2] = 0.0;
+        for (int k = 3 * c.begin + threadIdx.x; k < 3 * c.end; k += blockDim.x) {
+            const double r = dbc[k / 3] ? 0.0 : b[k];
+            x[k] = 0.0;
+            res[k] = r;
+            acc += r * r;
+        }
+    inst_sum(sum, c.inst, acc);
 }
 
 template <class T>
@@ -215,44 +222,53 @@ __global__ void k_spmv_plain(long V, const int* __restrict__ vinst, const unsign
                              const int* __restrict__ trp, const int* __restrict__ tcol, const T* __restrict__ tval,
                              const unsigned char* __restrict__ dbc, const double* __restrict__ x,
                              double* __restrict__ y) {
-    long v = (long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (v >= V || !active[vinst[v]]) return;
+    const long v = ((long)blockIdx.x * blockDim.x + threadIdx.x) >> 3;
+    const int l = threadIdx.x & 7;
+    const bool on = v < V && active[vinst[v]];
+    const bool fixed = on && dbc[v];
     double o[3];
-    spmv_row<T, double, double>(v, rowptr, colidx, val, trp, tcol, tval, dbc, x, o);
-    y[3 * v] = o[0]; y[3 * v + 1] = o[1]; y[3 * v + 2] = o[2];
+    row8_f64<T>(on && !fixed, v, l, rowptr, colidx, val, trp, tcol, tval, dbc, x, o);
+    if (on && l < 3) y[3 * v + l] = fixed ? x[3 * v + l] : (l == 0 ? o[0] : (l == 1 ? o[1] : o[2]));
 }
 
 // ---- per-vertex Newton kernels
+// 8 lanes per vertex: lane l takes its corners l, l + 8, ...
 __global__ void k_grad_gather_tet(long V, const int* __restrict__ vinst, const unsigned char* __restrict__ active,
                                   const int* __restrict__ vcp, const int* __restrict__ vc,
                                   const double* __restrict__ tg, const double* __restrict__ mass,
                                   const double* __restrict__ X, const double* __restrict__ Xt, double* __restrict__ g) {
-    long v = (long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (v >= V || !active[vinst[v]]) return;
+    const long v = ((long)blockIdx.x * blockDim.x + threadIdx.x) >> 3;
+    const int l = threadIdx.x & 7;
+    const bool on = v < V && active[vinst[v]];
     double s0 = 0, s1 = 0, s2 = 0;
-    for (int k = vcp[v]; k < vcp[v + 1]; ++k) {
-        int code = vc[k];  // tet*4 + corner
-        const double* p = tg + 12 * (long)(code >> 2) + 3 * (code & 3);
-        s0 += p[0]; s1 += p[1]; s2 += p[2];
+    if (on) {
+        const int k1 = vcp[v + 1];
+        for (int k = vcp[v] + l; k < k1; k += 8) {
+            int code = vc[k];  // tet*4 + corner
+            const double* p = tg + 12 * (long)(code >> 2) + 3 * (code & 3);
+            s0 += p[0]; s1 += p[1]; s2 += p[2];
+        }
     }
-    double m = mass[v];
-    g[3 * v] = s0 + m * (X[3 * v] - Xt[3 * v]);
-    g[3 * v + 1] = s1 + m * (X[3 * v + 1] - Xt[3 * v + 1]);
-    g[3 * v + 2] = s2 + m * (X[3 * v + 2] - Xt[3 * v + 2]);
+    for (int o = 4; o > 0; o >>= 1) {
+        s0 += __shfl_xor_sync(0xffffffffu, s0, o);
+        s1 += __shfl_xor_sync(0xffffffffu, s1, o);
+        s2 += __shfl_xor_sync(0xffffffffu, s2, o);
+    }
+    if (on && l < 3)
+        g[3 * v + l] = (l == 0 ? s0 : (l == 1 ? s1 : s2)) + mass[v] * (X[3 * v + l] - Xt[3 * v + l]);
 }
 
 __global__ void k_inertia_energy(const Chunk* __restrict__ chunks, const unsigned char* __restrict__ active,
                                  const double* __restrict__ mass, const double* __restrict__ X,
-                                 const double* __restrict__ Xt, double* __restrict__ part) {
-    Chunk c = chunks[blockIdx.x];
+                                 const double* __restrict__ Xt, InstSum sum) {
+    const Chunk c = chunks[blockIdx.x];
     double acc = 0;
     if (active[c.inst])
         for (int v = c.begin + threadIdx.x; v < c.end; v += blockDim.x) {
             double d0 = X[3 * v] - Xt[3 * v], d1 = X[3 * v + 1] - Xt[3 * v + 1], d2 = X[3 * v + 2] - Xt[3 * v + 2];
             acc += 0.5 * mass[v] * (d0 * d0 + d1 * d1 + d2 * d2);
         }
-    double s = cta_sum(acc);
-    if (threadIdx.x == 0) part[blockIdx.x] = s;
+    inst_sum(sum, c.inst, acc);
 }
 
 // per instance: its chunk partials summed by one warp (lane-strided, then a
@@ -1211,24 +1227,31 @@ int chunk_reduce_off(Arena& A, const int* coff, const double* part, double* out,
     return cudaGetLastError() == cudaSuccess ? IDP_OK : IDP_ERR_CUDA;
 }
 
-int chunk_reduce(Arena& A, Work& W, const Chunk* chunks, int nchunks, const double* part, double* out, cudaStream_t s) {
-    (void)W;
-    (void)nchunks;
-    const int* coff = (chunks == A.tet_chunks) ? A.tet_chunk_off : A.vert_chunk_off;
-    return chunk_reduce_off(A, coff, part, out, false, s);
+int inst_sum_args(Arena& A, Work& W, const int* coff, int nchunks, int per, double* out, bool accumulate, InstSum& r,
+                  cudaStream_t s) {
+    if (W[W_CHUNK_SUM].ensure(sizeof(double) * ((size_t)nchunks * per + 2))) return IDP_ERR_CUDA;
+    if (W.sum_counters < A.nI) {  // the kernels leave them at zero
+        if (W[W_SUMCNT].ensure(sizeof(unsigned int) * A.nI)) return IDP_ERR_CUDA;
+        IDP_CUDA_TRY(cudaMemsetAsync(W[W_SUMCNT].p, 0, W[W_SUMCNT].bytes, s));
+        W.sum_counters = (int)(W[W_SUMCNT].bytes / sizeof(unsigned int));
+    }
+    r = {coff, per, A.nI, W[W_CHUNK_SUM].as<double>(), W[W_SUMCNT].as<unsigned int>(), out, accumulate ? 1 : 0};
+    return IDP_OK;
 }
 
 int vec_inertia(Arena& A, Work& W, const double* X, double* inst_E, double* g, cudaStream_t s) {
     (void)g;
-    if (W[W_CHUNK_SUM].ensure(sizeof(double) * (A.n_vert_chunks + A.n_tet_chunks + 2))) return IDP_ERR_CUDA;
-    double* part = W[W_CHUNK_SUM].as<double>();
-    (::idp::count_launch(), k_inertia_energy<<<A.n_vert_chunks, kBlock, 0, s>>>(A.vert_chunks, A.active, A.mass, X, A.Xtilde, part));
-    return chunk_reduce_off(A, A.vert_chunk_off, part, inst_E, false, s);
+    InstSum r;
+    if (int rc = inst_sum_args(A, W, A.vert_chunk_off, A.n_vert_chunks, 1, inst_E, false, r, s)) return rc;
+    (::idp::count_launch(), k_inertia_energy<<<A.n_vert_chunks, kBlock, 0, s>>>(A.vert_chunks, A.active, A.mass, X,
+                                                                               A.Xtilde, r));
+    return cudaGetLastError() == cudaSuccess ? IDP_OK : IDP_ERR_CUDA;
 }
 
 int grad_gather_tet(Arena& A, Work& W, const double* X, double* g, cudaStream_t s) {
-    (::idp::count_launch(), k_grad_gather_tet<<<grid_for(A.V), kBlock, 0, s>>>(A.V, A.vinst, A.active, A.vert_corner_ptr, A.vert_corner,
-                                                       W[W_TET_GRAD].as<double>(), A.mass, X, A.Xtilde, g));
+    (::idp::count_launch(), k_grad_gather_tet<<<grid_for(8 * A.V), kBlock, 0, s>>>(
+                                A.V, A.vinst, A.active, A.vert_corner_ptr, A.vert_corner, W[W_TET_GRAD].as<double>(),
+                                A.mass, X, A.Xtilde, g));
     return cudaGetLastError() == cudaSuccess ? IDP_OK : IDP_ERR_CUDA;
 }
 
@@ -1270,11 +1293,11 @@ int hessian_apply(Arena& A, Work& W, bool fp64, const double* x, double* y, cuda
     const int* trp = W[W_TAIL_ROWPTR].as<int>();
     const int* tcol = W[W_TAIL_COL].as<int>();
     if (fp64)
-        (::idp::count_launch(), k_spmv_plain<double><<<grid_for(A.V), kBlock, 0, s>>>(A.V, A.vinst, A.active, A.rowptr, A.colidx,
+        (::idp::count_launch(), k_spmv_plain<double><<<grid_for(8 * A.V), kBlock, 0, s>>>(A.V, A.vinst, A.active, A.rowptr, A.colidx,
                                                               W[W_BSR_VAL].as<double>(), trp, tcol,
                                                               W[W_TAIL_VAL].as<double>(), A.dbc, x, y));
     else
-        (::idp::count_launch(), k_spmv_plain<float><<<grid_for(A.V), kBlock, 0, s>>>(A.V, A.vinst, A.active, A.rowptr, A.colidx,
+        (::idp::count_launch(), k_spmv_plain<float><<<grid_for(8 * A.V), kBlock, 0, s>>>(A.V, A.vinst, A.active, A.rowptr, A.colidx,
                                                              W[W_BSR_VAL].as<float>(), trp, tcol,
                                                              W[W_TAIL_VAL].as<float>(), A.dbc, x, y));
     return cudaGetLastError() == cudaSuccess ? IDP_OK : IDP_ERR_CUDA;
@@ -1558,16 +1581,12 @@ int pcg_solve(Arena& A, Work& W, const ContactSet& cs, bool fp64, const double* 
     iters_out.assign(nI, 0);
     relres_out.assign(nI, 0.0);
     if (W[W_PCG_VEC64].ensure(sizeof(double) * (n3 + 4)) ||
-        W[W_INST_SUM].ensure(sizeof(double) * 8 * (nI + 1)) || W[W_MISC].ensure(sizeof(double) * (A.n_vert_chunks + 2)))
+        W[W_INST_SUM].ensure(sizeof(double) * 8 * (nI + 1)))
         return IDP_ERR_CUDA;
     double* res = W[W_PCG_VEC64].as<double>();
     double* inst_rr = W[W_INST_SUM].as<double>();
-    double* part = W[W_MISC].as<double>();
     const int* trp = W[W_TAIL_ROWPTR].as<int>();
     const int* tcol = W[W_TAIL_COL].as<int>();
-    // only the active instances' solutions are reset: a later solve of some
-    // instances (FP64 fallback) must not disturb the others' directions
-    (::idp::count_launch(), k_zero_masked<<<grid_for(A.V), kBlock, 0, s>>>(A.V, A.vinst, A.active, sol));
     std::vector<double> b2(nI, 0.0), hrr(nI);
     std::vector<unsigned char> act(nI), act0(nI);
     IDP_CUDA_TRY(cudaMemcpyAsync(act0.data(), A.active, nI, cudaMemcpyDeviceToHost, s));
@@ -1576,17 +1595,18 @@ int pcg_solve(Arena& A, Work& W, const ContactSet& cs, bool fp64, const double* 
     // synchronisation of the stream (sync = true waits here)
     double* hres = W.pinned_doubles(nI);
     if (!hres) return IDP_ERR_CUDA;
+    InstSum r8;
+    if (int r = inst_sum_args(A, W, A.vert_chunk_off, A.n_vert_chunks, kResPer, inst_rr, false, r8, s)) return r;
     auto residual_async = [&]() -> int {
+        const int grid = A.n_vert_chunks * kResPer;
         if (fp64)
-            (::idp::count_launch(), k_residual64<double><<<grid_for(A.V, 64), 64, 0, s>>>(A.V, A.vinst, A.active, A.rowptr, A.colidx,
-                                                                    W[W_BSR_VAL].as<double>(), trp, tcol,
-                                                                    W[W_TAIL_VAL].as<double>(), A.dbc, rhs, sol, res));
+            (::idp::count_launch(), k_residual64<double><<<grid, kBlock, 0, s>>>(
+                                        A.vert_chunks, A.active, A.rowptr, A.colidx, W[W_BSR_VAL].as<double>(), trp, tcol,
+                                        W[W_TAIL_VAL].as<double>(), A.dbc, rhs, sol, res, r8));
         else
-            (::idp::count_launch(), k_residual64<float><<<grid_for(A.V, 64), 64, 0, s>>>(A.V, A.vinst, A.active, A.rowptr, A.colidx,
-                                                                   W[W_BSR_VAL].as<float>(), trp, tcol,
-                                                                   W[W_TAIL_VAL].as<float>(), A.dbc, rhs, sol, res));
-        (::idp::count_launch(), k_norm2_chunks<<<A.n_vert_chunks, kBlock, 0, s>>>(A.vert_chunks, A.active, res, part));
-        if (chunk_reduce_off(A, A.vert_chunk_off, part, inst_rr, false, s)) return IDP_ERR_CUDA;
+            (::idp::count_launch(), k_residual64<float><<<grid, kBlock, 0, s>>>(
+                                        A.vert_chunks, A.active, A.rowptr, A.colidx, W[W_BSR_VAL].as<float>(), trp, tcol,
+                                        W[W_TAIL_VAL].as<float>(), A.dbc, rhs, sol, res, r8));
         IDP_CUDA_TRY(cudaMemcpyAsync(hres, inst_rr, sizeof(double) * nI, cudaMemcpyDeviceToHost, s));
         return IDP_OK;
     };
@@ -1599,8 +1619,14 @@ int pcg_solve(Arena& A, Work& W, const ContactSet& cs, bool fp64, const double* 
     };
     // |b|^2 (x = 0 gives res = b); read after the first sweep, whose own
     // synchronisation brings it back (every active instance runs sweep 0)
-    int rc = residual_async();
-    if (rc) return rc;
+    int rc = IDP_OK;
+    {
+        InstSum r1 = r8;
+        r1.per = 1;
+        (::idp::count_launch(), k_refine_start<<<A.n_vert_chunks, kBlock, 0, s>>>(A.vert_chunks, A.active, A.dbc, rhs, sol,
+                                                                                 res, r1));
+        IDP_CUDA_TRY(cudaMemcpyAsync(hres, inst_rr, sizeof(double) * nI, cudaMemcpyDeviceToHost, s));
+    }
     bool b2_pending = true;
     bool hrr_current = false;
     const int max_refine = fp64 ? 1 : 8;

@@ -58,16 +58,12 @@ __device__ double block_sum(double v) {
 __global__ void k_tet_energy(const Chunk* __restrict__ chunks, const unsigned char* __restrict__ active,
                              const double* __restrict__ X, const int4* __restrict__ tet, const double* __restrict__ IB,
                              const double* __restrict__ vol, const double* __restrict__ lam,
-                             const double* __restrict__ mu, double w, double* __restrict__ chunk_E,
-                             int* __restrict__ inst_bad) {
-    Chunk c = chunks[blockIdx.x];
-    if (!active[c.inst]) {
-        if (threadIdx.x == 0) chunk_E[blockIdx.x] = 0.0;
-        return;
-    }
+                             const double* __restrict__ mu, double w, InstSum sum, int* __restrict__ inst_bad) {
+    const Chunk c = chunks[blockIdx.x];
+    const bool on = active[c.inst] != 0;
     double acc = 0.0;
     int bad = 0;
-    for (int t = c.begin + threadIdx.x; t < c.end; t += blockDim.x) {
+    for (int t = c.begin + threadIdx.x; on && t < c.end; t += blockDim.x) {
         double F[9];
         load_F(X, tet[t], IB + 9 * (long)t, F);
         double J = det3(F);
@@ -79,9 +75,8 @@ __global__ void k_tet_energy(const Chunk* __restrict__ chunks, const unsigned ch
         double m = mu[t], l = lam[t];
         acc += w * vol[t] * (m / 2.0 * (f2 - 3.0) - (m - l / 2.0 * lJ) * lJ);
     }
-    double s = block_sum(acc);
     if (bad) inst_bad[c.inst] = 1;
-    if (threadIdx.x == 0) chunk_E[blockIdx.x] = s;
+    inst_sum(sum, c.inst, acc);
 }
 
 // PK1 stress times IB^T per corner (12 doubles per tet)
@@ -320,10 +315,11 @@ __global__ void k_tet_hessian(long T_, const int* __restrict__ tinst, const unsi
 }  // namespace
 
 int tet_energy(Arena& A, Work& W, const double* X, double w_h2, double* inst_E, int* inst_bad, cudaStream_t s) {
-    if (W[W_CHUNK_SUM].ensure(sizeof(double) * (A.n_tet_chunks + 1))) return IDP_ERR_CUDA;
-    (::idp::count_launch(), k_tet_energy<<<A.n_tet_chunks, kBlock, 0, s>>>(A.tet_chunks, A.active, X, A.tet, A.IB, A.vol, A.lam, A.mu, w_h2,
-                                                     W[W_CHUNK_SUM].as<double>(), inst_bad));
-    return chunk_reduce(A, W, A.tet_chunks, A.n_tet_chunks, W[W_CHUNK_SUM].as<double>(), inst_E, s);
+    InstSum r;
+    if (int rc = inst_sum_args(A, W, A.tet_chunk_off, A.n_tet_chunks, 1, inst_E, false, r, s)) return rc;
+    (::idp::count_launch(), k_tet_energy<<<A.n_tet_chunks, kBlock, 0, s>>>(A.tet_chunks, A.active, X, A.tet, A.IB, A.vol,
+                                                                          A.lam, A.mu, w_h2, r, inst_bad));
+    return cudaGetLastError() == cudaSuccess ? IDP_OK : IDP_ERR_CUDA;
 }
 
 int tet_gradient(Arena& A, Work& W, const double* X, double w_h2, double* g_corners_unused, cudaStream_t s) {
@@ -367,6 +363,7 @@ namespace {
 // arena path (CTA tree per 1024-tet chunk, then the chunk sums in order),
 // using only the fixed scratch below for the chunk sums and the inversion
 // flag.
+constexpr int kNoAllocChunk = 1024;       // tets per chunk
 constexpr int kNoAllocMaxChunks = 16384;  // => at most 16,777,216 tets per call
 constexpr size_t kNoAllocScratchBytes = sizeof(double) * kNoAllocMaxChunks + 256;
 // Held by every GPU that loads the library, until exit (128 KB + 256 B).
@@ -380,7 +377,7 @@ __global__ void k_tet_energy_noalloc(int T, const int4* __restrict__ tet, const 
                                      unsigned char* __restrict__ scratch) {
     double* chunk_E = reinterpret_cast<double*>(scratch);
     int* bad_flag = reinterpret_cast<int*>(scratch + sizeof(double) * kNoAllocMaxChunks);
-    const int begin = blockIdx.x * kChunk, end = min(T, begin + kChunk);
+    const int begin = blockIdx.x * kNoAllocChunk, end = min(T, begin + kNoAllocChunk);
     double acc = 0.0;
     int bad = 0;
     for (int t = begin + threadIdx.x; t < end; t += blockDim.x) {
@@ -458,7 +455,7 @@ extern "C" int idp_tet_energy_noalloc(int T, const int32_t* tets, const double* 
     using namespace idp;
     if (T < 0 || !energy || !inverted) return IDP_ERR_INVALID_ARG;
     if (T > 0 && (!tets || !X || !IB || !vol || !lam || !mu)) return IDP_ERR_INVALID_ARG;
-    if ((long)T > (long)kNoAllocMaxChunks * kChunk) return IDP_ERR_CAPACITY;
+    if ((long)T > (long)kNoAllocMaxChunks * kNoAllocChunk) return IDP_ERR_CAPACITY;
     int dev = 0;
     if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= kNoAllocMaxDevices) return IDP_ERR_CUDA;
     unsigned char* scratch = nullptr;
@@ -478,7 +475,7 @@ extern "C" int idp_tet_energy_noalloc(int T, const int32_t* tets, const double* 
         scratch = g_noalloc_addr[dev];
     }
     cudaStream_t s = static_cast<cudaStream_t>(stream);
-    const int nchunks = (T + kChunk - 1) / kChunk;
+    const int nchunks = (T + kNoAllocChunk - 1) / kNoAllocChunk;
     if (cudaMemsetAsync(scratch + sizeof(double) * kNoAllocMaxChunks, 0, sizeof(int), s) != cudaSuccess)
         return IDP_ERR_CUDA;
     if (nchunks > 0)

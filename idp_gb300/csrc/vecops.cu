@@ -26,20 +26,12 @@ __global__ void k_copy_masked(long V, const int* __restrict__ vinst, const unsig
 }
 
 __global__ void k_dir_norm2(const Chunk* __restrict__ chunks, const unsigned char* __restrict__ active,
-                            const double* __restrict__ dir, double* __restrict__ part) {
-    __shared__ double sh[kBlock];
-    Chunk c = chunks[blockIdx.x];
+                            const double* __restrict__ dir, InstSum sum) {
+    const Chunk c = chunks[blockIdx.x];
     double acc = 0;
     if (active[c.inst])
-        for (int v = c.begin + threadIdx.x; v < c.end; v += blockDim.x)
-            for (int d = 0; d < 3; ++d) acc += dir[3 * v + d] * dir[3 * v + d];
-    sh[threadIdx.x] = acc;
-    __syncthreads();
-    for (int st = kBlock / 2; st > 0; st >>= 1) {
-        if (threadIdx.x < st) sh[threadIdx.x] += sh[threadIdx.x + st];
-        __syncthreads();
-    }
-    if (threadIdx.x == 0) part[blockIdx.x] = sh[0];
+        for (int k = 3 * c.begin + threadIdx.x; k < 3 * c.end; k += blockDim.x) acc += dir[k] * dir[k];
+    inst_sum(sum, c.inst, acc);
 }
 
 __global__ void k_velocity(long V, const int* __restrict__ vinst, const unsigned char* __restrict__ active,
@@ -131,10 +123,10 @@ int vec_copy_masked(Arena& A, const unsigned char* mask, const double* src, doub
 }
 
 int vec_dir_norm2(Arena& A, Work& W, const double* dir, double* inst_out, cudaStream_t s) {
-    if (W[W_CHUNK_SUM].ensure(sizeof(double) * (A.n_vert_chunks + A.n_tet_chunks + 2))) return IDP_ERR_CUDA;
-    double* part = W[W_CHUNK_SUM].as<double>();
-    (::idp::count_launch(), k_dir_norm2<<<A.n_vert_chunks, kBlock, 0, s>>>(A.vert_chunks, A.active, dir, part));
-    return chunk_reduce_off(A, A.vert_chunk_off, part, inst_out, false, s);
+    InstSum r;
+    if (int rc = inst_sum_args(A, W, A.vert_chunk_off, A.n_vert_chunks, 1, inst_out, false, r, s)) return rc;
+    (::idp::count_launch(), k_dir_norm2<<<A.n_vert_chunks, kBlock, 0, s>>>(A.vert_chunks, A.active, dir, r));
+    return cudaGetLastError() == cudaSuccess ? IDP_OK : IDP_ERR_CUDA;
 }
 
 int vec_velocity(Arena& A, const double* X, const double* Xn, double h, double* v, cudaStream_t s) {
