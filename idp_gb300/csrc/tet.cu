@@ -79,15 +79,14 @@ __global__ void k_tet_energy(const Chunk* __restrict__ chunks, const unsigned ch
     inst_sum(sum, c.inst, acc);
 }
 
-// PK1 stress times IB^T per corner (12 doubles per tet)
-__global__ void k_tet_gradient(long T, const int* __restrict__ tinst, const unsigned char* __restrict__ active,
-                               const double* __restrict__ X, const int4* __restrict__ tet,
+// PK1 stress times IB^T per corner (12 doubles per tet; stored through shared
+// memory so that a warp writes whole lines)
+__global__ void k_tet_gradient(long T, const double* __restrict__ X, const int4* __restrict__ tet,
                                const double* __restrict__ IB, const double* __restrict__ vol,
                                const double* __restrict__ lam, const double* __restrict__ mu, double w,
                                double* __restrict__ out) {
-    long t = (long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= T) return;
-    if (tinst && !active[tinst[t]]) return;
+    __shared__ double st[kBlock * 13];  // 12 values per tet, odd stride
+    const long t0 = (long)blockIdx.x * blockDim.x, t = min(t0 + threadIdx.x, T - 1);
     double F[9];
     const double* B = IB + 9 * t;
     load_F(X, tet[t], B, F);
@@ -110,9 +109,11 @@ __global__ void k_tet_gradient(long T, const int* __restrict__ tinst, const unsi
         for (int d = 0; d < 3; ++d) r[3 * (a + 1) + d] = B[a * 3 + 0] * P[d * 3 + 0] + B[a * 3 + 1] * P[d * 3 + 1] + B[a * 3 + 2] * P[d * 3 + 2];
 #pragma unroll
     for (int d = 0; d < 3; ++d) r[d] = -r[3 + d] - r[6 + d] - r[9 + d];
-    double* o = out + 12 * t;
 #pragma unroll
-    for (int k = 0; k < 12; ++k) o[k] = r[k];
+    for (int k = 0; k < 12; ++k) st[threadIdx.x * 13 + k] = r[k];
+    __syncthreads();
+    const long n = 12 * min((long)blockDim.x, T - t0);
+    for (int k = threadIdx.x; k < n; k += blockDim.x) out[12 * t0 + k] = st[(k / 12) * 13 + k % 12];
 }
 
 // ---- 3x3 symmetric eigen-decomposition by cyclic Jacobi (fixed sweeps)
@@ -228,6 +229,26 @@ __device__ __forceinline__ void rank1(T H[90], T lambda, const T g[12]) {
         }
 }
 
+// rank-1 update of the 6 upper 3x3 blocks of vertices 1..3 with lambda * g g^T
+// (g: their 9 components; the blocks of vertex 0 follow from the zero row sums)
+template <class T>
+__device__ __forceinline__ void rank1_inner(T H[54], T lambda, const T g[9]) {
+    if (lambda <= T(0)) return;
+    int k = 0;
+#pragma unroll
+    for (int a = 0; a < 3; ++a)
+#pragma unroll
+        for (int b = a; b < 3; ++b) {
+#pragma unroll
+            for (int d = 0; d < 3; ++d) {
+                T ga = lambda * g[3 * a + d];
+#pragma unroll
+                for (int e = 0; e < 3; ++e) H[k * 9 + d * 3 + e] += ga * g[3 * b + e];
+            }
+            ++k;
+        }
+}
+
 // g = dF/dx^T vec(Q) for Q = U * C * V^T given as a dense 3x3
 template <class T>
 __device__ __forceinline__ void mode_grad(const T Q[9], const T B[9], T g[12]) {
@@ -239,15 +260,80 @@ __device__ __forceinline__ void mode_grad(const T Q[9], const T B[9], T g[12]) {
     for (int d = 0; d < 3; ++d) g[d] = -g[3 + d] - g[6 + d] - g[9 + d];
 }
 
+// the same for vertices 1..3 alone
 template <class T>
-__global__ void k_tet_hessian(long T_, const int* __restrict__ tinst, const unsigned char* __restrict__ active,
-                              const double* __restrict__ X, const int4* __restrict__ tet,
+__device__ __forceinline__ void mode_grad_inner(const T Q[9], const T B[9], T g[9]) {
+#pragma unroll
+    for (int m = 0; m < 3; ++m)
+#pragma unroll
+        for (int d = 0; d < 3; ++d) g[3 * m + d] = Q[d * 3] * B[m * 3] + Q[d * 3 + 1] * B[m * 3 + 1] + Q[d * 3 + 2] * B[m * 3 + 2];
+}
+
+// FP64 (bound by its pipe): the 54 values of vertices 1..3 and the others from
+// the zero row sums, and no eigenvectors of the A block where it is positive
+// definite. FP32 keeps its sums of all 90 values.
+template <class T>
+struct HessAcc {
+    static constexpr bool inner = sizeof(T) == 8;
+    T H[inner ? 54 : 90];
+    __device__ __forceinline__ HessAcc() {
+#pragma unroll
+        for (int k = 0; k < (inner ? 54 : 90); ++k) H[k] = T(0);
+    }
+    __device__ __forceinline__ void add(T lambda, const T Q[9], const T B[9]) {
+        if constexpr (inner) {
+            T g[9];
+            mode_grad_inner(Q, B, g);
+            rank1_inner(H, lambda, g);
+        } else {
+            T g[12];
+            mode_grad(Q, B, g);
+            rank1(H, lambda, g);
+        }
+    }
+    // the 10 upper blocks (a, b), a <= b, of vertices 0..3
+    __device__ __forceinline__ void store(T* o) const {
+        if constexpr (!inner) {
+#pragma unroll
+            for (int k = 0; k < 90; ++k) o[k] = H[k];
+        } else {
+            // H holds (1,1) (1,2) (1,3) (2,2) (2,3) (3,3)
+#pragma unroll
+            for (int d = 0; d < 3; ++d)
+#pragma unroll
+                for (int e = 0; e < 3; ++e) {
+                    const int q = 3 * d + e, qt = 3 * e + d;
+                    o[9 + q] = -(H[q] + H[9 + qt] + H[18 + qt]);       // (0,1)
+                    o[18 + q] = -(H[9 + q] + H[27 + q] + H[36 + qt]);  // (0,2)
+                    o[27 + q] = -(H[18 + q] + H[36 + q] + H[45 + q]);  // (0,3)
+                }
+#pragma unroll
+            for (int d = 0; d < 3; ++d)
+#pragma unroll
+                for (int e = 0; e < 3; ++e) {  // (0,0), symmetric
+                    const T x = o[9 + 3 * d + e] + o[18 + 3 * d + e] + o[27 + 3 * d + e];
+                    const T y = o[9 + 3 * e + d] + o[18 + 3 * e + d] + o[27 + 3 * e + d];
+                    o[3 * d + e] = T(-0.5) * (x + y);
+                }
+#pragma unroll
+            for (int k = 0; k < 27; ++k) o[36 + k] = H[k];
+#pragma unroll
+            for (int k = 0; k < 27; ++k) o[63 + k] = H[27 + k];
+        }
+    }
+};
+
+// tets per CTA of the Hessian kernel: their 90 values each are stored through
+// shared memory (odd stride), so that a warp writes whole lines
+constexpr int kHessTets = 64;
+
+template <class T>
+__global__ void __launch_bounds__(kHessTets) k_tet_hessian(long T_, const double* __restrict__ X, const int4* __restrict__ tet,
                               const double* __restrict__ IB, const double* __restrict__ vol,
                               const double* __restrict__ lam, const double* __restrict__ mu, double w,
                               T* __restrict__ out) {
-    long t = (long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= T_) return;
-    if (tinst && !active[tinst[t]]) return;
+    __shared__ T st[kHessTets * 91];
+    const long t0 = (long)blockIdx.x * kHessTets, t = min(t0 + threadIdx.x, T_ - 1);
     double Fd[9];
     load_F(X, tet[t], IB + 9 * t, Fd);
     T F[9], B[9];
@@ -268,13 +354,23 @@ __global__ void k_tet_hessian(long T_, const int* __restrict__ tinst, const unsi
     A[1] = A[3] = l / (S[0] * S[1]);
     A[5] = A[7] = l / (S[1] * S[2]);
     A[2] = A[6] = l / (S[2] * S[0]);
+    HessAcc<T> acc;
+    T Q[9];
+    // A-block modes: Q = U diag(e) V^T with A = sum of weight * e e^T: its
+    // eigenvectors, negative weights dropped; in FP64, where A is positive
+    // definite, the columns of its LDL^T
     T aw[3], aV[9];
-    eig3(A, aw, aV);
-    T H[90];
-#pragma unroll
-    for (int k = 0; k < 90; ++k) H[k] = T(0);
-    T Q[9], g[12];
-    // A-block modes: Q = U diag(e) V^T
+    bool pd = false;
+    if constexpr (HessAcc<T>::inner) {
+        const T l10 = A[3] / A[0], l20 = A[6] / A[0], D1 = A[4] - l10 * A[3], a21 = A[7] - l20 * A[3];
+        const T l21 = a21 / D1, D2 = A[8] - l20 * A[6] - l21 * a21;
+        pd = A[0] > T(0) && D1 > T(0) && D2 > T(0);
+        aw[0] = A[0]; aw[1] = D1; aw[2] = D2;
+        aV[0] = T(1); aV[3] = l10; aV[6] = l20;
+        aV[1] = T(0); aV[4] = T(1); aV[7] = l21;
+        aV[2] = T(0); aV[5] = T(0); aV[8] = T(1);
+    }
+    if (!pd) eig3(A, aw, aV);
 #pragma unroll
     for (int m = 0; m < 3; ++m) {
         T e0 = aV[0 * 3 + m], e1 = aV[1 * 3 + m], e2 = aV[2 * 3 + m];
@@ -282,8 +378,7 @@ __global__ void k_tet_hessian(long T_, const int* __restrict__ tinst, const unsi
         for (int i = 0; i < 3; ++i)
 #pragma unroll
             for (int j = 0; j < 3; ++j) Q[i * 3 + j] = U[i * 3] * e0 * V[j * 3] + U[i * 3 + 1] * e1 * V[j * 3 + 1] + U[i * 3 + 2] * e2 * V[j * 3 + 2];
-        mode_grad(Q, B, g);
-        rank1(H, wv * aw[m], g);
+        acc.add(wv * aw[m], Q, B);
     }
     // pair modes (i, j) = (0,1), (1,2), (2,0)
     const T middle = u - l * lp;
@@ -303,13 +398,13 @@ __global__ void k_tet_hessian(long T_, const int* __restrict__ tinst, const unsi
             for (int r = 0; r < 3; ++r)
 #pragma unroll
                 for (int q = 0; q < 3; ++q) Q[r * 3 + q] = rs2 * (U[r * 3 + i] * V[q * 3 + j] + sj * U[r * 3 + j] * V[q * 3 + i]);
-            mode_grad(Q, B, g);
-            rank1(H, wv * lamk, g);
+            acc.add(wv * lamk, Q, B);
         }
     }
-    T* o = out + 90 * t;
-#pragma unroll
-    for (int k = 0; k < 90; ++k) o[k] = H[k];
+    acc.store(st + threadIdx.x * 91);
+    __syncthreads();
+    const long n = 90 * min((long)kHessTets, T_ - t0);
+    for (int k = threadIdx.x; k < n; k += kHessTets) out[90 * t0 + k] = st[(k / 90) * 91 + k % 90];
 }
 
 }  // namespace
@@ -325,7 +420,8 @@ int tet_energy(Arena& A, Work& W, const double* X, double w_h2, double* inst_E, 
 int tet_gradient(Arena& A, Work& W, const double* X, double w_h2, double* g_corners_unused, cudaStream_t s) {
     (void)g_corners_unused;
     if (W[W_TET_GRAD].ensure(sizeof(double) * 12 * (A.T + 1))) return IDP_ERR_CUDA;
-    (::idp::count_launch(), k_tet_gradient<<<grid_for(A.T), kBlock, 0, s>>>(A.T, nullptr, A.active, X, A.tet, A.IB, A.vol, A.lam, A.mu, w_h2,
+    if (A.T <= 0) return IDP_OK;
+    (::idp::count_launch(), k_tet_gradient<<<grid_for(A.T), kBlock, 0, s>>>(A.T, X, A.tet, A.IB, A.vol, A.lam, A.mu, w_h2,
                                                      W[W_TET_GRAD].as<double>()));
     return cudaGetLastError() == cudaSuccess ? IDP_OK : IDP_ERR_CUDA;
 }
@@ -334,12 +430,13 @@ int tet_hessian(Arena& A, Work& W, const double* X, double w_h2, bool fp64, cuda
     size_t el = fp64 ? sizeof(double) : sizeof(float);
     // element blocks: 10 per tet, then 6 per elastic-shell face and 10 per hinge
     if (W[W_TET_HESS].ensure(el * 9 * (10 * (A.T + 1) + 6 * A.Fm + 10 * A.Hn))) return IDP_ERR_CUDA;
+    if (A.T <= 0) return IDP_OK;
     if (fp64)
-        (::idp::count_launch(), k_tet_hessian<double><<<grid_for(A.T, 128), 128, 0, s>>>(A.T, nullptr, A.active, X, A.tet, A.IB, A.vol, A.lam,
-                                                                  A.mu, w_h2, W[W_TET_HESS].as<double>()));
+        (::idp::count_launch(), k_tet_hessian<double><<<grid_for(A.T, kHessTets), kHessTets, 0, s>>>(
+                                    A.T, X, A.tet, A.IB, A.vol, A.lam, A.mu, w_h2, W[W_TET_HESS].as<double>()));
     else
-        (::idp::count_launch(), k_tet_hessian<float><<<grid_for(A.T, 128), 128, 0, s>>>(A.T, nullptr, A.active, X, A.tet, A.IB, A.vol, A.lam,
-                                                                 A.mu, w_h2, W[W_TET_HESS].as<float>()));
+        (::idp::count_launch(), k_tet_hessian<float><<<grid_for(A.T, kHessTets), kHessTets, 0, s>>>(
+                                    A.T, X, A.tet, A.IB, A.vol, A.lam, A.mu, w_h2, W[W_TET_HESS].as<float>()));
     return cudaGetLastError() == cudaSuccess ? IDP_OK : IDP_ERR_CUDA;
 }
 
