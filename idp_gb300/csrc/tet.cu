@@ -41,19 +41,6 @@ __device__ __forceinline__ T det3(const T F[9]) {
     return F[0] * (F[4] * F[8] - F[5] * F[7]) - F[1] * (F[3] * F[8] - F[5] * F[6]) + F[2] * (F[3] * F[7] - F[4] * F[6]);
 }
 
-__device__ double block_sum(double v) {
-    __shared__ double sh[kBlock];
-    sh[threadIdx.x] = v;
-    __syncthreads();
-    for (int st = kBlock / 2; st > 0; st >>= 1) {
-        if (threadIdx.x < st) sh[threadIdx.x] += sh[threadIdx.x + st];
-        __syncthreads();
-    }
-    double r = sh[0];
-    __syncthreads();
-    return r;
-}
-
 // one CTA per chunk of tets of one instance
 __global__ void k_tet_energy(const Chunk* __restrict__ chunks, const unsigned char* __restrict__ active,
                              const double* __restrict__ X, const int4* __restrict__ tet, const double* __restrict__ IB,
@@ -456,30 +443,35 @@ namespace {
 // frame after another), or a latency-bound loop that cannot afford the
 // device-wide synchronisation cudaMalloc/cudaFree imply. For them this entry
 // point evaluates w * sum_t vol_t * Psi(F_t) over caller-owned device arrays
-// with the same per-tet arithmetic and the same reduction order as the
-// arena path (CTA tree per 1024-tet chunk, then the chunk sums in order),
-// using only the fixed scratch below for the chunk sums and the inversion
-// flag.
-constexpr int kNoAllocChunk = 1024;       // tets per chunk
-constexpr int kNoAllocMaxChunks = 16384;  // => at most 16,777,216 tets per call
+// with the same per-tet arithmetic as the arena path, using only the fixed
+// scratch below. One launch: a thread per tet in CTAs of 64 (a mesh of 10,000
+// tets fills every SM; CTAs of 1024 tets left all but ten idle and took 33 us),
+// larger chunks once there would be more than kNoAllocMaxChunks of them, and the
+// last CTA to finish adds the chunk sums in a fixed order and clears the
+// scratch's counter and flag for the next call.
+constexpr int kNoAllocThreads = 64;
+constexpr int kNoAllocMaxChunks = 16384;
+constexpr long kNoAllocMaxTets = 16777216;  // per call
 constexpr size_t kNoAllocScratchBytes = sizeof(double) * kNoAllocMaxChunks + 256;
 // Held by every GPU that loads the library, until exit (128 KB + 256 B).
-// Every call shares it and the last call's contents stay: the flag word is
-// cleared at the start of each call, the chunk sums are overwritten.
+// Every call shares it: chunk sums (overwritten), inversion flag and arrival
+// counter (zero when the library is loaded, and again after every call).
 static __device__ __align__(256) unsigned char g_tet_energy_scratch[kNoAllocScratchBytes];
 
-__global__ void k_tet_energy_noalloc(int T, const int4* __restrict__ tet, const double* __restrict__ X,
-                                     const double* __restrict__ IB, const double* __restrict__ vol,
-                                     const double* __restrict__ lam, const double* __restrict__ mu, double w,
-                                     unsigned char* __restrict__ scratch) {
+__global__ void __launch_bounds__(kNoAllocThreads) k_tet_energy_noalloc(
+    int T, int chunk, const int4* __restrict__ tet, const double* __restrict__ X, const double* __restrict__ IB,
+    const double* __restrict__ vol, const double* __restrict__ lam, const double* __restrict__ mu, double w,
+    unsigned char* __restrict__ scratch, double* __restrict__ energy, int* __restrict__ inverted) {
+    __shared__ bool last;
     double* chunk_E = reinterpret_cast<double*>(scratch);
     int* bad_flag = reinterpret_cast<int*>(scratch + sizeof(double) * kNoAllocMaxChunks);
-    const int begin = blockIdx.x * kNoAllocChunk, end = min(T, begin + kNoAllocChunk);
+    unsigned int* counter = reinterpret_cast<unsigned int*>(bad_flag + 1);
+    const long begin = (long)blockIdx.x * chunk, end = min((long)T, begin + chunk);
     double acc = 0.0;
     int bad = 0;
-    for (int t = begin + threadIdx.x; t < end; t += blockDim.x) {
+    for (long t = begin + threadIdx.x; t < end; t += kNoAllocThreads) {
         double F[9];
-        load_F(X, tet[t], IB + 9 * (long)t, F);
+        load_F(X, tet[t], IB + 9 * t, F);
         double J = det3(F);
         if (J <= 0) { bad = 1; continue; }
         double f2 = 0;
@@ -489,19 +481,25 @@ __global__ void k_tet_energy_noalloc(int T, const int4* __restrict__ tet, const 
         double m = mu[t], l = lam[t];
         acc += w * vol[t] * (m / 2.0 * (f2 - 3.0) - (m - l / 2.0 * lJ) * lJ);
     }
-    double s = block_sum(acc);
     if (bad) *bad_flag = 1;
-    if (threadIdx.x == 0) chunk_E[blockIdx.x] = s;
-}
-
-__global__ void k_tet_energy_noalloc_sum(int nchunks, const unsigned char* __restrict__ scratch,
-                                         double* __restrict__ energy, int* __restrict__ inverted) {
-    const double* chunk_E = reinterpret_cast<const double*>(scratch);
-    const int* bad_flag = reinterpret_cast<const int*>(scratch + sizeof(double) * kNoAllocMaxChunks);
-    double s = 0;
-    for (int c = 0; c < nchunks; ++c) s += chunk_E[c];
-    *energy = s;
-    *inverted = *bad_flag;
+    const double s = cta_sum_fixed(acc);  // its barriers order the flag before the arrival
+    if (threadIdx.x == 0) {
+        chunk_E[blockIdx.x] = s;
+        __threadfence();
+        last = atomicAdd(counter, 1u) == gridDim.x - 1;
+    }
+    __syncthreads();
+    if (!last) return;
+    __threadfence();
+    double a = 0;
+    for (int k = threadIdx.x; k < (int)gridDim.x; k += kNoAllocThreads) a += __ldcg(chunk_E + k);
+    a = cta_sum_fixed(a);
+    if (threadIdx.x == 0) {
+        *energy = a;
+        *inverted = __ldcg(bad_flag);
+        *bad_flag = 0;
+        *counter = 0;
+    }
 }
 
 // Device address of the scratch array, looked up once per device and
@@ -552,7 +550,7 @@ extern "C" int idp_tet_energy_noalloc(int T, const int32_t* tets, const double* 
     using namespace idp;
     if (T < 0 || !energy || !inverted) return IDP_ERR_INVALID_ARG;
     if (T > 0 && (!tets || !X || !IB || !vol || !lam || !mu)) return IDP_ERR_INVALID_ARG;
-    if ((long)T > (long)kNoAllocMaxChunks * kNoAllocChunk) return IDP_ERR_CAPACITY;
+    if ((long)T > kNoAllocMaxTets) return IDP_ERR_CAPACITY;
     int dev = 0;
     if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= kNoAllocMaxDevices) return IDP_ERR_CUDA;
     unsigned char* scratch = nullptr;
@@ -572,13 +570,11 @@ extern "C" int idp_tet_energy_noalloc(int T, const int32_t* tets, const double* 
         scratch = g_noalloc_addr[dev];
     }
     cudaStream_t s = static_cast<cudaStream_t>(stream);
-    const int nchunks = (T + kNoAllocChunk - 1) / kNoAllocChunk;
-    if (cudaMemsetAsync(scratch + sizeof(double) * kNoAllocMaxChunks, 0, sizeof(int), s) != cudaSuccess)
-        return IDP_ERR_CUDA;
-    if (nchunks > 0)
-        (::idp::count_launch(),
-         k_tet_energy_noalloc<<<nchunks, kBlock, 0, s>>>(T, reinterpret_cast<const int4*>(tets), X, IB, vol, lam, mu,
-                                                         weight, scratch));
-    (::idp::count_launch(), k_tet_energy_noalloc_sum<<<1, 1, 0, s>>>(nchunks, scratch, energy, inverted));
+    int chunk = kNoAllocThreads;
+    while ((T + (long)chunk - 1) / chunk > kNoAllocMaxChunks) chunk *= 2;
+    const int nchunks = T > 0 ? (T + chunk - 1) / chunk : 1;
+    (::idp::count_launch(),
+     k_tet_energy_noalloc<<<nchunks, kNoAllocThreads, 0, s>>>(T, chunk, reinterpret_cast<const int4*>(tets), X, IB, vol,
+                                                             lam, mu, weight, scratch, energy, inverted));
     return cudaGetLastError() == cudaSuccess ? IDP_OK : IDP_ERR_CUDA;
 }

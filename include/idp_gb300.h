@@ -431,8 +431,8 @@ int idp_newton_direction(idp_ctx* ctx, int inst, const double* X, double* p, int
  * whole GPU budget up front and lends the library only its own buffers, or a
  * frame loop that cannot take the device-wide synchronisation of
  * cudaMalloc/cudaFree). No counterpart in the reference; it gives the same
- * number as idp_eval_energy's elastic term (same per-tet arithmetic and
- * reduction order) for a context-free caller.
+ * number as idp_eval_energy's elastic term to rounding (same per-tet arithmetic,
+ * another fixed order of the sum) for a context-free caller.
  *   tets (4T int32), X (3V), IB (9T, row-major inverse rest basis), vol (T),
  *   lam (T), mu (T): device pointers. energy (1 double) and inverted (1 int32,
  *   set to 1 when some det F <= 0) are device pointers written by the call.
