@@ -23,6 +23,7 @@
 #include "far.cuh"
 #include "geom.cuh"
 #include "prims.cuh"
+#include "serial_sum.cuh"
 
 namespace idp {
 
@@ -74,7 +75,12 @@ __global__ void k_span_tiles(const SpanTile* __restrict__ tiles, const unsigned 
     if (threadIdx.x == 0) out[blockIdx.x] = a[0];
 }
 
-constexpr int kStageTile = 1024;  // items staged in shared memory per step (multiple of 8)
+constexpr int kSumThreads = 256;  // of the kernels that call it: eight warps
+
+struct StrideItems {
+    const double* __restrict__ x;
+    __device__ double operator()(long i) const { return __ldg(x + 8 * i); }
+};
 
 // Sum of x[0..n) in the order of Eigen's vectorised redux of a dense double
 // vector on the reference's AVX build (`eLen.mean()`, SPATIAL_HASH.h:455-464;
@@ -83,31 +89,17 @@ constexpr int kStageTile = 1024;  // items staged in shared memory per step (mul
 // items 4+l, 12+l, ... over the first 8*floor(n/8) items; the accumulators
 // are added lane by lane, one more 4-item packet is added when n mod 8 >= 4,
 // the lanes reduce as (l0 + l2) + (l1 + l3) and the last n mod 4 items follow
-// one at a time; fewer than 4 items are summed left to right. The whole CTA
-// stages the items through shared memory (double-buffered tiles); threads
-// 0-7 carry the eight accumulator lanes. Every thread must call it; thread 0
+// one at a time; fewer than 4 items are summed left to right. Warp l of the
+// CTA's eight forms accumulator lane l. Every thread must call it; thread 0
 // receives the result.
-__device__ double cta_eigen_sum(const double* __restrict__ x, long n, double (*buf)[kStageTile]) {
-    const int tid = threadIdx.x;
+__device__ double cta_eigen_sum(const double* __restrict__ x, long n) {
+    const int tid = threadIdx.x, warp = tid >> 5;
     const long aligned = n & ~3L, aligned2 = n & ~7L;
     double acc = 0.0;
-    if (aligned > 4) {
-        for (long base = 0, k = 0; base < aligned2; base += kStageTile, ++k) {
-            double* t = buf[k & 1];
-            const long m = min((long)kStageTile, aligned2 - base);
-            for (long i = tid; i < m; i += blockDim.x) t[i] = x[base + i];
-            __syncthreads();
-            if (tid < 8) {
-#pragma unroll 8
-                for (long i = tid; i < m; i += 8) acc += t[i];
-            }
-        }
-        __syncthreads();
-    } else if (aligned == 4 && tid < 4) {
-        acc = x[tid];
-    }
+    if (aligned > 4) acc = serial_sum<1>(StrideItems{x + warp}, aligned2 / 8);
+    else if (aligned == 4 && warp < 4) acc = x[warp];
     __shared__ double lanes[8];
-    if (tid < 8) lanes[tid] = acc;
+    if ((tid & 31) == 0) lanes[warp] = acc;
     __syncthreads();
     double res = 0.0;
     if (tid == 0) {
@@ -129,27 +121,6 @@ __device__ double cta_eigen_sum(const double* __restrict__ x, long n, double (*b
     }
     __syncthreads();
     return res;
-}
-
-// x(0) + x(1) + ... + x(n-1) added left to right into one accumulator (the
-// reference's serial loop), the items staged through shared memory by the
-// whole CTA while thread 0 adds the previous tile. Every thread must call
-// it; thread 0 receives the result.
-__device__ double cta_serial_sum(const AbsDir x, long n, double (*buf)[kStageTile]) {
-    const int tid = threadIdx.x;
-    double acc = 0.0;
-    for (long base = 0, k = 0; base < n; base += kStageTile, ++k) {
-        double* t = buf[k & 1];
-        const long m = min((long)kStageTile, n - base);
-        for (long i = tid; i < m; i += blockDim.x) t[i] = x(base + i);
-        __syncthreads();
-        if (tid == 0) {
-#pragma unroll 8
-            for (long i = 0; i < m; ++i) acc += t[i];
-        }
-    }
-    __syncthreads();
-    return acc;
 }
 
 // fixed-order sum of the tile sums (used for the span-cap estimate only)
@@ -189,18 +160,16 @@ __device__ double cta_tree_sum(const double* x, long n, double* scratch) {
 
 // per instance: voxel size and span cap (SPATIAL_HASH.h:455-482). The voxel
 // size is the Eigen-order mean edge length. pSize is the reference's serial
-// sum; it only matters when the span exceeds 1, so it is computed (by one
-// thread, 3 Sn dependent additions) only when a fixed-order estimate of the
-// span is within the two sums' rounding-error bound ((n + 32) u) of 1 or
-// above it.
+// sum; it only matters when the span exceeds 1, so it is computed only when a
+// fixed-order estimate of the span is within the two sums' rounding-error bound
+// ((n + 32) u) of 1 or above it.
 // voxel size per instance: the mean surface edge length at X, summed in the
 // reference's order (SPATIAL_HASH.h:455-465, Eigen's mean())
 __global__ void k_mean_edge(int nI, const int* __restrict__ se_off, const double* __restrict__ len,
                             double* __restrict__ voxel_size) {
-    __shared__ double buf[2][kStageTile];
     const int i = blockIdx.x;
     const long e0 = se_off[i], ne = se_off[i + 1] - se_off[i];
-    const double es = cta_eigen_sum(len + e0, ne, buf);
+    const double es = cta_eigen_sum(len + e0, ne);
     if (threadIdx.x == 0) voxel_size[i] = ne ? 1.0 * (es / (double)ne) : 1.0;
 }
 
@@ -210,7 +179,6 @@ __global__ void k_span_cap(int nI, const unsigned char* __restrict__ active, con
                            const int* __restrict__ nodes, const double* __restrict__ dir, double* __restrict__ scratch,
                            double* __restrict__ alpha, double* __restrict__ voxel_size,
                            const double* __restrict__ voxel_pre, unsigned long long* __restrict__ bb) {
-    __shared__ double buf[2][kStageTile];
     __shared__ double s_vsz, s_est;
     int i = blockIdx.x;
     if (threadIdx.x < 6) bb[6 * i + threadIdx.x] = threadIdx.x < 3 ? 0xffffffffffffffffull : 0ull;  // empty box
@@ -220,7 +188,7 @@ __global__ void k_span_cap(int nI, const unsigned char* __restrict__ active, con
     const int tn0 = tile_off[2 * i + 1], tn1 = tile_off[2 * i + 2];
     const int ntn = tn1 - tn0;
     double* sc = scratch + 2 * (long)tile_off[2 * i] + 8 * (long)i;
-    const double es = voxel_pre ? 0.0 : cta_eigen_sum(len + e0, ne, buf);
+    const double es = voxel_pre ? 0.0 : cta_eigen_sum(len + e0, ne);
     const double ps = ntn == 0 ? 0.0 : (ntn == 1 ? tsum[tn0] : cta_tree_sum(tsum + tn0, ntn, sc));
     const double cnt = (double)(nn * 3);
     if (threadIdx.x == 0) {
@@ -232,7 +200,7 @@ __global__ void k_span_cap(int nI, const unsigned char* __restrict__ active, con
     double a = alpha[i];
     const double bound = 1.0 - ((double)(3 * nn) + 32.0) * 2.3e-16;
     if (!(s_est < bound)) {
-        double pSize = cta_serial_sum(AbsDir{nodes + n0, dir}, 3 * nn, buf);
+        double pSize = serial_sum<kSumThreads / 32>(AbsDir{nodes + n0, dir}, 3 * nn);
         if (threadIdx.x == 0) {
             pSize /= cnt;
             const double spanSize = a * pSize / vsz;
@@ -770,7 +738,7 @@ int ccd_voxel_size(Arena& A, Work& W, const double* X, cudaStream_t s) {
     if (W[W_CCD_VOX].ensure(sizeof(double) * (Se + nI + 8))) return IDP_ERR_CUDA;
     double* len = W[W_CCD_VOX].as<double>() + nI;
     if (A.Se) (::idp::count_launch(), k_edge_len<<<grid_for(A.Se), kBlock, 0, s>>>(A.Se, A.sedge, X, len));
-    (::idp::count_launch(), k_mean_edge<<<nI, 256, 0, s>>>(nI, A.d_se_off, len, W[W_CCD_VOX].as<double>()));
+    (::idp::count_launch(), k_mean_edge<<<nI, kSumThreads, 0, s>>>(nI, A.d_se_off, len, W[W_CCD_VOX].as<double>()));
     return cudaGetLastError() == cudaSuccess ? IDP_OK : IDP_ERR_CUDA;
 }
 
@@ -801,7 +769,7 @@ int ccd_stepsize(Arena& A, Work& W, const double* X, const double* dir, double* 
     if (A.Se && !voxel_pre) (::idp::count_launch(), k_edge_len<<<grid_for(A.Se), kBlock, 0, s>>>(A.Se, A.sedge, X, len));
     if (A.n_span_tiles > 0)
         (::idp::count_launch(), k_span_tiles<<<A.n_span_tiles, 256, 0, s>>>(A.span_tiles, A.active, A.snode, dir, tsum));
-    (::idp::count_launch(), k_span_cap<<<nI, 256, 0, s>>>(nI, A.active, A.d_se_off, A.d_sn_off, A.span_tile_off, tsum,
+    (::idp::count_launch(), k_span_cap<<<nI, kSumThreads, 0, s>>>(nI, A.active, A.d_se_off, A.d_sn_off, A.span_tile_off, tsum,
                                                           len, A.snode, dir, sumsc, alpha, vsz, voxel_pre, bb));
     // grid
     if (A.Sn)
@@ -846,8 +814,7 @@ int ccd_stepsize(Arena& A, Work& W, const double* X, const double* dir, double* 
             (::idp::count_launch(), k_prim_boxes_from_nodes<<<grid_for(A.St + A.Se), kBlock, 0, s>>>(
                                         A.St, A.Se, A.stri, A.sedge, A.st_inst, A.se_inst, A.active, A.v2s, nbox, gc,
                                         tbox, ebox, tboxc, eboxc, t.cbase, t.cap, t.ccount));
-        rc = grids_build(W, 1, tboxc, A.St, A.st_inst, eboxc, A.Se, A.se_inst, A.active, gc, nI, ccount + 2, gt, ge, s,
-                         t.ccount != nullptr);
+        rc = grids_build(W, 1, tboxc, A.St, A.st_inst, eboxc, A.Se, A.se_inst, A.active, gc, nI, ccount + 2, gt, ge, s);
         if (rc) return rc;
         if (W[W_CAND].ensure(sizeof(CCand) * (cap_pt + cap_ee))) return IDP_ERR_CUDA;
         CCand* cand = W[W_CAND].as<CCand>();

@@ -181,8 +181,7 @@ __global__ void k_box_emit(long n, const BoxI* __restrict__ boxes, const int* __
 // first cell of every instance (prefix of the per-instance cell counts) and
 // the total; one thread, instances are few
 __global__ void k_cell_bases(int nI, const GridP* __restrict__ gp, uint32_t* __restrict__ cbase,
-                             unsigned long long* __restrict__ total, unsigned long long cap,
-                             unsigned int* __restrict__ flag) {
+                             unsigned long long* __restrict__ total) {
     unsigned long long acc = 0;
     for (int i = 0; i < nI; ++i) {
         cbase[i] = (uint32_t)(acc < 0xffffffffull ? acc : 0xffffffffull);
@@ -191,7 +190,6 @@ __global__ void k_cell_bases(int nI, const GridP* __restrict__ gp, uint32_t* __r
     }
     cbase[nI] = (uint32_t)(acc < 0xffffffffull ? acc : 0xffffffffull);
     *total = acc;
-    if (flag && acc > cap) atomicOr(flag, 1u);
 }
 
 // both grids of a broad phase in one pass (boxes [0, nt) are triangles,
@@ -205,18 +203,6 @@ __device__ __forceinline__ bool dense2_box(long i, long nt, const BoxI* __restri
     if (!active[inst]) return false;
     b = grid ? ebox[i - nt] : tbox[i];
     return true;
-}
-
-__global__ void k_dense_count2(long nt, long ne, const BoxI* __restrict__ tbox, const int* __restrict__ tinst,
-                               const BoxI* __restrict__ ebox, const int* __restrict__ einst,
-                               const unsigned char* __restrict__ active, const GridP* __restrict__ gp,
-                               const uint32_t* __restrict__ cbase, uint32_t cap, uint32_t* __restrict__ ccount) {
-    long i = (long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= nt + ne) return;
-    BoxI b;
-    int inst, grid;
-    if (!dense2_box(i, nt, tbox, tinst, ebox, einst, active, b, inst, grid)) return;
-    count_cells(b, gp[inst], cbase[inst], cap, ccount + (size_t)grid * (cap + 1));
 }
 
 __global__ void k_dense_fill2(long nt, long ne, const BoxI* __restrict__ tbox, const int* __restrict__ tinst,
@@ -678,7 +664,7 @@ int grid_cell_bases(Work& W, const GridP* gp, int nI, unsigned long long* h_cell
     uint32_t* cbase = W[W_CBASE].as<uint32_t>();
     unsigned long long* total = reinterpret_cast<unsigned long long*>(W[W_CBASE].as<char>() +
                                                                       ((sizeof(uint32_t) * (nI + 1) + 15) & ~size_t(15)));
-    (::idp::count_launch(), k_cell_bases<<<1, 1, 0, s>>>(nI, gp, cbase, total, ~0ull, nullptr));
+    (::idp::count_launch(), k_cell_bases<<<1, 1, 0, s>>>(nI, gp, cbase, total));
     IDP_CUDA_TRY(cudaMemcpyAsync(h_cells, total, sizeof(unsigned long long), cudaMemcpyDeviceToHost, s));
     return IDP_OK;
 }
@@ -770,13 +756,12 @@ bool grids_overflowed(Work& W, int set, unsigned int flag) {
 
 int grids_build(Work& W, int set, const BoxI* tbox, long nt, const int* tinst, const BoxI* ebox, long ne,
                 const int* einst, const unsigned char* active, const GridP* gp, int nI, unsigned int* d_flag,
-                BoxGrid& gt, BoxGrid& ge, cudaStream_t s, bool counted) {
+                BoxGrid& gt, BoxGrid& ge, cudaStream_t s) {
     if (W[W_CBASE].ensure(sizeof(uint32_t) * (nI + 1) + 64)) return IDP_ERR_CUDA;
     uint32_t* cbase = W[W_CBASE].as<uint32_t>();
-    unsigned long long* d_total = reinterpret_cast<unsigned long long*>(W[W_CBASE].as<char>() +
-                                                                        ((sizeof(uint32_t) * (nI + 1) + 15) & ~size_t(15)));
     if (W.dense_ready[set]) {
-        // dense tables at the capacities of earlier builds, no round trip
+        // dense tables at the capacities of earlier builds, no round trip; the
+        // caller's kernels made the cell bases and counted the boxes (grids_tables)
         const unsigned long long cap = W.dense_cells_cap[set];
         const long ent_cap = W.dense_ent_cap[set];
         const size_t slots = 2 * (size_t)(cap + 1);
@@ -788,13 +773,6 @@ int grids_build(Work& W, int set, const BoxI* tbox, long nt, const int* tinst, c
         uint32_t* ccount = tab.as<uint32_t>();
         uint32_t* cstart = ccount + slots + 1;
         const long n = nt + ne;
-        if (!counted) {
-            (::idp::count_launch(), k_cell_bases<<<1, 1, 0, s>>>(nI, gp, cbase, d_total, cap, d_flag));
-            IDP_CUDA_TRY(cudaMemsetAsync(ccount, 0, sizeof(uint32_t) * slots, s));
-        }
-        if (n > 0 && !counted)
-            (::idp::count_launch(), k_dense_count2<<<grid_for(n), kBlock, 0, s>>>(nt, ne, tbox, tinst, ebox, einst, active,
-                                                                                  gp, cbase, (uint32_t)cap, ccount));
         if (scan_exclusive(ccount, cstart, (long)slots, cstart + slots, W[W_SCRATCH].p, s) != cudaSuccess)
             return IDP_ERR_CUDA;
         if (n > 0)
@@ -853,10 +831,10 @@ int grids_tables(Work& W, int set, int nI, GridTables& t, cudaStream_t s) {
 
 // per-instance grid over the surface at X and the integer boxes of every
 // surface triangle and edge in it; when the tables' capacities are known the
-// cells are counted on the way (counted, d_flag as in grids_build). The FP32
+// cells are counted on the way (d_flag as in grids_build). The FP32
 // positions go to W_XF.
 static int surface_boxes(Arena& A, Work& W, const double* X, GridP*& gp, BoxI*& tbox, BoxI*& ebox,
-                         unsigned int* d_flag, bool& counted, cudaStream_t s) {
+                         unsigned int* d_flag, cudaStream_t s) {
     const int nI = A.nI;
     if (W[W_BBOX].ensure(sizeof(unsigned long long) * 6 * nI) || W[W_GRIDP].ensure(sizeof(GridP) * nI))
         return IDP_ERR_CUDA;
@@ -864,7 +842,6 @@ static int surface_boxes(Arena& A, Work& W, const double* X, GridP*& gp, BoxI*& 
     gp = W[W_GRIDP].as<GridP>();
     GridTables t;
     if (int r = grids_tables(W, 0, nI, t, s)) return r;
-    counted = t.ccount != nullptr;
     if (W[W_XF].ensure(sizeof(float4) * (A.V + 1))) return IDP_ERR_CUDA;
     float4* Xf = W[W_XF].as<float4>();
     (::idp::count_launch(), k_bbox_init<<<grid_for(6 * nI), kBlock, 0, s>>>(nI, bb));
@@ -900,12 +877,11 @@ int build_constraint_set(Arena& A, Work& W, const double* X, ContactSet& cs, cud
         // 1-2. per-instance grid parameters, triangle and edge boxes
         GridP* gp = nullptr;
         BoxI *tbox = nullptr, *ebox = nullptr;
-        bool counted = false;
         IDP_CUDA_TRY(cudaMemsetAsync(ccount, 0, 4 * sizeof(unsigned int), s));
-        if ((rc = surface_boxes(A, W, X, gp, tbox, ebox, ccount + 2, counted, s))) return rc;
+        if ((rc = surface_boxes(A, W, X, gp, tbox, ebox, ccount + 2, s))) return rc;
         BoxGrid gt, ge;
         if ((rc = grids_build(W, 0, tbox, A.St, A.st_inst, ebox, A.Se, A.se_inst, A.active, gp, nI, ccount + 2, gt, ge,
-                              s, counted)))
+                              s)))
             return rc;
         const long rcap = cap_pt + cap_ee;
         if (W[W_CAND].ensure(sizeof(Cand) * rcap) || W[W_CONS_TMP].ensure(sizeof(Rec) * rcap)) return IDP_ERR_CUDA;
@@ -1011,12 +987,11 @@ int edge_tri_intersections(Arena& A, Work& W, const double* X, unsigned int* ins
         GridP* gp = nullptr;
         BoxI *tbox = nullptr, *ebox = nullptr;
         BoxGrid gt, ge;
-        bool counted = false;
         IDP_CUDA_TRY(cudaMemsetAsync(ccount, 0, 3 * sizeof(unsigned int), s));
         IDP_CUDA_TRY(cudaMemsetAsync(inst_count, 0, sizeof(unsigned int) * nI, s));
-        if (int r = surface_boxes(A, W, X, gp, tbox, ebox, ccount + 2, counted, s)) return r;
+        if (int r = surface_boxes(A, W, X, gp, tbox, ebox, ccount + 2, s)) return r;
         if (int r = grids_build(W, 0, tbox, A.St, A.st_inst, ebox, A.Se, A.se_inst, A.active, gp, nI, ccount + 2, gt,
-                                ge, s, counted))
+                                ge, s))
             return r;
         if (W[W_CAND].ensure(sizeof(Cand) * cap)) return IDP_ERR_CUDA;
         Cand* out = W[W_CAND].as<Cand>();

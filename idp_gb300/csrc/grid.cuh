@@ -294,11 +294,11 @@ int box_grid_finish(Work& W, int slot, const BoxI* boxes, const int* inst, const
 // *d_flag (bit 0: more cells, bit 1: more entries than the capacities) what
 // did not fit, and the caller, at its next synchronisation, calls
 // grids_overflowed and rebuilds when it returns true.
-// counted: the caller's kernels already made the cell bases and counted the boxes
-// into grids_tables' counters (only when that returned true).
+// Such a later build needs the cell bases made and the boxes counted into
+// grids_tables' counters by the caller's kernels.
 int grids_build(Work& W, int set, const BoxI* tbox, long nt, const int* tinst, const BoxI* ebox, long ne,
                 const int* einst, const unsigned char* active, const GridP* gp, int nI, unsigned int* d_flag,
-                BoxGrid& gt, BoxGrid& ge, cudaStream_t s, bool counted = false);
+                BoxGrid& gt, BoxGrid& ge, cudaStream_t s);
 // tables of a set whose capacities are known (see grids_build), their counters
 // cleared; false: the set has not been built yet, or not as a dense table
 struct GridTables {
