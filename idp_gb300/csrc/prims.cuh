@@ -1,5 +1,5 @@
-// Device primitives written for this engine: LSD radix sort of (u64 key,
-// u32 value) pairs, exclusive scan of u32 counts, and a fixed-order double
+// Device primitives written for this engine: stable sort of (u64 key, u32
+// value) pairs, exclusive scan of u32 counts, and a fixed-order double
 // sum. All three are deterministic: their results do not depend on thread
 // scheduling.
 #pragma once
@@ -11,9 +11,9 @@ namespace idp {
 size_t radix_sort_scratch_bytes(long n);
 size_t scan_scratch_bytes(long n);
 
-// Stable LSD sort of keys[0..n) (only the low `bits` bits are significant)
+// Stable sort of keys[0..n) (only the low `bits` bits are significant)
 // with values carried along. keys/vals are sorted in place; keys_alt/vals_alt
-// are ping-pong buffers of the same size. scratch must hold
+// are buffers of the same size. scratch must hold
 // radix_sort_scratch_bytes(n).
 cudaError_t radix_sort_pairs(uint64_t* keys, uint32_t* vals, uint64_t* keys_alt, uint32_t* vals_alt, long n,
                              int bits, void* scratch, cudaStream_t s);
