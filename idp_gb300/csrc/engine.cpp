@@ -67,11 +67,13 @@ struct idp_ctx {
     DBuf stage;               // 3V doubles in the caller's vertex order (transfers across the interface)
     DBuf bacc;                // body-force accelerations M^-1 b (3V), when some instance has one
     bool has_bacc = false;
+    std::vector<unsigned char> mask_dev;  // the active mask on the device (empty: unknown)
     bool stepping = false;    // a step is in flight (begun, instances still iterating)
     // side stream: the CCD voxel size of an iteration's positions, computed
     // while the gradient and Hessian of the same positions are
     cudaStream_t s2 = nullptr;
     cudaEvent_t ev_x = nullptr, ev_vox = nullptr;
+    cudaEvent_t ev_norm = nullptr;  // the gradient norms have reached the host
     std::chrono::steady_clock::time_point t_begin;  // the step's begin (latency origin)
 };
 
@@ -197,7 +199,10 @@ double* dsc(idp_ctx* c, int k) { return c->inst_buf.as<double>() + (long)k * c->
 int* isc(idp_ctx* c, int k) { return reinterpret_cast<int*>(c->inst_buf.as<double>() + (long)S_NUMD * c->A.nI) + (long)k * c->A.nI; }
 
 int set_mask(idp_ctx* c, const std::vector<unsigned char>& m) {
+    if (c->mask_dev == m) return IDP_OK;
+    c->mask_dev.clear();
     IDP_CUDA_TRY(cudaMemcpyAsync(c->A.active, m.data(), m.size(), cudaMemcpyHostToDevice, c->s));
+    c->mask_dev = m;
     return IDP_OK;
 }
 
@@ -516,10 +521,12 @@ idp_ctx* idp_create(const idp_params* p, int* status) {
         cudaDeviceGetStreamPriorityRange(&prio_lo, &prio_hi) != cudaSuccess ||
         cudaStreamCreateWithPriority(&c->s2, cudaStreamNonBlocking, prio_hi) != cudaSuccess ||
         cudaEventCreateWithFlags(&c->ev_x, cudaEventDisableTiming) != cudaSuccess ||
-        cudaEventCreateWithFlags(&c->ev_vox, cudaEventDisableTiming) != cudaSuccess) {
+        cudaEventCreateWithFlags(&c->ev_vox, cudaEventDisableTiming) != cudaSuccess ||
+        cudaEventCreateWithFlags(&c->ev_norm, cudaEventDisableTiming) != cudaSuccess) {
         if (c->s) cudaStreamDestroy(c->s);
         if (c->s2) cudaStreamDestroy(c->s2);
         if (c->ev_x) cudaEventDestroy(c->ev_x);
+        if (c->ev_vox) cudaEventDestroy(c->ev_vox);
         delete c;
         if (status) *status = IDP_ERR_CUDA;
         return nullptr;
@@ -541,6 +548,7 @@ void idp_destroy(idp_ctx* c) {
     c->snap.release();
     cudaEventDestroy(c->ev_x);
     cudaEventDestroy(c->ev_vox);
+    cudaEventDestroy(c->ev_norm);
     cudaStreamDestroy(c->s2);
     cudaStreamDestroy(c->s);
     delete c;
@@ -564,6 +572,7 @@ int idp_reset(idp_ctx* c) {
     c->W.stats = idp_stats{};
     c->W.dense_ready[0] = c->W.dense_ready[1] = false;
     c->W.sell.ready = false;
+    c->mask_dev.clear();
     return IDP_OK;
 }
 
@@ -942,6 +951,7 @@ int idp_commit(idp_ctx* c) {
     const int nI = (int)c->inst.size();
     A.nI = nI;
     c->W.sell.ready = false;
+    c->mask_dev.clear();
     A.v_off.assign(nI + 1, 0);
     A.t_off.assign(nI + 1, 0);
     A.f_off.assign(nI + 1, 0);
@@ -1637,12 +1647,17 @@ int step_iterate(idp_ctx* c, int max_iters, idp_result* results, int* n_active) 
         // inexact Newton: PCG tolerance per instance follows |g| / |g_0|
         // (tight near convergence, where the step-length test is decided)
         if ((rc = vec_dir_norm2(A, W, A.g, dsc(c, S_NORM2), s))) return rc;
-        if ((rc = fetch(c, dsc(c, S_NORM2), hv))) return rc;
+        double* hnorm = W.pinned_doubles(2 * (long)nI);
+        if (!hnorm) return IDP_ERR_CUDA;
+        IDP_CUDA_TRY(cudaMemcpyAsync(hnorm, dsc(c, S_NORM2), sizeof(double) * nI, cudaMemcpyDeviceToHost, s));
+        IDP_CUDA_TRY(cudaEventRecord(c->ev_norm, s));
         std::vector<double> tol(nI, c->P.pcg_rel_tol);
-        {
+        // called when the Hessian is enqueued: the wait is over long before it
+        auto tolerances = [&]() -> int {
+            IDP_CUDA_TRY(cudaEventSynchronize(c->ev_norm));
             for (int i = 0; i < nI; ++i) {
                 if (!mask[i]) continue;
-                double gn = std::sqrt(hv[i]);
+                double gn = std::sqrt(hnorm[i]);
                 if (st[i].iters == 0 || !(st[i].g0 > 0)) st[i].g0 = gn;
                 double eta = st[i].g0 > 0 ? gn / st[i].g0 : 1.0;
                 tol[i] = std::max(c->P.pcg_rel_tol, std::min(1e-2, eta));
@@ -1650,7 +1665,8 @@ int step_iterate(idp_ctx* c, int max_iters, idp_result* results, int* n_active) 
                 if (c->inst[i].flow()) tol[i] = c->P.pcg_rel_tol;
             }
             IDP_CUDA_TRY(cudaMemcpyAsync(W.tol_inst, tol.data(), sizeof(double) * nI, cudaMemcpyHostToDevice, s));
-        }
+            return IDP_OK;
+        };
         if ((rc = vec_neg(3 * A.V, A.g, A.g, s))) return rc;  // rhs = -g
         std::vector<unsigned char> newton(nI, 0), gd(nI, 0);
         bool any_newton = false, any_gd = false;
@@ -1662,10 +1678,11 @@ int step_iterate(idp_ctx* c, int max_iters, idp_result* results, int* n_active) 
         if (any_newton) {
             if ((rc = set_mask(c, newton))) return rc;
             if ((rc = eval_hessian(c, A.X))) return rc;
+            if ((rc = tolerances())) return rc;
             std::vector<int> its;
             std::vector<double> rel;
             IDP_CUDA_TRY(cudaStreamWaitEvent(s, c->ev_vox, 0));  // the side stream is idle during the PCG
-            if ((rc = pcg_solve(A, W, c->cs, fp64, A.g, A.dir, c->P.pcg_rel_tol, c->P.pcg_max_iters, its, rel, s,
+            if ((rc = pcg_solve(A, W, c->cs, fp64, A.g, A.dir, c->P.pcg_rel_tol, c->P.pcg_max_iters, newton, its, rel, s,
                                  tol.data())))
                 return rc;
             for (int i = 0; i < nI; ++i)
@@ -1684,8 +1701,8 @@ int step_iterate(idp_ctx* c, int max_iters, idp_result* results, int* n_active) 
                 if (any_fb) {
                     if ((rc = set_mask(c, fb))) return rc;
                     if ((rc = eval_hessian(c, A.X, true))) return rc;
-                    if ((rc = pcg_solve(A, W, c->cs, true, A.g, A.dir, c->P.pcg_rel_tol, c->P.pcg_max_iters, its, rel, s,
-                                         tol.data())))
+                    if ((rc = pcg_solve(A, W, c->cs, true, A.g, A.dir, c->P.pcg_rel_tol, c->P.pcg_max_iters, fb, its, rel,
+                                         s, tol.data())))
                         return rc;
                     for (int i = 0; i < nI; ++i)
                         if (fb[i]) {
@@ -1695,6 +1712,7 @@ int step_iterate(idp_ctx* c, int max_iters, idp_result* results, int* n_active) 
                 }
             }
         }
+        if (!any_newton && (rc = tolerances())) return rc;  // |g_0| is recorded there
         if (any_gd) {  // gradient descent direction (IMPLICIT_EULER.h:507-510)
             if ((rc = set_mask(c, gd))) return rc;
             if ((rc = vec_copy_masked(A, A.active, A.g, A.dir, s))) return rc;
@@ -1707,6 +1725,7 @@ int step_iterate(idp_ctx* c, int max_iters, idp_result* results, int* n_active) 
         std::vector<double> alpha(nI, 1.0);
         // inversion-feasible alpha (halve while any det F <= 0)
         std::vector<unsigned char> srch = mask;
+        int inv_trials = 0;  // its last energies are those of X = Xprev + alpha dir
         for (int trial = 0; trial < 80; ++trial) {
             bool anys = false;
             for (int i = 0; i < nI; ++i) anys |= srch[i] != 0;
@@ -1717,6 +1736,7 @@ int step_iterate(idp_ctx* c, int max_iters, idp_result* results, int* n_active) 
             IDP_CUDA_TRY(cudaMemsetAsync(isc(c, SI_BAD), 0, sizeof(int) * nI, s));
             if ((rc = tet_energy(A, W, A.X, h * h, dsc(c, S_ETET), isc(c, SI_BAD), s))) return rc;
             if ((rc = fetch(c, isc(c, SI_BAD), hi))) return rc;
+            ++inv_trials;
             for (int i = 0; i < nI; ++i) {
                 if (!srch[i]) continue;
                 if (hi[i]) alpha[i] /= 2.0;
@@ -1728,6 +1748,7 @@ int step_iterate(idp_ctx* c, int max_iters, idp_result* results, int* n_active) 
         IDP_CUDA_TRY(cudaMemcpyAsync(A.alpha, alpha.data(), sizeof(double) * nI, cudaMemcpyHostToDevice, s));
         W.timer.start(PhaseTimer::CCD, s);
         hi.resize(nI);
+        const std::vector<double> alpha_inv = alpha;
         rc = ccd_stepsize(A, W, A.Xprev, A.dir, A.alpha, isc(c, SI_CCDF), s, ccd_voxel_sizes(A, W), alpha.data(),
                           hi.data());
         W.timer.stop(s);
@@ -1748,17 +1769,22 @@ int step_iterate(idp_ctx* c, int max_iters, idp_result* results, int* n_active) 
             for (int i = 0; i < nI; ++i) anys |= srch[i] != 0;
             if (!anys) break;
             if ((rc = set_mask(c, srch))) return rc;
-            IDP_CUDA_TRY(cudaMemcpyAsync(A.alpha, alpha.data(), sizeof(double) * nI, cudaMemcpyHostToDevice, s));
-            if ((rc = vec_axpy_trial(A, A.Xprev, A.dir, A.X, s))) return rc;
+            // the CCD left every step as the inversion check's single trial took
+            // it: X, the inversion flags and the elastic energies stand
+            const bool same = trial == 0 && inv_trials == 1 && alpha == alpha_inv;
+            if (!same) {
+                IDP_CUDA_TRY(cudaMemcpyAsync(A.alpha, alpha.data(), sizeof(double) * nI, cudaMemcpyHostToDevice, s));
+                if ((rc = vec_axpy_trial(A, A.Xprev, A.dir, A.X, s))) return rc;
+            }
             // one pass over every searching instance: validity (det F > 0)
             // and elastic energy, inertia, constraint set, minimum distance
             // and barrier energy; one readback decides. An instance that
             // turns out inverted, or fails the distance safeguard, ignores
             // the values computed past that point.
-            IDP_CUDA_TRY(cudaMemsetAsync(isc(c, SI_BAD), 0, sizeof(int) * nI * 2, s));
+            IDP_CUDA_TRY(cudaMemsetAsync(isc(c, same ? SI_BADB : SI_BAD), 0, sizeof(int) * nI * (same ? 1 : 2), s));
             IDP_CUDA_TRY(cudaMemsetAsync(dsc(c, S_EBAR), 0, sizeof(double) * nI, s));
             W.timer.start(PhaseTimer::TET, s);
-            if ((rc = tet_energy(A, W, A.X, h * h, dsc(c, S_ETET), isc(c, SI_BAD), s))) return rc;
+            if (!same && (rc = tet_energy(A, W, A.X, h * h, dsc(c, S_ETET), isc(c, SI_BAD), s))) return rc;
             if ((rc = flow_energy(A, W, A.X, dsc(c, S_ETET), s))) return rc;
             if ((rc = shell_energy(A, W, A.X, h * h, dsc(c, S_ETET), s))) return rc;
             W.timer.stop(s);
@@ -2310,7 +2336,7 @@ int idp_newton_direction(idp_ctx* c, int i, const double* X, double* p, int* ite
     std::vector<int> its;
     std::vector<double> rel;
     if ((rc = pcg_solve(c->A, c->W, c->cs, c->P.mode == IDP_MODE_FP64, c->A.g, c->A.dir, c->P.pcg_rel_tol,
-                        c->P.pcg_max_iters, its, rel, c->s)))
+                        c->P.pcg_max_iters, c->mask_dev, its, rel, c->s)))
         return rc;
     if ((rc = download3(c, i, c->A.dir, p))) return rc;
     IDP_CUDA_TRY(cudaStreamSynchronize(c->s));

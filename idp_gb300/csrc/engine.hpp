@@ -341,6 +341,18 @@ struct Work {
         }
         return hpin_d;
     }
+    int* hpin_i = nullptr;                  // pinned host ints (iteration counts of a PCG in flight)
+    long hpin_i_n = 0;
+    int* pinned_ints(long n) {
+        if (n > hpin_i_n) {
+            if (hpin_i) cudaFreeHost(hpin_i);
+            hpin_i = nullptr;
+            hpin_i_n = 0;
+            if (cudaMallocHost(reinterpret_cast<void**>(&hpin_i), sizeof(int) * (n + 8)) != cudaSuccess) return nullptr;
+            hpin_i_n = n;
+        }
+        return hpin_i;
+    }
     DBuf& operator[](int i) { return b[i]; }
     void release() {
         for (auto& x : b) x.release();
@@ -350,6 +362,9 @@ struct Work {
         if (hpin_d) cudaFreeHost(hpin_d);
         hpin_d = nullptr;
         hpin_d_n = 0;
+        if (hpin_i) cudaFreeHost(hpin_i);
+        hpin_i = nullptr;
+        hpin_i_n = 0;
     }
 };
 
@@ -430,8 +445,9 @@ template <class T>
 int sell_solve(Arena& A, Work& W, const std::vector<int>& which, const double* b, T* x, double rel_tol, int max_iters,
                int* d_iters, int* d_err, cudaStream_t s);
 int pcg_solve(Arena& A, Work& W, const ContactSet& cs, bool fp64, const double* rhs, double* sol,
-              double rel_tol, int max_iters, std::vector<int>& iters_out, std::vector<double>& relres_out,
-              cudaStream_t s, const double* tol_host = nullptr);
+              double rel_tol, int max_iters, const std::vector<unsigned char>& mask /* the active mask on the device */,
+              std::vector<int>& iters_out, std::vector<double>& relres_out, cudaStream_t s,
+              const double* tol_host = nullptr);
 
 // vector helpers (solver.cu)
 int vec_inertia(Arena& A, Work& W, const double* X, double* inst_E, double* g /*nullable*/, cudaStream_t s);

@@ -13,6 +13,7 @@
 // its own scalars and stops on its own). Mixed mode runs PCG in FP32 and
 // recovers the direction by iterative refinement against an FP64 residual
 // r = b - A x (FP32 matrix, FP64 accumulation); FP64 mode runs PCG in FP64.
+#include <algorithm>
 #include <atomic>
 #include <cooperative_groups.h>
 #include "engine.hpp"
@@ -1287,10 +1288,40 @@ int hessian_apply(Arena& A, Work& W, bool fp64, const double* x, double* y, cuda
     return cudaGetLastError() == cudaSuccess ? IDP_OK : IDP_ERR_CUDA;
 }
 
-// PCG on b (FP64 rhs), result added to nothing: x (type T) holds the solution
+// Iteration counts of the instances solved by pcg_sell.cu, read back with the
+// stream's next synchronisation
+struct SellPending {
+    std::vector<int> inst;
+    const int* host = nullptr;  // nI counts, the error flag at nI + 16
+};
+
+// after that synchronisation
 template <class T>
-static int pcg_inner(Arena& A, Work& W, const double* b, double rel_tol, int max_iters, std::vector<int>& iters,
-                     T** xout, cudaStream_t s) {
+static int sell_finish(Arena& A, Work& W, SellPending& pend, std::vector<int>& iters) {
+    if (pend.inst.empty()) return IDP_OK;
+    int most = 0;
+    for (int i : pend.inst) {
+        most = std::max(most, iters[i] = pend.host[i]);
+        W.stats.pcg_iters += iters[i];
+        if ((int)W.pcg_bytes_per_iter.size() == A.nI)
+            W.stats.pcg_bytes += (double)iters[i] * W.pcg_bytes_per_iter[i] * (sizeof(T) / 4.0);
+    }
+    pend.inst.clear();
+    W.sell.tag += (unsigned int)most + 4;  // the tags this solve used
+    if (pend.host[A.nI + 16]) {  // a poll ran out (never expected): its tags are not reused
+        W.sell.xch_bytes = 0;
+        return IDP_ERR_CUDA;
+    }
+    return IDP_OK;
+}
+
+// PCG on b (FP64 rhs) for the instances of act (the mask on the device), result
+// added to nothing: x (type T) holds the solution. iters are final once the
+// stream is synchronised and sell_finish has run.
+template <class T>
+static int pcg_inner(Arena& A, Work& W, const double* b, double rel_tol, int max_iters,
+                     const std::vector<unsigned char>& act, std::vector<int>& iters, SellPending& pend, T** xout,
+                     cudaStream_t s) {
     const int nI = A.nI;
     long n3 = 3 * A.V;
     if (W[W_PCG_VEC].ensure(sizeof(T) * 10 * (n3 + 4))) return IDP_ERR_CUDA;
@@ -1304,9 +1335,7 @@ static int pcg_inner(Arena& A, Work& W, const double* b, double rel_tol, int max
     const T* tval = W[W_TAIL_VAL].as<T>();
     // instances up to W.grid_min_v vertices: one thread-block cluster each,
     // grouped by cluster size (one launch per size); larger ones: grid PCG
-    std::vector<unsigned char> act(nI), small(nI, 0), large(nI, 0);
-    IDP_CUDA_TRY(cudaMemcpyAsync(act.data(), A.active, nI, cudaMemcpyDeviceToHost, s));
-    IDP_CUDA_TRY(cudaStreamSynchronize(s));
+    std::vector<unsigned char> small(nI, 0), large(nI, 0);
     bool any_small = false, any_large = false;
     // instances without contact blocks: pcg_sell.cu, unless they are too large
     // for it or the CTA-local polynomial preconditioner is asked for
@@ -1314,8 +1343,8 @@ static int pcg_inner(Arena& A, Work& W, const double* b, double rel_tol, int max
         const int rc = sell_plan(A, W, s);
         if (rc) return rc;
     }
-    std::vector<int> sells;
-    std::vector<unsigned char> by_sell(nI, 0);
+    std::vector<int>& sells = pend.inst;
+    sells.clear();
     std::vector<int> by_size[5];  // cluster sizes 1, 2, 4, 8, 16
     for (int i = 0; i < nI; ++i) {
         if (!act[i]) continue;
@@ -1323,7 +1352,6 @@ static int pcg_inner(Arena& A, Work& W, const double* b, double rel_tol, int max
         const bool blocks = W.cl.ioff_h[i + 1] > W.cl.ioff_h[i];
         if (!blocks && W.sell.first[i] >= 0 && (W.local_deg == 0 || vi <= W.grid_min_v)) {
             sells.push_back(i);
-            by_sell[i] = 1;
             continue;
         }
         if (vi > W.grid_min_v) { large[i] = 1; any_large = true; continue; }
@@ -1348,28 +1376,18 @@ static int pcg_inner(Arena& A, Work& W, const double* b, double rel_tol, int max
                     W.stats.pcg_bytes += (double)iters[i] * W.pcg_bytes_per_iter[i] * (sizeof(T) / 4.0);
             }
     };
+    *xout = x;
     if (!sells.empty()) {
+        int* hit = W.pinned_ints(nI + 17);
+        if (!hit) return IDP_ERR_CUDA;
+        pend.host = hit;
         int* d_bad = d_iters + nI + 16;
         IDP_CUDA_TRY(cudaMemsetAsync(d_bad, 0, sizeof(int), s));
         W.timer.start(PhaseTimer::PCG, s);
         const int rc = sell_solve<T>(A, W, sells, b, x, rel_tol, max_iters, d_iters, d_bad, s);
         W.timer.stop(s);
         if (rc) return rc;
-        std::vector<int> hit(nI + 17);
-        IDP_CUDA_TRY(cudaMemcpyAsync(hit.data(), d_iters, sizeof(int) * (nI + 17), cudaMemcpyDeviceToHost, s));
-        IDP_CUDA_TRY(cudaStreamSynchronize(s));
-        int most = 0;
-        for (int i : sells) most = std::max(most, iters[i] = hit[i]);
-        W.sell.tag += (unsigned int)most + 4;  // the tags this solve used
-        if (hit[nI + 16]) {  // a poll ran out (never expected): its tags are not reused
-            W.sell.xch_bytes = 0;
-            return IDP_ERR_CUDA;
-        }
-        account(by_sell);
-        if (!any_small && !any_large) {
-            *xout = x;
-            return IDP_OK;
-        }
+        IDP_CUDA_TRY(cudaMemcpyAsync(hit, d_iters, sizeof(int) * (nI + 17), cudaMemcpyDeviceToHost, s));
     }
     if (any_small) {
         std::vector<int> flat;
@@ -1423,10 +1441,7 @@ static int pcg_inner(Arena& A, Work& W, const double* b, double rel_tol, int max
             if (small[i]) iters[i] = hit[i];
     }
     account(small);
-    if (!any_large) {
-        *xout = x;
-        return IDP_OK;
-    }
+    if (!any_large) return IDP_OK;
     // large instances: grid-wide PCG, in waves of at most gmax CTAs
     static std::atomic<int> gmax_cache{0};  // one per instantiation
     int gmax = gmax_cache.load();
@@ -1552,13 +1567,12 @@ static int pcg_inner(Arena& A, Work& W, const double* b, double rel_tol, int max
     for (int i = 0; i < nI; ++i)
         if (large[i]) iters[i] = hit[i];
     account(large);
-    *xout = x;
     return IDP_OK;
 }
 
 int pcg_solve(Arena& A, Work& W, const ContactSet& cs, bool fp64, const double* rhs, double* sol, double rel_tol,
-              int max_iters, std::vector<int>& iters_out, std::vector<double>& relres_out, cudaStream_t s,
-              const double* tol_host) {
+              int max_iters, const std::vector<unsigned char>& mask, std::vector<int>& iters_out,
+              std::vector<double>& relres_out, cudaStream_t s, const double* tol_host) {
     (void)cs;
     const int nI = A.nI;
     long n3 = 3 * A.V;
@@ -1571,14 +1585,13 @@ int pcg_solve(Arena& A, Work& W, const ContactSet& cs, bool fp64, const double* 
     double* inst_rr = W[W_INST_SUM].as<double>();
     const int* trp = W[W_TAIL_ROWPTR].as<int>();
     const int* tcol = W[W_TAIL_COL].as<int>();
-    std::vector<double> b2(nI, 0.0), hrr(nI);
-    std::vector<unsigned char> act(nI), act0(nI);
-    IDP_CUDA_TRY(cudaMemcpyAsync(act0.data(), A.active, nI, cudaMemcpyDeviceToHost, s));
+    std::vector<double> prev(nI, 0.0);
     // FP64 residual res = b - A sol and its squared norm per instance; the
-    // norms are copied to pinned host memory, valid after the next
-    // synchronisation of the stream (sync = true waits here)
-    double* hres = W.pinned_doubles(nI);
-    if (!hres) return IDP_ERR_CUDA;
+    // norms are copied to pinned host memory (after |b|^2 there), valid after
+    // the next synchronisation of the stream
+    double* b2 = W.pinned_doubles(2 * (long)nI);
+    if (!b2) return IDP_ERR_CUDA;
+    double* hres = b2 + nI;
     InstSum r8;
     if (int r = inst_sum_args(A, W, A.vert_chunk_off, A.n_vert_chunks, kResPer, inst_rr, false, r8, s)) return r;
     auto residual_async = [&]() -> int {
@@ -1594,86 +1607,60 @@ int pcg_solve(Arena& A, Work& W, const ContactSet& cs, bool fp64, const double* 
         IDP_CUDA_TRY(cudaMemcpyAsync(hres, inst_rr, sizeof(double) * nI, cudaMemcpyDeviceToHost, s));
         return IDP_OK;
     };
-    auto residual = [&](std::vector<double>& out) -> int {
-        int r = residual_async();
-        if (r) return r;
-        IDP_CUDA_TRY(cudaStreamSynchronize(s));
-        out.assign(hres, hres + nI);
-        return IDP_OK;
-    };
-    // |b|^2 (x = 0 gives res = b); read after the first sweep, whose own
-    // synchronisation brings it back (every active instance runs sweep 0)
-    int rc = IDP_OK;
+    // |b|^2 (x = 0 gives res = b)
     {
         InstSum r1 = r8;
         r1.per = 1;
         (::idp::count_launch(), k_refine_start<<<A.n_vert_chunks, kBlock, 0, s>>>(A.vert_chunks, A.active, A.dbc, rhs, sol,
                                                                                  res, r1));
-        IDP_CUDA_TRY(cudaMemcpyAsync(hres, inst_rr, sizeof(double) * nI, cudaMemcpyDeviceToHost, s));
+        IDP_CUDA_TRY(cudaMemcpyAsync(b2, inst_rr, sizeof(double) * nI, cudaMemcpyDeviceToHost, s));
     }
-    bool b2_pending = true;
-    bool hrr_current = false;
+    // Sweeps of PCG on the residual, correction and new residual, one
+    // synchronisation each. Instances whose FP64 residual is small, or that
+    // stopped improving (the FP32 operator cannot resolve them), stop refining
+    // and keep their residual.
     const int max_refine = fp64 ? 1 : 8;
     const double inner_tol = fp64 ? rel_tol : std::max(rel_tol, 2e-3);
-    std::vector<double> prev(nI, 0.0);
-    for (int ref = 0; ref < max_refine; ++ref) {
-        // instances whose FP64 residual is already small, or that stopped
-        // improving (the FP32 operator cannot resolve them), stop refining
-        bool any = false;
-        if (ref > 0) {
-            if (b2_pending) {  // the first sweep synchronised the stream
-                b2.assign(hres, hres + nI);
-                b2_pending = false;
-                for (int i = 0; i < nI; ++i) prev[i] = b2[i];
-            }
-            rc = residual(hrr);
-            if (rc) return rc;
-            hrr_current = true;
-            for (int i = 0; i < nI; ++i) {
-                if (!act[i]) continue;  // stopped at an earlier sweep: its residual stands
-                const double ti = tol_host ? std::max(rel_tol, tol_host[i]) : rel_tol;
-                const bool stalled = hrr[i] > 0.25 * prev[i];
-                act[i] = b2[i] > 0 && hrr[i] > ti * ti * b2[i] && !stalled;
-                relres_out[i] = b2[i] > 0 ? std::sqrt(hrr[i] / b2[i]) : 0.0;
-                prev[i] = hrr[i];
-                any |= act[i] != 0;
-            }
-        } else {
-            for (int i = 0; i < nI; ++i) {
-                act[i] = act0[i];
-                any |= act[i] != 0;
-            }
-        }
-        if (!any) break;
-        hrr_current = false;
-        IDP_CUDA_TRY(cudaMemcpyAsync(A.active, act.data(), nI, cudaMemcpyHostToDevice, s));
+    std::vector<unsigned char> act = mask;
+    bool changed = false;  // the mask on the device is not `mask`
+    int rc = IDP_OK;
+    for (int ref = 0; ref < max_refine && std::find(act.begin(), act.end(), 1) != act.end(); ++ref) {
         std::vector<int> its;
+        SellPending pend;
         if (fp64) {
             double* e = nullptr;
-            rc = pcg_inner<double>(A, W, res, inner_tol, max_iters, its, &e, s);
-            if (rc) break;
+            if ((rc = pcg_inner<double>(A, W, res, inner_tol, max_iters, act, its, pend, &e, s))) break;
             (::idp::count_launch(), k_add_correction<double><<<grid_for(A.V), kBlock, 0, s>>>(A.V, A.vinst, A.active, e, sol));
         } else {
             float* e = nullptr;
-            rc = pcg_inner<float>(A, W, res, inner_tol, max_iters, its, &e, s);
-            if (rc) break;
+            if ((rc = pcg_inner<float>(A, W, res, inner_tol, max_iters, act, its, pend, &e, s))) break;
             (::idp::count_launch(), k_add_correction<float><<<grid_for(A.V), kBlock, 0, s>>>(A.V, A.vinst, A.active, e, sol));
         }
-        for (int i = 0; i < nI; ++i)
-            if (act[i]) iters_out[i] += its[i];
-    }
-    IDP_CUDA_TRY(cudaMemcpyAsync(A.active, act0.data(), nI, cudaMemcpyHostToDevice, s));
-    if (rc) return rc;
-    if (b2_pending) {
+        if ((rc = residual_async())) break;
         IDP_CUDA_TRY(cudaStreamSynchronize(s));
-        b2.assign(hres, hres + nI);
+        if ((rc = fp64 ? sell_finish<double>(A, W, pend, its) : sell_finish<float>(A, W, pend, its))) break;
+        bool drop = false;
+        for (int i = 0; i < nI; ++i) {
+            if (!act[i]) continue;
+            iters_out[i] += its[i];
+            if (ref == 0) prev[i] = b2[i];
+            const double ti = tol_host ? std::max(rel_tol, tol_host[i]) : rel_tol;
+            const bool stalled = hres[i] > 0.25 * prev[i];
+            relres_out[i] = b2[i] > 0 ? std::sqrt(hres[i] / b2[i]) : 0.0;
+            prev[i] = hres[i];
+            if (!(b2[i] > 0 && hres[i] > ti * ti * b2[i] && !stalled)) {
+                act[i] = 0;
+                drop = true;
+            }
+        }
+        if (drop && std::find(act.begin(), act.end(), 1) != act.end() && ref + 1 < max_refine) {
+            IDP_CUDA_TRY(cudaMemcpyAsync(A.active, act.data(), nI, cudaMemcpyHostToDevice, s));
+            changed = true;
+        }
     }
-    if (!hrr_current) {
-        rc = residual(hrr);
-        if (rc) return rc;
-        for (int i = 0; i < nI; ++i) relres_out[i] = b2[i] > 0 ? std::sqrt(hrr[i] / b2[i]) : 0.0;
-    }
-    return IDP_OK;
+    if (rc) W.sell.xch_bytes = 0;  // tags may be in use: clear the exchange words before the next solve
+    if (changed) IDP_CUDA_TRY(cudaMemcpyAsync(A.active, mask.data(), nI, cudaMemcpyHostToDevice, s));
+    return rc;
 }
 
 }  // namespace idp
