@@ -217,30 +217,22 @@ __global__ void k_spmv_plain(long V, const int* __restrict__ vinst, const unsign
 }
 
 // ---- per-vertex Newton kernels
-// 8 lanes per vertex: lane l takes its corners l, l + 8, ...
+// 4 lanes per vertex: lane l < 3 adds component l of its corners, in their order
 __global__ void k_grad_gather_tet(long V, const int* __restrict__ vinst, const unsigned char* __restrict__ active,
                                   const int* __restrict__ vcp, const int* __restrict__ vc,
                                   const double* __restrict__ tg, const double* __restrict__ mass,
                                   const double* __restrict__ X, const double* __restrict__ Xt, double* __restrict__ g) {
-    const long v = ((long)blockIdx.x * blockDim.x + threadIdx.x) >> 3;
-    const int l = threadIdx.x & 7;
-    const bool on = v < V && active[vinst[v]];
-    double s0 = 0, s1 = 0, s2 = 0;
-    if (on) {
-        const int k1 = vcp[v + 1];
-        for (int k = vcp[v] + l; k < k1; k += 8) {
-            int code = vc[k];  // tet*4 + corner
-            const double* p = tg + 12 * (long)(code >> 2) + 3 * (code & 3);
-            s0 += p[0]; s1 += p[1]; s2 += p[2];
-        }
+    const long v = ((long)blockIdx.x * blockDim.x + threadIdx.x) >> 2;
+    const int l = threadIdx.x & 3;
+    if (v >= V || l == 3 || !active[vinst[v]]) return;
+    const int k1 = vcp[v + 1];
+    double s = 0;
+#pragma unroll 8
+    for (int k = vcp[v]; k < k1; ++k) {
+        const int code = vc[k];  // tet*4 + corner
+        s += tg[12 * (long)(code >> 2) + 3 * (code & 3) + l];
     }
-    for (int o = 4; o > 0; o >>= 1) {
-        s0 += __shfl_xor_sync(0xffffffffu, s0, o);
-        s1 += __shfl_xor_sync(0xffffffffu, s1, o);
-        s2 += __shfl_xor_sync(0xffffffffu, s2, o);
-    }
-    if (on && l < 3)
-        g[3 * v + l] = (l == 0 ? s0 : (l == 1 ? s1 : s2)) + mass[v] * (X[3 * v + l] - Xt[3 * v + l]);
+    g[3 * v + l] = s + mass[v] * (X[3 * v + l] - Xt[3 * v + l]);
 }
 
 __global__ void k_inertia_energy(const Chunk* __restrict__ chunks, const unsigned char* __restrict__ active,
@@ -1234,7 +1226,7 @@ int vec_inertia(Arena& A, Work& W, const double* X, double* inst_E, double* g, c
 }
 
 int grad_gather_tet(Arena& A, Work& W, const double* X, double* g, cudaStream_t s) {
-    (::idp::count_launch(), k_grad_gather_tet<<<grid_for(8 * A.V), kBlock, 0, s>>>(
+    (::idp::count_launch(), k_grad_gather_tet<<<grid_for(4 * A.V), kBlock, 0, s>>>(
                                 A.V, A.vinst, A.active, A.vert_corner_ptr, A.vert_corner, W[W_TET_GRAD].as<double>(),
                                 A.mass, X, A.Xtilde, g));
     return cudaGetLastError() == cudaSuccess ? IDP_OK : IDP_ERR_CUDA;
