@@ -480,8 +480,8 @@ def run_flow(args):
         "roofline": {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s",
                      "frac": (achieved / peak) if achieved else None,
                      "traffic": traffic.get("bytes_per_launch") if traffic else None,
-                     "kernel": "k_pcg_grid (grid-wide cooperative PCG: BSR rows resident in shared memory, "
-                               "FP32 SpMV + block-Jacobi, one reduction round per iteration)",
+                     "kernel": "k_pcg_sell (persistent CTAs: matrix rows resident in shared memory, vectors in "
+                               "registers, FP32 SpMV + block-Jacobi, tagged exchange per iteration)",
                      "achieved_basis": "algorithmic bytes of the PCG iterations / PCG event time",
                      "traffic_basis": "ncu DRAM read+write bytes of one launch (profiles/pcg_traffic.json)",
                      "peak_source": peak_kind},
@@ -717,7 +717,7 @@ def run_gpu(args):
         "e2e": {"value": e2e_val, "unit": unit, "h2d_bytes_per_step": h2d, "d2h_bytes_per_step": d2h},
         "roofline": {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s",
                      "frac": (achieved / peak) if achieved else None,
-                     "traffic": None,  # the committed ncu capture covers k_pcg_grid on the blob only
+                     "traffic": None,  # the committed ncu capture covers the PCG on the blob only
                      "kernel": "k_pcg_cluster (block-Jacobi + contact-block PCG, one thread-block cluster per "
                                "instance)",
                      "peak_source": peak_kind},
