@@ -564,7 +564,8 @@ __device__ __forceinline__ void ccd_query_ee(long eI, const int2* __restrict__ e
 }
 
 // both queries in one launch: the first bpt CTAs take the nodes, the others
-// the edges
+// the edges. Bound by latency, as the constraint set's. Stack of seven plates:
+// edges alone 409 us -> both 299; blob of 220,000 tets: 186 -> 105.
 __global__ void k_ccd_query(unsigned int bpt, long nN, const int* __restrict__ nodes, const int* __restrict__ ninst,
                             long nE, const int2* __restrict__ edges, const int* __restrict__ einst,
                             const unsigned char* __restrict__ active, const double* __restrict__ X,

@@ -25,10 +25,15 @@ namespace idp {
 
 namespace {
 
-// nine threads per BSR block, one value each (value q = 3 r + c): the element
-// blocks are read and the row of blocks written as whole lines. (A thread per
-// block moved 36 bytes in nine strided accesses: 75 us on 720,000 blocks.)
+// N threads per BSR block, 9 / N of its values each (value q = 3 r + c). FP64:
+// nine, so that the element blocks are read and the row of blocks written as
+// whole lines (220,000 blocks: 71 us with one thread per block, 42 with nine).
+// FP32: one, because the source list is then walked once per block (613,000
+// blocks: 75 us with one thread per block, 174 with nine).
 template <class T>
+constexpr int kAsmThreads = sizeof(T) == 8 ? 9 : 1;
+
+template <class T, int N>
 __global__ void k_assemble_tet(long B, const int* __restrict__ src_ptr, const int* __restrict__ src,
                                const T* __restrict__ tet_hess, const int* __restrict__ brow,
                                const int* __restrict__ colidx, const double* __restrict__ mass,
@@ -36,14 +41,16 @@ __global__ void k_assemble_tet(long B, const int* __restrict__ src_ptr, const in
                                const unsigned char* __restrict__ active, const double* __restrict__ fvol, double h,
                                const double* __restrict__ dstiff, const unsigned char* __restrict__ excl,
                                T* __restrict__ val) {
+    constexpr int M = 9 / N;
     const long i = (long)blockIdx.x * blockDim.x + threadIdx.x;
-    const long b = i / 9;
+    const long b = i / N;
     if (b >= B) return;
-    const int q = (int)(i - 9 * b), qt = (q % 3) * 3 + q / 3;
-    const bool diag = q % 4 == 0;
+    const int q0 = M * (int)(i - N * b);
     int row = brow[b], col = colidx[b];
     if (!active[vinst[row]]) return;
-    T acc = T(0);
+    T acc[M];
+#pragma unroll
+    for (int m = 0; m < M; ++m) acc[m] = T(0);
     for (int k = src_ptr[b]; k < src_ptr[b + 1]; ++k) {
         const int code = src[k];  // (element block) * 2 + transposed
         if (code < 0) {
@@ -51,19 +58,31 @@ __global__ void k_assemble_tet(long B, const int* __restrict__ src_ptr, const in
             // 2 h vol/6 I on the diagonal, -h vol/6 I off it
             const int cf = -code - 1;
             const double w = h * fvol[cf >> 1] / 6.0;
-            if (diag) acc += (T)((cf & 1) ? 2.0 * w : -w);
+            const T v = (T)((cf & 1) ? 2.0 * w : -w);
+#pragma unroll
+            for (int m = 0; m < M; ++m)
+                if ((q0 + m) % 4 == 0) acc[m] += v;
             continue;
         }
-        acc += tet_hess[(long)(code >> 1) * 9 + ((code & 1) ? qt : q)];
+        const T* p = tet_hess + (long)(code >> 1) * 9;
+#pragma unroll
+        for (int m = 0; m < M; ++m) {
+            const int q = q0 + m;
+            acc[m] += p[(code & 1) ? (q % 3) * 3 + q / 3 : q];
+        }
     }
-    if (row == col && diag) {
-        acc += (T)mass[row];
-        // moving-DBC penalty stiff * m on the diagonal (Compute_DBC_Hessian,
-        // FEM/Shell/DIRICHLET.h:72-90)
-        if (excl[row] && dstiff[vinst[row]] > 0) acc += (T)(dstiff[vinst[row]] * mass[row]);
+#pragma unroll
+    for (int m = 0; m < M; ++m) {
+        const bool diag = row == col && (q0 + m) % 4 == 0;
+        if (diag) {
+            acc[m] += (T)mass[row];
+            // moving-DBC penalty stiff * m on the diagonal (Compute_DBC_Hessian,
+            // FEM/Shell/DIRICHLET.h:72-90)
+            if (excl[row] && dstiff[vinst[row]] > 0) acc[m] += (T)(dstiff[vinst[row]] * mass[row]);
+        }
+        if (dbc[row] || dbc[col]) acc[m] = diag ? T(1) : T(0);
+        val[9 * b + q0 + m] = acc[m];
     }
-    if (dbc[row] || dbc[col]) acc = row == col && diag ? T(1) : T(0);
-    val[i] = acc;
 }
 
 template <class T>
@@ -106,15 +125,17 @@ __global__ void k_diag_inv(long V, const int* __restrict__ diagblk, const T* __r
 }
 
 // Row v of A x in FP64 (FP32 or FP64 matrix) by 8 lanes: lane l takes blocks
-// l, l + 8, ... of the row and of its contact tail; every lane gets the sums.
-// (A thread per row was a chain of up to 19 dependent gathers: 35 us for 160
-// vertices, 52 us for 49,863.) All lanes of the warp call this together.
+// l, l + 8, ... of the row and of its contact tail; lane j < 3 gets component j.
+// Bound by latency on small meshes (a thread per row was a chain of up to 19
+// dependent gathers: 160 rows 35 us, with 8 lanes 15; 17,000 rows 58 and 34) and by
+// the FP64 pipe on large ones, so the sums over the lanes halve the components a
+// lane carries: 4 additions, not 9. All lanes of the warp call this together.
 template <class T>
-__device__ __forceinline__ void row8_f64(bool on, long v, int l, const int* __restrict__ rowptr,
+__device__ __forceinline__ double row8_f64(bool on, long v, int l, const int* __restrict__ rowptr,
                                          const int* __restrict__ colidx, const T* __restrict__ val,
                                          const int* __restrict__ trp, const int* __restrict__ tcol,
                                          const T* __restrict__ tval, const unsigned char* __restrict__ dbc,
-                                         const double* __restrict__ x, double y[3]) {
+                                         const double* __restrict__ x) {
     double a0 = 0, a1 = 0, a2 = 0;
     if (on) {
         const int k1 = rowptr[v + 1];
@@ -139,14 +160,17 @@ __device__ __forceinline__ void row8_f64(bool on, long v, int l, const int* __re
             a2 += (double)m[6] * x0 + (double)m[7] * x1 + (double)m[8] * x2;
         }
     }
-    for (int o = 4; o > 0; o >>= 1) {
-        a0 += __shfl_xor_sync(0xffffffffu, a0, o);
-        a1 += __shfl_xor_sync(0xffffffffu, a1, o);
-        a2 += __shfl_xor_sync(0xffffffffu, a2, o);
-    }
-    y[0] = a0;
-    y[1] = a1;
-    y[2] = a2;
+    // lanes 0-3 go on with components 0 and 1, lanes 4-7 with 2; then lanes 0, 1
+    // with 0 and lanes 2, 3 with 1
+    const bool up = l & 4, odd = l & 2;
+    double k0 = up ? a2 : a0;
+    k0 += __shfl_xor_sync(0xffffffffu, up ? a0 : a2, 4);
+    const double k1 = a1 + __shfl_xor_sync(0xffffffffu, a1, 4);
+    const double give = up || odd ? k0 : k1;  // lanes 4-7 add component 2 again
+    double r = !up && odd ? k1 : k0;
+    r += __shfl_xor_sync(0xffffffffu, give, 2);
+    r += __shfl_xor_sync(0xffffffffu, r, 1);
+    return __shfl_sync(0xffffffffu, r, 2 * (l & 3), 8);
 }
 
 // CTAs per vertex chunk of the residual: 32 rows each
@@ -164,11 +188,10 @@ __global__ void k_residual64(const Chunk* __restrict__ chunks, const unsigned ch
     const long v = c.begin + 32 * (blockIdx.x % kResPer) + (threadIdx.x >> 3);
     const bool on = active[c.inst] && v < c.end;
     const bool fixed = on && dbc[v];
-    double y[3];
-    row8_f64<T>(on && !fixed, v, l, rowptr, colidx, val, trp, tcol, tval, dbc, x, y);
+    const double y = row8_f64<T>(on && !fixed, v, l, rowptr, colidx, val, trp, tcol, tval, dbc, x);
     double acc = 0;
     if (on && l < 3) {
-        const double r = fixed ? 0.0 : b[3 * v + l] - (l == 0 ? y[0] : (l == 1 ? y[1] : y[2]));
+        const double r = fixed ? 0.0 : b[3 * v + l] - y;
         res[3 * v + l] = r;
         acc = r * r;
     }
@@ -211,9 +234,8 @@ __global__ void k_spmv_plain(long V, const int* __restrict__ vinst, const unsign
     const int l = threadIdx.x & 7;
     const bool on = v < V && active[vinst[v]];
     const bool fixed = on && dbc[v];
-    double o[3];
-    row8_f64<T>(on && !fixed, v, l, rowptr, colidx, val, trp, tcol, tval, dbc, x, o);
-    if (on && l < 3) y[3 * v + l] = fixed ? x[3 * v + l] : (l == 0 ? o[0] : (l == 1 ? o[1] : o[2]));
+    const double o = row8_f64<T>(on && !fixed, v, l, rowptr, colidx, val, trp, tcol, tval, dbc, x);
+    if (on && l < 3) y[3 * v + l] = fixed ? x[3 * v + l] : o;
 }
 
 // ---- per-vertex Newton kernels
@@ -1249,14 +1271,14 @@ int assemble(Arena& A, Work& W, const ContactSet& cs, bool fp64, cudaStream_t s)
     const int* trp = W[W_TAIL_ROWPTR].as<int>();
     const int* tcol = W[W_TAIL_COL].as<int>();
     if (fp64) {
-        (::idp::count_launch(), k_assemble_tet<double><<<grid_for(9 * A.B), kBlock, 0, s>>>(A.B, A.src_ptr, A.src, W[W_TET_HESS].as<double>(), A.brow,
+        (::idp::count_launch(), k_assemble_tet<double, kAsmThreads<double>><<<grid_for(kAsmThreads<double> * A.B), kBlock, 0, s>>>(A.B, A.src_ptr, A.src, W[W_TET_HESS].as<double>(), A.brow,
                                                                 A.colidx, A.mass, A.dbc, A.vinst, A.active, A.fvol, A.h, A.dstiff, A.dbc_excl,
                                                                 W[W_BSR_VAL].as<double>()));
         (::idp::count_launch(), k_diag_inv<double><<<grid_for(A.V), kBlock, 0, s>>>(A.V, A.diagblk, W[W_BSR_VAL].as<double>(), trp, tcol,
                                                             W[W_TAIL_VAL].as<double>(), A.dbc, A.vinst, A.active,
                                                             W[W_DIAG_INV].as<double>()));
     } else {
-        (::idp::count_launch(), k_assemble_tet<float><<<grid_for(9 * A.B), kBlock, 0, s>>>(A.B, A.src_ptr, A.src, W[W_TET_HESS].as<float>(), A.brow,
+        (::idp::count_launch(), k_assemble_tet<float, kAsmThreads<float>><<<grid_for(kAsmThreads<float> * A.B), kBlock, 0, s>>>(A.B, A.src_ptr, A.src, W[W_TET_HESS].as<float>(), A.brow,
                                                                A.colidx, A.mass, A.dbc, A.vinst, A.active, A.fvol, A.h, A.dstiff, A.dbc_excl,
                                                                W[W_BSR_VAL].as<float>()));
         (::idp::count_launch(), k_diag_inv<float><<<grid_for(A.V), kBlock, 0, s>>>(A.V, A.diagblk, W[W_BSR_VAL].as<float>(), trp, tcol,
