@@ -1,6 +1,6 @@
 // PCG for instances without contact blocks: persistent CTAs that hold their
 // rows' matrix in shared memory and every vector in registers, exchanging
-// nothing but the vector the SpMV gathers and three partial sums per iteration.
+// nothing but two values per halo component and five partial sums per iteration.
 //
 // Partition. An instance of V vertices is cut into runs of consecutive vertices
 // (rows), one CTA each; the cut depends on V (and the context's parameters)
@@ -12,26 +12,39 @@
 // sorted by length and a slice stores its blocks as slot rows of 32 lanes, the
 // nine values in nine arrays of 32 (shared-memory reads without bank
 // conflicts). Blocks whose column lies in the CTA's own rows come first in a
-// slice, so that their part of A m runs while the neighbours' m is under way;
-// the other columns are numbered in the CTA's halo list. Both lists depend on
-// the pattern only and are laid out once per commit (k_sell_plan).
+// slice; the other columns are numbered in the CTA's halo list. Both lists depend
+// on the pattern only and are laid out once per commit (k_sell_plan).
 //
 // Exchange. A value is stored as a 64-bit word of 32 payload bits and a 32-bit
 // tag that no earlier exchange used (FP64: two words), and its readers poll the
 // data itself: neither a fence nor a flag is waited for, and a halo value is
 // usable one L2 round trip after it was written. The CTAs' partial sums travel
 // the same way and every CTA adds them in the same order. Two slots by parity
-// suffice: a CTA overwrites exchange e with e + 2 only after it has read every
-// CTA's sums of e + 1, which each wrote after reading e.
+// suffice: a CTA overwrites exchange e with e + 2 only after it has every CTA's
+// sums of e + 1, which each wrote after it had read all of e.
 //
-// Pipelined PCG (Ghysels & Vanroose) as in k_pcg_grid, one reduction per
-// iteration. On the 220,515-tet blob (49,863 vertices, FP32) k_pcg_grid took
-// 12 us per iteration: vectors in global memory, the gathers from L2 and a
-// counter, a release word and a reduction by the last CTA to arrive; here 5.7,
-// most of it reading the matrix (328 rows per SM: 20 shared-memory wavefronts
-// per slot row, 10 of them bank conflicts of the gathers). A bar of 160
-// vertices: 10.5 us on one cluster CTA (k_pcg_cluster) -> 2.4 on one CTA here; a
-// blob of 5,838 vertices in FP64: 66 us on 16 cluster CTAs -> 13.
+// PCG with one exchange per iteration (predict and recompute, after Chen &
+// Carson 2020): s = A p and q = M^{-1} s are formed, and the sums p.s, r.u, r.q,
+// s.q and r.r travel together with q; they give alpha, and beta by predicting
+// the next r.u, which the next iteration recomputes. The owner of a row sends u =
+// M^{-1} r a phase ahead, so that a neighbour can form the next u = u - alpha q
+// and p = u + beta p of its halo by itself: only the halo's p is carried on.
+// No product with A and no residual but r is kept by recurrence, and on the
+// matrices of bars with E = 1e4 to 1e11 (h = 0.1) the solves end at the residual
+// of classical PCG, and up to 1e7 within 10 % of its iterations, in FP32 and FP64.
+// (The pipelined recurrences of Ghysels & Vanroose, which hide the exchange behind
+// half of the product, lose the residual on stiff bodies: E = 1e9, FP32 sweeps
+// stall at 2e-3 to 2e-2, FP64 ends at 1e-8 for an asked 1e-12.)
+//
+// Bound by the shared-memory reads of the matrix (20 wavefronts per slot row, 10 of
+// them bank conflicts of the gathers), the FP64 pipe, or, with few rows, the
+// exchange. Microseconds per iteration, with the pipelined recurrences -> now: blob of
+// 220,515 tets (49,863 vertices, 328 rows per SM) in FP32 5.7 -> 6.9 (k_pcg_grid: 12),
+// blob of 18,210 vertices 2.9 -> 3.7, bar of 160 vertices on one CTA 2.3 (k_pcg_cluster:
+// 10.5); blob of 5,838 vertices in FP64 14 (66 on 16 cluster CTAs). Tried on the
+// exchange and taken back: copies of the sums for groups of CTAs, warps that poll the
+// sums while others gather the halo (5.8 against 4.5 per iteration of that blob in
+// FP32), waits before the first poll, 6 or 8 polls in flight.
 #include <algorithm>
 #include <atomic>
 #include "engine.hpp"
@@ -45,14 +58,15 @@ constexpr int kSW = kST / 32;
 constexpr int kSliceRows = 8;
 // Rows per CTA at least, where there are several, and the largest instance of one
 // CTA, {FP32, FP64}. Microseconds per iteration on bars and blobs of 160 to
-// 18,210 vertices: FP32 2.8-3.0 with 40 to 128 rows, 3.7 with 160 (a second slice
-// per warp); 2.4 on one CTA of 160 rows, 3.4 of 320. FP64 is bound by its pipe:
-// 13.3-14 with 40 rows, 17 with 128, 18 on one CTA of 160.
+// 18,210 vertices: FP32 2.8-3.5 with 40 to 128 rows, 3.8-4.5 with 160 (a second slice
+// per warp); 2.3 on one CTA of 160 rows, 3.5 of 320. FP64 is bound by its pipe:
+// 12.3-14 with 40 rows, 13-17.5 with 128, 17 on one CTA of 160.
 constexpr int kSellRows[2] = {64, 40}, kSellSolo[2] = {192, 40};
 constexpr int kSellMaxRows = 3 * kSW * kSliceRows;  // rows per CTA: three slices per warp
 constexpr int kHaloTable = 4096;         // hash slots of the halo search
 constexpr int kHaloMax = 2600;           // halo vertices per CTA
 constexpr int kSellSmem = 222 * 1024;    // dynamic shared memory limit
+constexpr int kPollCtas = 5;             // CTAs whose sums a lane polls at a time (152 / 32)
 constexpr unsigned int kSellSpin = 1u << 21;  // polls before giving up (about 1 s)
 
 template <class T>
@@ -67,23 +81,72 @@ __device__ __forceinline__ unsigned long long get_word(const unsigned long long*
     asm volatile("ld.relaxed.gpu.global.u64 %0, [%1];" : "=l"(w) : "l"(p) : "memory");
     return w;
 }
-__device__ __forceinline__ void put_value(unsigned long long* p, float v, unsigned int tag) {
+__device__ __forceinline__ void get_words2(const unsigned long long* p, unsigned long long& a, unsigned long long& b) {
+    asm volatile("ld.relaxed.gpu.global.v2.u64 {%0, %1}, [%2];" : "=l"(a), "=l"(b) : "l"(p) : "memory");
+}
+__device__ __forceinline__ bool tagged(unsigned long long w, unsigned int tag) { return (unsigned int)(w >> 32) == tag; }
+__device__ __forceinline__ double join(unsigned long long lo, unsigned long long hi) {
+    return __longlong_as_double((long long)((hi << 32) | (lo & 0xffffffffull)));
+}
+// a value at p (FP64: its halves `next` words apart)
+__device__ __forceinline__ void put_value(unsigned long long* p, long, float v, unsigned int tag) {
     put_word(p, __float_as_uint(v), tag);
 }
-__device__ __forceinline__ void put_value(unsigned long long* p, double v, unsigned int tag) {
+__device__ __forceinline__ void put_value(unsigned long long* p, long next, double v, unsigned int tag) {
     const unsigned long long b = (unsigned long long)__double_as_longlong(v);
     put_word(p, (unsigned int)b, tag);
-    put_word(p + 1, (unsigned int)(b >> 32), tag);
+    put_word(p + next, (unsigned int)(b >> 32), tag);
 }
-__device__ __forceinline__ bool get_value(const unsigned long long* p, float& v, unsigned int tag) {
+__device__ __forceinline__ bool get_value(const unsigned long long* p, long, float& v, unsigned int tag) {
     const unsigned long long w = get_word(p);
     v = __uint_as_float((unsigned int)w);
-    return (unsigned int)(w >> 32) == tag;
+    return tagged(w, tag);
 }
-__device__ __forceinline__ bool get_value(const unsigned long long* p, double& v, unsigned int tag) {
-    const unsigned long long a = get_word(p), b = get_word(p + 1);
-    v = __longlong_as_double((long long)((b << 32) | (a & 0xffffffffull)));
-    return (unsigned int)(a >> 32) == tag && (unsigned int)(b >> 32) == tag;
+__device__ __forceinline__ bool get_value(const unsigned long long* p, long next, double& v, unsigned int tag) {
+    const unsigned long long a = get_word(p), b = get_word(p + next);
+    v = join(a, b);
+    return tagged(a, tag) && tagged(b, tag);
+}
+// the pair (u, q) at p; without `both` only u has to have arrived
+__device__ __forceinline__ bool get_pair(const unsigned long long* p, float& u, float& q, unsigned int tag, bool both) {
+    unsigned long long a, b;
+    get_words2(p, a, b);
+    u = __uint_as_float((unsigned int)a);
+    q = __uint_as_float((unsigned int)b);
+    return tagged(a, tag) && (!both || tagged(b, tag));
+}
+__device__ __forceinline__ bool get_pair(const unsigned long long* p, double& u, double& q, unsigned int tag, bool both) {
+    unsigned long long a, b, c, d;
+    get_words2(p, a, b);
+    get_words2(p + 2, c, d);
+    u = join(a, b);
+    q = join(c, d);
+    return tagged(a, tag) && tagged(b, tag) && (!both || (tagged(c, tag) && tagged(d, tag)));
+}
+
+// The warp's sums of kSums values: value j ends on the lanes whose bits 4, 3, 2
+// are those of j (sum_value). The lanes halve the values they carry at each of
+// the first three steps: 9 additions, not 25.
+constexpr int kSums = 5;
+__device__ __forceinline__ int sum_value(int lane) { return (lane >> 4 & 1) << 2 | (lane >> 3 & 1) << 1 | (lane >> 2 & 1); }
+template <class T>
+__device__ __forceinline__ T warp_sums(const T (&v)[kSums], int lane) {
+    const unsigned full = 0xffffffffu;
+    const bool b4 = lane & 16, b3 = lane & 8, b2 = lane & 4;
+    // the upper half goes on with value 4 alone
+    T a0 = b4 ? v[4] : v[0], a1 = b4 ? T(0) : v[1], a2 = b4 ? T(0) : v[2], a3 = b4 ? T(0) : v[3];
+    a0 += __shfl_xor_sync(full, b4 ? v[0] : v[4], 16);
+    a1 += __shfl_xor_sync(full, b4 ? v[1] : T(0), 16);
+    a2 += __shfl_xor_sync(full, b4 ? v[2] : T(0), 16);
+    a3 += __shfl_xor_sync(full, b4 ? v[3] : T(0), 16);
+    T c0 = b3 ? a2 : a0, c1 = b3 ? a3 : a1;
+    c0 += __shfl_xor_sync(full, b3 ? a0 : a2, 8);
+    c1 += __shfl_xor_sync(full, b3 ? a1 : a3, 8);
+    T r = b2 ? c1 : c0;
+    r += __shfl_xor_sync(full, b2 ? c0 : c1, 4);
+    r += __shfl_xor_sync(full, r, 2);
+    r += __shfl_xor_sync(full, r, 1);
+    return r;
 }
 
 // Layout of one CTA's rows: halo list (hash of the columns outside its rows),
@@ -235,6 +298,13 @@ __global__ void k_sell_plan(SellCta* __restrict__ cta, const int* __restrict__ r
     }
 }
 
+// halo values whose u and q a thread keeps in registers, and those that go to
+// shared memory
+template <class T>
+constexpr int kHeld = sizeof(T) == 4 ? 4 : 2;
+template <class T>
+__host__ __device__ inline int halo_rest(int nh) { return 3 * nh > kHeld<T> * kST ? 3 * nh - kHeld<T> * kST : 0; }
+
 template <class T>
 struct SellArgs {
     const SellCta* cta;
@@ -249,9 +319,10 @@ struct SellArgs {
     const unsigned char* dbc;
     const double* b;
     T* x;
-    unsigned long long* xm;       // [2][3 V] values
-    unsigned long long* xr;       // [2][3 plan CTAs] values
-    long xm_half, xr_half;        // words per parity
+    unsigned long long* xu;       // [2][3 V] pairs of values (u, q)
+    unsigned long long* xr;       // [2][kSums][words of a value][plan CTAs]
+    long xu_half, xr_half;        // words per parity
+    long xr_row;                  // plan CTAs
     unsigned int tag0;
     int nvmax, nhmax, cap;        // rows and halo entries of the largest CTA; slot rows held in shared memory
     const double* tol_inst;
@@ -265,11 +336,12 @@ template <class T, int STEPS>
 __global__ void __launch_bounds__(kST, 1) k_pcg_sell(const SellArgs<T> A) {
     extern __shared__ __align__(16) unsigned char sell_smem[];
     T* sval = reinterpret_cast<T*>(sell_smem);                    // [cap][9][32]
-    T* sm = sval + 288L * A.cap;                                  // m of the own rows, two parities
-    T* smh = sm + 6L * A.nvmax;                                   // m of the halo
-    unsigned short* scol = reinterpret_cast<unsigned short*>(smh + 3L * A.nhmax);  // [cap][32]
-    __shared__ T spart[kSW][3];   // partial sums by warp
-    __shared__ T sred[kSW][3];    // the CTAs' sums by polling warp
+    T* sp = sval + 288L * A.cap;                                  // p of the own rows
+    T* sph = sp + 3L * A.nvmax;                                   // of the halo: p
+    T* suq = sph + 3L * A.nhmax;                                  // and (u, q) past the threads' own
+    unsigned short* scol = reinterpret_cast<unsigned short*>(suq + 2L * halo_rest<T>(A.nhmax));  // [cap][32]
+    __shared__ T spart[kSW][kSums];   // partial sums by warp
+    __shared__ T sred[kSums];         // the instance's
     __shared__ T sscal[2];
     __shared__ int sstop, sbad;
     const SellCta me = A.cta[A.list[blockIdx.x]];
@@ -288,11 +360,12 @@ __global__ void __launch_bounds__(kST, 1) k_pcg_sell(const SellArgs<T> A) {
 #pragma unroll
         for (int j = 0; j < 9; ++j) sval[(9 * t + j) * 32 + lane] = k >= 0 ? m[j] : T(0);
     }
+    __syncthreads();
     // ---- this lane's rows (component l4 < 3 of row position p) and their state
     int lv[STEPS], off[STEPS], wl[STEPS], wt[STEPS];
     bool own[STEPS], fixed[STEPS];
     T D0[STEPS], D1[STEPS], D2[STEPS];
-    T z[STEPS], q[STEPS], s[STEPS], p[STEPS], u[STEPS], w[STEPS], x[STEPS], r[STEPS], m[STEPS];
+    T p[STEPS], x[STEPS], r[STEPS];
 #pragma unroll
     for (int t = 0; t < STEPS; ++t) {
         const int sl = warp + kSW * t, pos = sl * kSliceRows + (lane >> 2);
@@ -308,7 +381,7 @@ __global__ void __launch_bounds__(kST, 1) k_pcg_sell(const SellArgs<T> A) {
         const int v = v0 + lv[t];
         fixed[t] = act && A.dbc[v];
         own[t] = act && l4 < 3;
-        D0[t] = D1[t] = D2[t] = z[t] = q[t] = s[t] = p[t] = u[t] = w[t] = x[t] = r[t] = m[t] = T(0);
+        D0[t] = D1[t] = D2[t] = p[t] = x[t] = r[t] = T(0);
         if (own[t] && !fixed[t]) {
             const T* D = A.dinv + 9L * v + 3 * l4;
             D0[t] = D[0]; D1[t] = D[1]; D2[t] = D[2];
@@ -355,158 +428,162 @@ __global__ void __launch_bounds__(kST, 1) k_pcg_sell(const SellArgs<T> A) {
         }
         return l4 == 0 ? y0 : (l4 == 1 ? y1 : y2);
     };
-    // own value a of step t: to shared memory and, as exchange e, to the neighbours
-    auto publish = [&](int t, T a, unsigned int e) {
-        if (!own[t]) return;
-        sm[(e & 1) * 3 * A.nvmax + 3 * lv[t] + l4] = a;
-        if (nc > 1) put_value(A.xm + (e & 1) * A.xm_half + (3L * (v0 + lv[t]) + l4) * W, a, A.tag0 + e);
+    // own u (which = 0) or q (1) of step t to the neighbours, as exchange e
+    auto publish = [&](int t, int which, T a, unsigned int e) {
+        if (nc > 1 && own[t])
+            put_value(A.xu + (e & 1) * A.xu_half + (2 * (3L * (v0 + lv[t]) + l4) + which) * W, 1, a, A.tag0 + e);
     };
-    // halo values of exchange e into shared memory, four polls in flight per thread
-    auto gather = [&](unsigned int e) {
-        const unsigned long long* from = A.xm + (e & 1) * A.xm_half;
-        for (int i0 = tid; i0 < nh3; i0 += 4 * kST) {
-            const unsigned long long* a[4];
-            bool need[4];
+    // the halo's u and q of exchange e (before the first iteration: u alone, which
+    // is its p): kHeld<T> values per thread stay in its registers, the rest goes to
+    // shared memory; all of a thread's polls are in flight together
+    constexpr int H = kHeld<T>;
+    int ha[H];                    // word of the value in the pairs, -1: none
 #pragma unroll
-            for (int j = 0; j < 4; ++j) {
-                const int i = i0 + j * kST;
-                need[j] = i < nh3;
-                a[j] = need[j] ? from + (3L * A.halo[me.halo0 + i / 3] + i % 3) * W : from;
-            }
-            for (unsigned int n = 0;; ++n) {
-                bool wait = false;
-                T v[4];
-                bool got[4];
+    for (int j = 0; j < H; ++j) {
+        const int i = tid + j * kST;
+        ha[j] = i < nh3 ? 2 * W * (3 * A.halo[me.halo0 + i / 3] + i % 3) : -1;
+    }
+    T hu[H], hq[H];
+    auto gather = [&](unsigned int e, bool both) {
+        const unsigned long long* from = A.xu + (e & 1) * A.xu_half;
+        bool need[H];
 #pragma unroll
-                for (int j = 0; j < 4; ++j) got[j] = need[j] && get_value(a[j], v[j], A.tag0 + e);
+        for (int j = 0; j < H; ++j) need[j] = ha[j] >= 0;
+        for (unsigned int k = 0;; ++k) {
+            bool wait = false;
 #pragma unroll
-                for (int j = 0; j < 4; ++j) {
-                    if (got[j]) {
-                        smh[i0 + j * kST] = v[j];
-                        need[j] = false;
-                    }
-                    wait |= need[j];
-                }
-                if (!wait) break;
-                if (n > kSellSpin) { sbad = 1; break; }
-            }
+            for (int j = 0; j < H; ++j)
+                if (need[j]) need[j] = !get_pair(from + ha[j], hu[j], hq[j], A.tag0 + e, both);
+#pragma unroll
+            for (int j = 0; j < H; ++j) wait |= need[j];
+            if (!wait) break;
+            if (k > kSellSpin) { sbad = 1; break; }
+        }
+        for (int i = H * kST + tid; i < nh3; i += kST) {
+            const unsigned long long* a = from + 2L * W * (3 * A.halo[me.halo0 + i / 3] + i % 3);
+            T u, q;
+            for (unsigned int k = 0; !get_pair(a, u, q, A.tag0 + e, both); ++k)
+                if (k > kSellSpin) { sbad = 1; break; }
+            suq[2 * (i - H * kST)] = u;
+            suq[2 * (i - H * kST) + 1] = q;
         }
     };
-    T gam_l, del_l, rho_l;
-    // partial sums of this CTA: by warp, then (warp 0) in warp order; the others'
-    // copies travel as exchange e
-    auto reduce_out = [&](unsigned int e) {
-        for (int o = 16; o > 0; o >>= 1) {
-            gam_l += __shfl_xor_sync(0xffffffffu, gam_l, o);
-            del_l += __shfl_xor_sync(0xffffffffu, del_l, o);
-            rho_l += __shfl_xor_sync(0xffffffffu, rho_l, o);
-        }
-        if (lane == 0) { spart[warp][0] = gam_l; spart[warp][1] = del_l; spart[warp][2] = rho_l; }
-        __syncthreads();
-        if (warp == 0) {
-            T a = lane < kSW ? spart[lane][0] : T(0), b = lane < kSW ? spart[lane][1] : T(0),
-              c = lane < kSW ? spart[lane][2] : T(0);
-            for (int o = 8; o > 0; o >>= 1) {
-                a += __shfl_xor_sync(0xffffffffu, a, o);
-                b += __shfl_xor_sync(0xffffffffu, b, o);
-                c += __shfl_xor_sync(0xffffffffu, c, o);
-            }
-            if (nc == 1) {
-                if (lane == 0) { sred[0][0] = a; sred[0][1] = b; sred[0][2] = c; }
-            } else if (lane < 3) {
-                put_value(A.xr + (e & 1) * A.xr_half + (3L * (me.c0 + me.rank) + lane) * W,
-                          lane == 0 ? a : (lane == 1 ? b : c), A.tag0 + e);
-            }
-        }
-    };
-    // every CTA's sums of exchange e: a thread per CTA, added by warp
-    auto reduce_in = [&](unsigned int e) {
-        if (32 * warp >= nc) return;
-        T v[3] = {T(0), T(0), T(0)};
-        if (tid < nc) {
-            const unsigned long long* a = A.xr + (e & 1) * A.xr_half + 3L * (me.c0 + tid) * W;
-            for (unsigned int n = 0;; ++n) {
-                const bool g0 = get_value(a, v[0], A.tag0 + e), g1 = get_value(a + W, v[1], A.tag0 + e),
-                           g2 = get_value(a + 2 * W, v[2], A.tag0 + e);
-                if (g0 && g1 && g2) break;
-                if (n > kSellSpin) { sbad = 1; break; }
-            }
-        }
-        for (int o = 16; o > 0; o >>= 1)
+    // the halo's next p
+    auto advance_halo = [&](T alpha, T beta) {
 #pragma unroll
-            for (int j = 0; j < 3; ++j) v[j] += __shfl_xor_sync(0xffffffffu, v[j], o);
-        if (lane == 0)
-#pragma unroll
-            for (int j = 0; j < 3; ++j) sred[warp][j] = v[j];
+        for (int j = 0; j < H; ++j) {
+            const int i = tid + j * kST;
+            if (i < nh3) sph[i] = (hu[j] - alpha * hq[j]) + beta * sph[i];
+        }
+        for (int i = H * kST + tid; i < nh3; i += kST)
+            sph[i] = (suq[2 * (i - H * kST)] - alpha * suq[2 * (i - H * kST) + 1]) + beta * sph[i];
     };
-    // ---- u = M^{-1} r, w = A u, m = M^{-1} w
+    // ---- u = M^{-1} r, p = u
+    T nu_l = T(0), rr_l = T(0);
 #pragma unroll
     for (int t = 0; t < STEPS; ++t) {
-        u[t] = precond(t, r[t]);
-        publish(t, u[t], 0);
+        p[t] = precond(t, r[t]);
+        publish(t, 0, p[t], 0);
+        if (own[t]) sp[3 * lv[t] + l4] = p[t];
+        nu_l += r[t] * p[t];
+        rr_l += r[t] * r[t];
     }
-    __syncthreads();
-    if (nc > 1) gather(0);
-    __syncthreads();
-    if (sbad) {
-        if (tid == 0) atomicExch(A.err, 1);
-        return;
-    }
-    gam_l = del_l = rho_l = T(0);
+    if (nc > 1) {
+        gather(0, false);
 #pragma unroll
-    for (int t = 0; t < STEPS; ++t) {
-        T y0 = 0, y1 = 0, y2 = 0;
-        spmv(off[t], off[t] + wl[t], sm, y0, y1, y2);
-        spmv(off[t] + wl[t], off[t] + wt[t], smh, y0, y1, y2);
-        const T y = row_sum(y0, y1, y2);
-        w[t] = own[t] && !fixed[t] ? y : T(0);
-        m[t] = precond(t, w[t]);
-        publish(t, m[t], 1);
-        gam_l += r[t] * u[t];
-        del_l += w[t] * u[t];
-        rho_l += r[t] * r[t];
+        for (int j = 0; j < H; ++j)
+            if (tid + j * kST < nh3) sph[tid + j * kST] = hu[j];
+        for (int i = H * kST + tid; i < nh3; i += kST) sph[i] = suq[2 * (i - H * kST)];
     }
-    reduce_out(1);
-    // ---- iterations; warp 0 carries the scalar recurrences
+    // ---- iterations; warp 0 carries the scalars
     int it = 0;
-    T gam_prev = 1, inv_alpha = 0, tol2 = 0;  // gam and 1 / alpha of the previous iteration
-    for (unsigned int e = 1;; ++e) {
-        const T* mo = sm + (e & 1) * 3 * A.nvmax;
-        T y0[STEPS], y1[STEPS], y2[STEPS];
+    T tol2 = 0;
+    for (unsigned int e = 0;; ++e) {
+        __syncthreads();
+        // s = A p, q = M^{-1} s
+        T s[STEPS], v[kSums] = {T(0), nu_l, T(0), T(0), rr_l};  // p.s, r.u, r.q, s.q, r.r
 #pragma unroll
         for (int t = 0; t < STEPS; ++t) {
-            y0[t] = y1[t] = y2[t] = T(0);
-            spmv(off[t], off[t] + wl[t], mo, y0[t], y1[t], y2[t]);
+            T y0 = 0, y1 = 0, y2 = 0;
+            spmv(off[t], off[t] + wl[t], sp, y0, y1, y2);
+            spmv(off[t] + wl[t], off[t] + wt[t], sph, y0, y1, y2);
+            const T y = row_sum(y0, y1, y2);
+            s[t] = own[t] && !fixed[t] ? y : T(0);
+            const T q = precond(t, s[t]);
+            publish(t, 1, q, e);
+            v[0] += p[t] * s[t];
+            v[2] += r[t] * q;
+            v[3] += s[t] * q;
         }
-        if (nc > 1) {
-            gather(e);
-            reduce_in(e);
+        {
+            const T a = warp_sums(v, lane);
+            const int j = sum_value(lane);
+            if (l4 == 0 && j < kSums) spart[warp][j] = a;
         }
         __syncthreads();
+        // the CTA's sums (warp 0), the halo, then the instance's sums: warp j < kSums
+        // polls value j of every CTA
         if (warp == 0) {
-            T gam = 0, del = 0, rho = 0;
-            for (int k = 0; 32 * k < nc; ++k) { gam += sred[k][0]; del += sred[k][1]; rho += sred[k][2]; }
-            int stop = 0;
+#pragma unroll
+            for (int j = 0; j < kSums; ++j) v[j] = lane < kSW ? spart[lane][j] : T(0);
+            const T a = warp_sums(v, lane);
+            const int j = sum_value(lane);
+            if (nc == 1) {
+                if (l4 == 0 && j < kSums) sred[j] = a;
+                __syncwarp();
+            } else if (l4 == 0 && j < kSums) {
+                put_value(A.xr + (e & 1) * A.xr_half + (long)j * W * A.xr_row + me.c0 + me.rank, A.xr_row, a, A.tag0 + e);
+            }
+        }
+        if (nc > 1) {
+            gather(e, true);
+            if (warp < kSums) {
+                const unsigned long long* from = A.xr + (e & 1) * A.xr_half + (long)warp * W * A.xr_row + me.c0;
+                T sum = T(0);
+                // polls of sums that cannot be there yet hold up the stores of those that
+                // come: not before this CTA's own are out (FP64: they take 1000 cycles
+                // longer; in FP32 the halo's polls are wait enough)
+                if constexpr (sizeof(T) == 8) asm volatile("bar.sync 1, %0;" ::"n"(32 * kSums) : "memory");
+                for (int c0 = lane; c0 < nc; c0 += 32 * kPollCtas) {
+                    T val[kPollCtas];
+                    for (unsigned int k = 0;; ++k) {
+                        bool wait = false;
+#pragma unroll
+                        for (int i = 0; i < kPollCtas; ++i) {
+                            const int c = c0 + 32 * i;
+                            val[i] = T(0);
+                            if (c < nc) wait |= !get_value(from + c, A.xr_row, val[i], A.tag0 + e);
+                        }
+                        if (!wait) break;
+                        if (k > kSellSpin) { sbad = 1; break; }
+                    }
+#pragma unroll
+                    for (int i = 0; i < kPollCtas; ++i) sum += val[i];
+                }
+                for (int o = 16; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
+                if (lane == 0) sred[warp] = sum;
+                __syncwarp();
+                asm volatile("bar.sync 1, %0;" ::"n"(32 * kSums) : "memory");
+            }
+        }
+        if (warp == 0) {
+            const T mu = sred[0], nu = sred[1], de = sred[2], ga = sred[3], rr = sred[4];
             if (it == 0) {
                 const double tl = A.tol_inst ? fmax(A.tol_inst[me.inst], A.rel_tol) : A.rel_tol;
-                tol2 = (T)(tl * tl) * rho;
-                if (!(rho > T(0)) || !(rho > tol2)) stop = 1;
-            } else if (rho <= tol2) {
-                stop = 1;
+                tol2 = (T)(tl * tl) * rr;
             }
-            if (it >= A.max_iters) stop = 1;
-            const T beta = it == 0 ? T(0) : gam / gam_prev, alpha = gam / (del - beta * gam * inv_alpha);
-            if (!(alpha > T(0)) || !(alpha < T(INFINITY)) || !(beta < T(INFINITY))) stop = 1;  // breakdown: keep x
+            const T alpha = nu / mu;
+            // the next r.u as these sums predict it
+            T beta = (nu - T(2) * alpha * de + alpha * alpha * ga) / nu;
+            if (!(beta >= T(0)) || !(beta < T(INFINITY))) beta = T(0);
             if (lane == 0) {
                 sscal[0] = alpha;
                 sscal[1] = beta;
-                sstop = stop;
+                // converged, out of iterations, or broken down (x is kept)
+                sstop = !(rr > T(0)) || !(rr > tol2) || it >= A.max_iters || !(mu > T(0)) || !(alpha > T(0)) ||
+                        !(alpha < T(INFINITY));
             }
-            gam_prev = gam;
-            inv_alpha = T(1) / alpha;
         }
-#pragma unroll
-        for (int t = 0; t < STEPS; ++t) spmv(off[t] + wl[t], off[t] + wt[t], smh, y0[t], y1[t], y2[t]);
         __syncthreads();
         if (sbad) {
             if (tid == 0) atomicExch(A.err, 1);
@@ -514,27 +591,20 @@ __global__ void __launch_bounds__(kST, 1) k_pcg_sell(const SellArgs<T> A) {
         }
         if (sstop) break;
         const T alpha = sscal[0], beta = sscal[1];
-        gam_l = del_l = rho_l = T(0);
+        nu_l = rr_l = T(0);
 #pragma unroll
         for (int t = 0; t < STEPS; ++t) {
-            const T y = row_sum(y0[t], y1[t], y2[t]);
-            const T n = own[t] && !fixed[t] ? y : T(0);
-            z[t] = n + beta * z[t];
-            q[t] = m[t] + beta * q[t];
-            s[t] = w[t] + beta * s[t];
-            p[t] = u[t] + beta * p[t];
             x[t] += alpha * p[t];
             r[t] -= alpha * s[t];
-            u[t] -= alpha * q[t];
-            w[t] -= alpha * z[t];
-            m[t] = precond(t, w[t]);
-            publish(t, m[t], e + 1);
-            gam_l += r[t] * u[t];
-            del_l += w[t] * u[t];
-            rho_l += r[t] * r[t];
+            const T u = precond(t, r[t]);
+            publish(t, 0, u, e + 1);
+            p[t] = u + beta * p[t];
+            if (own[t]) sp[3 * lv[t] + l4] = p[t];
+            nu_l += r[t] * u;
+            rr_l += r[t] * r[t];
         }
+        advance_halo(alpha, beta);
         ++it;
-        reduce_out(e + 1);
     }
 #pragma unroll
     for (int t = 0; t < STEPS; ++t)
@@ -544,7 +614,9 @@ __global__ void __launch_bounds__(kST, 1) k_pcg_sell(const SellArgs<T> A) {
 
 // dynamic shared memory besides the slot rows
 template <class T>
-size_t sell_fixed(int nvmax, int nhmax) { return sizeof(T) * (6 * (size_t)nvmax + 3 * (size_t)nhmax) + 16; }
+size_t sell_fixed(int nvmax, int nhmax) { 
+    return sizeof(T) * (3 * (size_t)nvmax + 3 * (size_t)nhmax + 2 * (size_t)halo_rest<T>(nhmax)) + 16;
+}
 template <class T>
 size_t sell_row() { return 32 * (9 * sizeof(T) + 2); }
 
@@ -640,8 +712,8 @@ int sell_solve(Arena& A, Work& W, const std::vector<int>& which, const double* b
     Work::Sell& P = W.sell;
     const long nC = (long)P.cta.size();
     DBuf& bx = W[W_SELL_XCH];
-    const size_t xm_half = 3 * (size_t)A.V * words<T>(), xr_half = 3 * (size_t)nC * words<T>();
-    const size_t need = 8 * 2 * (xm_half + xr_half) + 64;
+    const size_t xu_half = 6 * (size_t)A.V * words<T>(), xr_half = (size_t)kSums * nC * words<T>();
+    const size_t need = 8 * 2 * (xu_half + xr_half) + 64;
     if (need > P.xch_bytes || P.tag > 0xe0000000u) {
         if (bx.ensure(need)) return IDP_ERR_CUDA;
         P.xch_bytes = bx.bytes;
@@ -685,10 +757,11 @@ int sell_solve(Arena& A, Work& W, const std::vector<int>& which, const double* b
         a.dbc = A.dbc;
         a.b = b;
         a.x = x;
-        a.xm = bx.as<unsigned long long>();
-        a.xr = a.xm + 2 * xm_half;
-        a.xm_half = (long)xm_half;
+        a.xu = bx.as<unsigned long long>();
+        a.xr = a.xu + 2 * xu_half;
+        a.xu_half = (long)xu_half;
         a.xr_half = (long)xr_half;
+        a.xr_row = nC;
         a.tag0 = P.tag;
         a.nvmax = nvmax;
         a.nhmax = nhmax;
