@@ -25,8 +25,6 @@ COMMON = ["-O3", "-lineinfo", "-std=c++17", "-Xcompiler", "-fPIC", "--expt-relax
 EXACT_FP64 = {"contact.cu", "ccd.cu", "flow.cu", "dirichlet.cu"}
 UNITS = ["prims.cu", "tet.cu", "contact.cu", "barrier.cu", "ccd.cu", "solver.cu", "pcg_sell.cu", "precond.cu", "vecops.cu",
          "flow.cu", "shell.cu", "shell_elastic.cu", "dirichlet.cu", "surface.cu", "engine.cpp", "server.cpp"]
-HEADERS = ["common.cuh", "prims.cuh", "geom.cuh", "grid.cuh", "engine.hpp", "predicates.cuh", "psd.cuh", "far.cuh",
-           "reduce.cuh"]
 
 
 def nvcc():
@@ -34,9 +32,13 @@ def nvcc():
     return p
 
 
+def dependencies():
+    """Headers that every unit counts as depending on: all of the library's."""
+    return [os.path.join(d, h) for d in (SRC, INCLUDE) for h in sorted(os.listdir(d)) if h.endswith((".cuh", ".hpp", ".h"))]
+
+
 def _newest_dep():
-    deps = [os.path.join(SRC, h) for h in HEADERS] + [os.path.join(INCLUDE, "idp_gb300.h")]
-    return max(os.path.getmtime(d) for d in deps)
+    return max(os.path.getmtime(d) for d in dependencies())
 
 
 def _compile(unit, extra=()):
