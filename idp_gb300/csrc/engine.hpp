@@ -6,6 +6,7 @@
 #include <vector>
 #include <string>
 #include <chrono>
+#include "attributes.hpp"
 #include "common.cuh"
 #include "reduce.cuh"
 #include "../../include/idp_gb300.h"
@@ -323,6 +324,8 @@ struct Work {
     unsigned long long grid_prof[5] = {0, 0, 0, 0, 0};  // grid PCG phase ns (IDP_PROFILE)
     bool grid_prof_init = false;
     int sum_counters = 0;                    // counters of W_SUMCNT cleared so far
+    KernelAttributes attr;
+    int grid_max[2] = {0, 0};                // CTAs of the grid-wide PCG that fit the device, {FP32, FP64}
     uint32_t* hpin = nullptr;                // 64 words of pinned host memory for batched readbacks
     uint32_t* pinned() {
         if (!hpin && cudaMallocHost(reinterpret_cast<void**>(&hpin), 64 * sizeof(uint32_t)) != cudaSuccess)

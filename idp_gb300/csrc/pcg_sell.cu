@@ -46,7 +46,6 @@
 // sums while others gather the halo (5.8 against 4.5 per iteration of that blob in
 // FP32), waits before the first poll, 6 or 8 polls in flight.
 #include <algorithm>
-#include <atomic>
 #include "engine.hpp"
 
 namespace idp {
@@ -621,14 +620,10 @@ template <class T>
 size_t sell_row() { return 32 * (9 * sizeof(T) + 2); }
 
 template <class T, int STEPS>
-cudaError_t launch_steps(const cudaLaunchConfig_t& cfg, const SellArgs<T>& a) {
-    static std::atomic<bool> attr{false};  // one per instantiation
-    if (!attr.load()) {
-        const cudaError_t e = cudaFuncSetAttribute(k_pcg_sell<T, STEPS>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                                   kSellSmem);
-        if (e != cudaSuccess) return e;
-        attr.store(true);
-    }
+cudaError_t launch_steps(Work& W, const cudaLaunchConfig_t& cfg, const SellArgs<T>& a) {
+    const cudaError_t e = W.attr.set(reinterpret_cast<const void*>(&k_pcg_sell<T, STEPS>),
+                                     cudaFuncAttributeMaxDynamicSharedMemorySize, kSellSmem);
+    if (e != cudaSuccess) return e;
     ::idp::count_launch();
     return cudaLaunchKernelEx(&cfg, k_pcg_sell<T, STEPS>, a);
 }
@@ -782,8 +777,8 @@ int sell_solve(Arena& A, Work& W, const std::vector<int>& which, const double* b
         cfg.attrs = at;
         cfg.numAttrs = 1;
         const int steps = (nvmax + kSW * kSliceRows - 1) / (kSW * kSliceRows);
-        IDP_CUDA_TRY(steps <= 1 ? (launch_steps<T, 1>(cfg, a))
-                                : (steps == 2 ? (launch_steps<T, 2>(cfg, a)) : (launch_steps<T, 3>(cfg, a))));
+        IDP_CUDA_TRY(steps <= 1 ? (launch_steps<T, 1>(W, cfg, a))
+                                : (steps == 2 ? (launch_steps<T, 2>(W, cfg, a)) : (launch_steps<T, 3>(W, cfg, a))));
         W.stats.pcg_launches += 1;
     }
     return IDP_OK;

@@ -14,7 +14,6 @@
 #include <deque>
 #include <numeric>
 #include <vector>
-#include <atomic>
 #include <cooperative_groups.h>
 #include "engine.hpp"
 
@@ -349,12 +348,8 @@ int factor_blocks(Arena& A, Work& W, const int* list, int nbig, int nfew, cudaSt
                                 cl.n, cl.off, cl.vert, cl.vcl, cl.vloc, cl.doff, A.rowptr, A.colidx,
                                 W[W_BSR_VAL].as<T>(), W[W_TAIL_ROWPTR].as<int>(), W[W_TAIL_COL].as<int>(),
                                 W[W_TAIL_VAL].as<T>(), A.dbc, K));
-    static std::atomic<bool> attr{false};  // one per instantiation
-    if (!attr.load()) {
-        IDP_CUDA_TRY(cudaFuncSetAttribute(k_cl_invert<T>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                          (int)invert_smem_bytes<T>()));
-        attr.store(true);
-    }
+    IDP_CUDA_TRY(W.attr.set(reinterpret_cast<const void*>(&k_cl_invert<T>),
+                            cudaFuncAttributeMaxDynamicSharedMemorySize, (int)invert_smem_bytes<T>()));
     for (int part = 0; part < 2; ++part) {
         const int n = part ? nfew : nbig, cs = part ? 1 : kInvCluster;
         if (!n) continue;

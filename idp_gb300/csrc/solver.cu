@@ -14,7 +14,6 @@
 // recovers the direction by iterative refinement against an FP64 residual
 // r = b - A x (FP32 matrix, FP64 accumulation); FP64 mode runs PCG in FP64.
 #include <algorithm>
-#include <atomic>
 #include <cooperative_groups.h>
 #include "engine.hpp"
 #include "prims.cuh"
@@ -1408,11 +1407,8 @@ static int pcg_inner(Arena& A, Work& W, const double* b, double rel_tol, int max
         std::vector<int> flat;
         for (int k = 0; k < 5; ++k) flat.insert(flat.end(), by_size[k].begin(), by_size[k].end());
         IDP_CUDA_TRY(cudaMemcpyAsync(d_list, flat.data(), sizeof(int) * flat.size(), cudaMemcpyHostToDevice, s));
-        static std::atomic<bool> attr_set{false};  // one per instantiation
-        if (!attr_set.load()) {
-            cudaFuncSetAttribute(k_pcg_cluster<T>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
-            attr_set.store(true);
-        }
+        IDP_CUDA_TRY(W.attr.set(reinterpret_cast<const void*>(&k_pcg_cluster<T>),
+                                cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
         ClusterPC<T> pcb;
         pcb.vcl = W.cl.vcl;
         pcb.ioff = W.cl.ioff;
@@ -1458,17 +1454,16 @@ static int pcg_inner(Arena& A, Work& W, const double* b, double rel_tol, int max
     account(small);
     if (!any_large) return IDP_OK;
     // large instances: grid-wide PCG, in waves of at most gmax CTAs
-    static std::atomic<int> gmax_cache{0};  // one per instantiation
-    int gmax = gmax_cache.load();
+    int& gmax = W.grid_max[sizeof(T) == 8];
     if (!gmax) {
         int dev = 0, nsm = 0, per = 0;
         IDP_CUDA_TRY(cudaGetDevice(&dev));
         IDP_CUDA_TRY(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev));
-        IDP_CUDA_TRY(cudaFuncSetAttribute(k_pcg_grid<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, kGridSmem));
+        IDP_CUDA_TRY(W.attr.set(reinterpret_cast<const void*>(&k_pcg_grid<T>),
+                                cudaFuncAttributeMaxDynamicSharedMemorySize, kGridSmem));
         IDP_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_pcg_grid<T>, GP_THREADS, kGridSmem));
+        if (nsm * per <= 0) return IDP_ERR_CUDA;
         gmax = nsm * per;
-        if (gmax <= 0) return IDP_ERR_CUDA;
-        gmax_cache.store(gmax);
     }
     const long vper = W.grid_vper;
     std::vector<GridCta> plan;
