@@ -451,15 +451,17 @@ namespace {
 // scratch below. One launch: a thread per tet in CTAs of 64 (a mesh of 10,000
 // tets fills every SM; CTAs of 1024 tets left all but ten idle and took 33 us),
 // larger chunks once there would be more than kNoAllocMaxChunks of them, and the
-// last CTA to finish adds the chunk sums in a fixed order and clears the
-// scratch's counter and flag for the next call.
+// last CTA to finish adds the chunk sums in a fixed order. The arrival counter and
+// the flag are cleared in stream order before the launch, not by the last CTA: calls
+// that overlap against the rule can leave any count behind, and that must not reach a
+// later call.
 constexpr int kNoAllocThreads = 64;
 constexpr int kNoAllocMaxChunks = 16384;
 constexpr long kNoAllocMaxTets = 16777216;  // per call
 constexpr size_t kNoAllocScratchBytes = sizeof(double) * kNoAllocMaxChunks + 256;
 // Held by every GPU that loads the library, until exit (128 KB + 256 B).
 // Every call shares it: chunk sums (overwritten), inversion flag and arrival
-// counter (zero when the library is loaded, and again after every call).
+// counter (both cleared by every call).
 static __device__ __align__(256) unsigned char g_tet_energy_scratch[kNoAllocScratchBytes];
 
 __global__ void __launch_bounds__(kNoAllocThreads) k_tet_energy_noalloc(
@@ -501,8 +503,6 @@ __global__ void __launch_bounds__(kNoAllocThreads) k_tet_energy_noalloc(
     if (threadIdx.x == 0) {
         *energy = a;
         *inverted = __ldcg(bad_flag);
-        *bad_flag = 0;
-        *counter = 0;
     }
 }
 
@@ -574,6 +574,9 @@ extern "C" int idp_tet_energy_noalloc(int T, const int32_t* tets, const double* 
         scratch = g_noalloc_addr[dev];
     }
     cudaStream_t s = static_cast<cudaStream_t>(stream);
+    if (cudaMemsetAsync(scratch + sizeof(double) * kNoAllocMaxChunks, 0, sizeof(int) + sizeof(unsigned int), s) !=
+        cudaSuccess)
+        return IDP_ERR_CUDA;
     int chunk = kNoAllocThreads;
     while ((T + (long)chunk - 1) / chunk > kNoAllocMaxChunks) chunk *= 2;
     const int nchunks = T > 0 ? (T + chunk - 1) / chunk : 1;

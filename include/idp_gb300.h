@@ -441,7 +441,8 @@ int idp_newton_direction(idp_ctx* ctx, int inst, const double* X, double* p, int
  * At most 16,777,216 tets per call (IDP_ERR_CAPACITY beyond). Scratch is a
  * fixed 128 KB device array inside the library shared by every call on a GPU:
  * calls that overlap on the GPU (other streams, other threads) race on it, so
- * order them. The first call on each device looks up that array's device
+ * order them; the results of calls that did overlap are undefined, those of later
+ * ones are not affected. The first call on each device looks up that array's device
  * address (again after the device's context is re-created, e.g. by
  * cudaDeviceReset). */
 int idp_tet_energy_noalloc(int T, const int32_t* tets, const double* X, const double* IB, const double* vol,

@@ -108,3 +108,45 @@ def test_tet_energy_noalloc_matches_context_entry(gpu_lib, oracle):
                                         inverted.data_ptr(), stream)
     assert rc == idp.IDP_ERR_CAPACITY
     ctx.close()
+
+
+@pytest.mark.parametrize("n", [(1, 1, 1), (6, 6, 24)], ids=lambda n: "x".join(map(str, n)))
+def test_overlapping_calls_leave_nothing_behind(gpu_lib, n):
+    """Calls that overlap against the rule may spoil one another's results (the
+    arrival counter and the flag are shared, every access stays in the scratch and
+    nothing waits), but not a call that comes after them: every call starts from a
+    cleared counter and flag, so its energy and flag are those from before."""
+    import torch
+
+    import idp_gb300 as idp
+    from idp_gb300 import meshgen
+
+    def arrays(n, mirror):
+        X0, tets = meshgen.bar(*n, seed=0)
+        IB, vol = _rest(X0, tets)
+        X = X0 * np.array([-1.0 if mirror else 1.01, 1.0, 1.0])
+        one = np.ones(tets.shape[0])
+        return [tets.shape[0], _dev(torch, tets, np.int32)] + [_dev(torch, a, np.float64) for a in (X, IB, vol, one, one)]
+
+    out = [(torch.zeros(1, dtype=torch.float64, device="cuda"), torch.zeros(1, dtype=torch.int32, device="cuda"))
+           for _ in range(3)]
+
+    def call(a, o, stream):
+        assert gpu_lib.idp_tet_energy_noalloc(a[0], *[t.data_ptr() for t in a[1:]], 0.01, o[0].data_ptr(), o[1].data_ptr(),
+                                              C.c_void_p(stream.cuda_stream)) == idp.IDP_OK
+
+    mine, other = arrays(n, False), arrays((13, 11, 30), True)
+    main, side = torch.cuda.current_stream(), torch.cuda.Stream()
+    call(mine, out[0], main)
+    torch.cuda.synchronize()
+    want = float(out[0][0].item())
+    assert want > 0 and int(out[0][1].item()) == 0
+    for _ in range(10):
+        for _ in range(4):
+            call(other, out[1], side)
+            call(mine, out[2], main)
+        torch.cuda.synchronize()
+        out[0][0].fill_(math.nan)
+        call(mine, out[0], main)
+        torch.cuda.synchronize()
+        assert float(out[0][0].item()) == want and int(out[0][1].item()) == 0
