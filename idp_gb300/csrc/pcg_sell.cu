@@ -641,7 +641,7 @@ static int sell_rows(const Work& W, long V, int sms) {
 
 int sell_plan(Arena& A, Work& W, cudaStream_t s) {
     Work::Sell& P = W.sell;
-    P.ready = true;
+    P.ready = false;  // until the layout is on the device: a plan that failed is made again
     P.first.assign(A.nI, -1);
     P.cta.clear();
     int dev = 0, sms = 0;
@@ -668,7 +668,10 @@ int sell_plan(Arena& A, Work& W, cudaStream_t s) {
             P.cta.push_back(c);
         }
     }
-    if (P.cta.empty()) return IDP_OK;
+    if (P.cta.empty()) {
+        P.ready = true;
+        return IDP_OK;
+    }
     const long nC = (long)P.cta.size();
     const unsigned int slot_cap = (unsigned int)std::min<long>(A.B / 12 + 4 * slices + 64, 0x7fffffffL / 32);
     const unsigned int halo_cap = (unsigned int)std::min<long>(A.B + 64, 0x7fffffffL);
@@ -695,6 +698,7 @@ int sell_plan(Arena& A, Work& W, cudaStream_t s) {
     IDP_CUDA_TRY(cudaStreamSynchronize(s));
     for (const SellCta& c : P.cta)  // an instance with a CTA that did not fit keeps to the other kernels
         if (c.nsr < 0) P.first[c.inst] = -1;
+    P.ready = true;
     return IDP_OK;
 }
 
