@@ -206,6 +206,16 @@ int set_mask(idp_ctx* c, const std::vector<unsigned char>& m) {
     return IDP_OK;
 }
 
+// directions of the instances of m, the mask on the device. The refinement narrows
+// that mask and puts it back only when it ends well: after an error its state is unknown.
+int solve_directions(idp_ctx* c, bool fp64, const std::vector<unsigned char>& m, std::vector<int>& its,
+                     std::vector<double>& rel, const double* tol = nullptr) {
+    const int rc = pcg_solve(c->A, c->W, c->cs, fp64, c->A.g, c->A.dir, c->P.pcg_rel_tol, c->P.pcg_max_iters, m, its,
+                             rel, c->s, tol);
+    if (rc) c->mask_dev.clear();
+    return rc;
+}
+
 template <class T>
 int fetch(idp_ctx* c, const T* d, std::vector<T>& h) {
     h.resize(c->A.nI);
@@ -1682,9 +1692,7 @@ int step_iterate(idp_ctx* c, int max_iters, idp_result* results, int* n_active) 
             std::vector<int> its;
             std::vector<double> rel;
             IDP_CUDA_TRY(cudaStreamWaitEvent(s, c->ev_vox, 0));  // the side stream is idle during the PCG
-            if ((rc = pcg_solve(A, W, c->cs, fp64, A.g, A.dir, c->P.pcg_rel_tol, c->P.pcg_max_iters, newton, its, rel, s,
-                                 tol.data())))
-                return rc;
+            if ((rc = solve_directions(c, fp64, newton, its, rel, tol.data()))) return rc;
             for (int i = 0; i < nI; ++i)
                 if (newton[i]) st[i].pcg_iters += its[i];
             if (!fp64) {
@@ -1701,9 +1709,7 @@ int step_iterate(idp_ctx* c, int max_iters, idp_result* results, int* n_active) 
                 if (any_fb) {
                     if ((rc = set_mask(c, fb))) return rc;
                     if ((rc = eval_hessian(c, A.X, true))) return rc;
-                    if ((rc = pcg_solve(A, W, c->cs, true, A.g, A.dir, c->P.pcg_rel_tol, c->P.pcg_max_iters, fb, its, rel,
-                                         s, tol.data())))
-                        return rc;
+                    if ((rc = solve_directions(c, true, fb, its, rel, tol.data()))) return rc;
                     for (int i = 0; i < nI; ++i)
                         if (fb[i]) {
                             st[i].pcg_iters += its[i];
@@ -2335,8 +2341,7 @@ int idp_newton_direction(idp_ctx* c, int i, const double* X, double* p, int* ite
     if ((rc = eval_hessian(c, c->A.Xprev))) return rc;
     std::vector<int> its;
     std::vector<double> rel;
-    if ((rc = pcg_solve(c->A, c->W, c->cs, c->P.mode == IDP_MODE_FP64, c->A.g, c->A.dir, c->P.pcg_rel_tol,
-                        c->P.pcg_max_iters, c->mask_dev, its, rel, c->s)))
+    if ((rc = solve_directions(c, c->P.mode == IDP_MODE_FP64, std::vector<unsigned char>(c->mask_dev), its, rel)))
         return rc;
     if ((rc = download3(c, i, c->A.dir, p))) return rc;
     IDP_CUDA_TRY(cudaStreamSynchronize(c->s));

@@ -1579,10 +1579,9 @@ static int pcg_inner(Arena& A, Work& W, const double* b, double rel_tol, int max
     return IDP_OK;
 }
 
-int pcg_solve(Arena& A, Work& W, const ContactSet& cs, bool fp64, const double* rhs, double* sol, double rel_tol,
-              int max_iters, const std::vector<unsigned char>& mask, std::vector<int>& iters_out,
-              std::vector<double>& relres_out, cudaStream_t s, const double* tol_host) {
-    (void)cs;
+static int pcg_refine(Arena& A, Work& W, bool fp64, const double* rhs, double* sol, double rel_tol, int max_iters,
+                      const std::vector<unsigned char>& mask, std::vector<int>& iters_out,
+                      std::vector<double>& relres_out, cudaStream_t s, const double* tol_host) {
     const int nI = A.nI;
     long n3 = 3 * A.V;
     iters_out.assign(nI, 0);
@@ -1632,22 +1631,22 @@ int pcg_solve(Arena& A, Work& W, const ContactSet& cs, bool fp64, const double* 
     const double inner_tol = fp64 ? rel_tol : std::max(rel_tol, 2e-3);
     std::vector<unsigned char> act = mask;
     bool changed = false;  // the mask on the device is not `mask`
-    int rc = IDP_OK;
     for (int ref = 0; ref < max_refine && std::find(act.begin(), act.end(), 1) != act.end(); ++ref) {
         std::vector<int> its;
         SellPending pend;
+        int rc = IDP_OK;
         if (fp64) {
             double* e = nullptr;
-            if ((rc = pcg_inner<double>(A, W, res, inner_tol, max_iters, act, its, pend, &e, s))) break;
+            if ((rc = pcg_inner<double>(A, W, res, inner_tol, max_iters, act, its, pend, &e, s))) return rc;
             (::idp::count_launch(), k_add_correction<double><<<grid_for(A.V), kBlock, 0, s>>>(A.V, A.vinst, A.active, e, sol));
         } else {
             float* e = nullptr;
-            if ((rc = pcg_inner<float>(A, W, res, inner_tol, max_iters, act, its, pend, &e, s))) break;
+            if ((rc = pcg_inner<float>(A, W, res, inner_tol, max_iters, act, its, pend, &e, s))) return rc;
             (::idp::count_launch(), k_add_correction<float><<<grid_for(A.V), kBlock, 0, s>>>(A.V, A.vinst, A.active, e, sol));
         }
-        if ((rc = residual_async())) break;
+        if ((rc = residual_async())) return rc;
         IDP_CUDA_TRY(cudaStreamSynchronize(s));
-        if ((rc = fp64 ? sell_finish<double>(A, W, pend, its) : sell_finish<float>(A, W, pend, its))) break;
+        if ((rc = fp64 ? sell_finish<double>(A, W, pend, its) : sell_finish<float>(A, W, pend, its))) return rc;
         bool drop = false;
         for (int i = 0; i < nI; ++i) {
             if (!act[i]) continue;
@@ -1667,8 +1666,16 @@ int pcg_solve(Arena& A, Work& W, const ContactSet& cs, bool fp64, const double* 
             changed = true;
         }
     }
-    if (rc) W.sell.xch_bytes = 0;  // tags may be in use: clear the exchange words before the next solve
     if (changed) IDP_CUDA_TRY(cudaMemcpyAsync(A.active, mask.data(), nI, cudaMemcpyHostToDevice, s));
+    return IDP_OK;
+}
+
+int pcg_solve(Arena& A, Work& W, const ContactSet& cs, bool fp64, const double* rhs, double* sol, double rel_tol,
+              int max_iters, const std::vector<unsigned char>& mask, std::vector<int>& iters_out,
+              std::vector<double>& relres_out, cudaStream_t s, const double* tol_host) {
+    (void)cs;
+    const int rc = pcg_refine(A, W, fp64, rhs, sol, rel_tol, max_iters, mask, iters_out, relres_out, s, tol_host);
+    if (rc) W.sell.xch_bytes = 0;  // tags may be in use: clear the exchange words before the next solve
     return rc;
 }
 

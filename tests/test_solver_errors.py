@@ -4,13 +4,14 @@ failed must not count as done, or the next solve would launch on a layout that
 was never made.
 """
 import os
+import re
 import subprocess
 
 import pytest
 
 from idp_gb300 import build
 
-PROGRAM = r"""
+LAYOUT = r"""
 #include "engine.hpp"
 using namespace idp;
 int main() {
@@ -22,6 +23,24 @@ int main() {
     if (sell_plan(A, W, nullptr) == IDP_OK) return 1;
     if (W.sell.ready) return 2;  // the next solve makes the layout
     return 0;
+}
+"""
+
+SOLVE = r"""
+#include "engine.hpp"
+using namespace idp;
+int main() {
+    Arena A;
+    Work W;
+    ContactSet cs;
+    A.nI = 1;
+    A.V = 500;
+    A.v_off = {0, 500};
+    W.sell.xch_bytes = 4096;
+    std::vector<int> its;
+    std::vector<double> rel;
+    if (pcg_solve(A, W, cs, false, nullptr, nullptr, 1e-6, 10, {1}, its, rel, nullptr) == IDP_OK) return 1;
+    return W.sell.xch_bytes == 0 ? 0 : 2;
 }
 """
 
@@ -46,4 +65,21 @@ def without_device(tmp_path_factory):
 
 
 def test_a_failed_layout_is_made_again(without_device):
-    assert without_device("layout", PROGRAM) == 0
+    assert without_device("layout", LAYOUT) == 0
+
+
+def test_a_failed_solve_clears_the_exchange(without_device):
+    """Its tags may have been used: the words are cleared before the next solve."""
+    assert without_device("solve", SOLVE) == 0
+
+
+def test_the_mask_of_a_failed_solve_is_unknown():
+    """The refinement narrows the mask on the device and puts it back only when it
+    ends well; set_mask skips an upload that it takes for held already. So every
+    solve of the engine goes through the one function that forgets the mask on an
+    error (the state is the library's own: read from the source)."""
+    text = open(os.path.join(build.SRC, "engine.cpp")).read()
+    assert len(re.findall(r"\bpcg_solve\(", text)) == 1
+    body = text[text.index("int solve_directions("):]
+    body = body[:body.index("\n}\n")]
+    assert "pcg_solve(" in body and "if (rc) c->mask_dev.clear();" in body
