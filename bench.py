@@ -17,8 +17,9 @@ steps and K timed steps continue one flow sequence (20 steps for K=17, W=3).
 * e2e: the same K steps through the public API with host buffers: pinned
   positions uploaded, normal flow set, solved, positions read back, all in
   the timed region (host wall clock around synchronous calls).
-* roofline: the cluster PCG kernel (dominant), algorithmic bytes per launch /
-  event time, against MEASURED_PEAKS.json hbm_gbs.
+* roofline: the PCG kernel (dominant), algorithmic bytes per launch / event time,
+  against MEASURED_PEAKS.json hbm_gbs. The matrix stays in shared memory, so the
+  fraction says how fast that stream is consumed; "limited_by" names what limits it.
 * cpu_baseline and oracle_check: the CPU oracle (FP64, sparse Cholesky)
   solving the first timed step(s) of the same full-size blob from the GPU's
   start states (at least one step, more while --cpu-sample-s lasts): its
@@ -480,6 +481,7 @@ def run_flow(args):
         "roofline": {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s",
                      "frac": (achieved / peak) if achieved else None,
                      "traffic": traffic.get("bytes_per_launch") if traffic else None,
+                     "limited_by": "shared-memory reads of the matrix and the exchange of each iteration, not HBM",
                      "kernel": "k_pcg_sell (persistent CTAs: matrix rows resident in shared memory, vectors in "
                                "registers, FP32 SpMV + block-Jacobi, tagged exchange per iteration)",
                      "achieved_basis": "algorithmic bytes of the PCG iterations / PCG event time",
@@ -719,7 +721,7 @@ def run_gpu(args):
                      "frac": (achieved / peak) if achieved else None,
                      "traffic": None,  # the committed ncu capture covers the PCG on the blob only
                      "kernel": "k_pcg_cluster (block-Jacobi + contact-block PCG, one thread-block cluster per "
-                               "instance)",
+                               "instance in contact) and k_pcg_sell (instances without contact)",
                      "peak_source": peak_kind},
         "gpu_launches": launches,
         "clocks": clocks.summary(),
@@ -1092,7 +1094,7 @@ def run_shellflow(args):
                 "d2h_bytes_per_step": 3 * X.shape[0] * 8},
         "roofline": {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s",
                      "frac": (achieved / peak) if achieved else None, "traffic": None,
-                     "kernel": "k_pcg_cluster", "peak_source": peak_kind},
+                     "kernel": "k_pcg_cluster (with contact), k_pcg_sell (without)", "peak_source": peak_kind},
         "gpu_launches": launches,
         "clocks": clocks.summary(),
     }

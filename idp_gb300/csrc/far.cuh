@@ -2,7 +2,8 @@
 // taken relative to a point of their instance and rounded to FP32; a pair is
 // called far only when a direction separates its two hulls by more than `lim`
 // (the support-function bound, which holds for every direction: the one tried
-// joins the pair's approximately closest points). Callers add kFarMargin times
+// joins the pair's approximately closest points, by the usual clamped solution of
+// their two linear equations). Callers add kFarMargin times
 // the instance's extent to lim, well above the rounding of the coordinates
 // (1e-7 of it) and of the products (1e-6), so that no pair that the FP64 tests
 // accept is rejected. NaN and degenerate pairs are never called far.

@@ -77,7 +77,9 @@ __global__ void rs_scatter(const uint64_t* __restrict__ keys, const uint32_t* __
 // per 8 bits of the key; the ranks by the n^2 / 1024 binary searches. 18-bit /
 // 42-bit keys, radix passes -> tiles: 1,000 items 48 / 89 -> 7.6 us, 8,192 items
 // 58 / 98 -> 14 us, 32,768 items 74 / 134 -> 28 us, 50,000 items 77 / 136 -> 57 us,
-// 100,000 items 78 / 139 against 167 us: the radix passes above kMergeMax.
+// 100,000 items 78 / 139 against 167 us. kMergeMax stays below the crossing of both
+// widths, which was not looked for between 50,000 and 100,000 items (by these figures
+// near 60,000 at 18 bits and 90,000 at 42).
 constexpr int MS_TILE = 1024;
 constexpr int MS_LANES = 8;  // per item, each with every 8th tile
 constexpr int MS_IDX = 10;   // bits of a place in a tile

@@ -49,7 +49,7 @@ __device__ bool chol_pd(const T* A, int n) {
 // (FP32) or the FP64 pipe. 22,000 random 12x12 matrices: FP32 0.17 ms (3.4 ms
 // for two-sided sweeps over A and V in shared memory, one warp per matrix,
 // whose FP32 runs never met their stopping test and took 20 sweeps), FP64
-// 4.3 ms (7.1 ms).
+// 4.3 to 4.6 ms (7.1 ms).
 constexpr int kPsdDim = 12;                 // row stride of the matrices in shared memory
 constexpr int kPsdGroup = 16;               // lanes per matrix
 constexpr int kPsdThreads = 128;

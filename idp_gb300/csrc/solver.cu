@@ -28,7 +28,8 @@ namespace {
 // nine, so that the element blocks are read and the row of blocks written as
 // whole lines (220,000 blocks: 71 us with one thread per block, 42 with nine).
 // FP32: one, because the source list is then walked once per block (613,000
-// blocks: 75 us with one thread per block, 174 with nine).
+// blocks: 75 us with one thread per block, 174 with nine). Each type was measured
+// at that one size.
 template <class T>
 constexpr int kAsmThreads = sizeof(T) == 8 ? 9 : 1;
 
@@ -126,9 +127,11 @@ __global__ void k_diag_inv(long V, const int* __restrict__ diagblk, const T* __r
 // Row v of A x in FP64 (FP32 or FP64 matrix) by 8 lanes: lane l takes blocks
 // l, l + 8, ... of the row and of its contact tail; lane j < 3 gets component j.
 // Bound by latency on small meshes (a thread per row was a chain of up to 19
-// dependent gathers: 160 rows 35 us, with 8 lanes 15; 17,000 rows 58 and 34) and by
+// dependent gathers: 160 rows 35 us, with 8 lanes 13; 18,000 rows 58 and 32) and by
 // the FP64 pipe on large ones, so the sums over the lanes halve the components a
-// lane carries: 4 additions, not 9. All lanes of the warp call this together.
+// lane carries: 4 additions, not 9. At 49,863 rows a thread per row is the faster by a
+// little: 52 us and 14 for the two kernels of the sums, against 73 with them.
+// All lanes of the warp call this together.
 template <class T>
 __device__ __forceinline__ double row8_f64(bool on, long v, int l, const int* __restrict__ rowptr,
                                          const int* __restrict__ colidx, const T* __restrict__ val,

@@ -454,7 +454,8 @@ namespace {
 // last CTA to finish adds the chunk sums in a fixed order. The arrival counter and
 // the flag are cleared in stream order before the launch, not by the last CTA: calls
 // that overlap against the rule can leave any count behind, and that must not reach a
-// later call.
+// later call. (It costs 1 us of the 11.2 of a call on 9,765 tets; two kernels, the second
+// adding the chunk sums in one thread, took 35.9.)
 constexpr int kNoAllocThreads = 64;
 constexpr int kNoAllocMaxChunks = 16384;
 constexpr long kNoAllocMaxTets = 16777216;  // per call
