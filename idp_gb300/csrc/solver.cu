@@ -241,7 +241,8 @@ __global__ void k_spmv_plain(long V, const int* __restrict__ vinst, const unsign
 }
 
 // ---- per-vertex Newton kernels
-// 4 lanes per vertex: lane l < 3 adds component l of its corners, in their order
+// 4 lanes per vertex: lane l < 3 adds component l of the inertia term and of its
+// corners, in their order
 __global__ void k_grad_gather_tet(long V, const int* __restrict__ vinst, const unsigned char* __restrict__ active,
                                   const int* __restrict__ vcp, const int* __restrict__ vc,
                                   const double* __restrict__ tg, const double* __restrict__ mass,
@@ -250,13 +251,13 @@ __global__ void k_grad_gather_tet(long V, const int* __restrict__ vinst, const u
     const int l = threadIdx.x & 3;
     if (v >= V || l == 3 || !active[vinst[v]]) return;
     const int k1 = vcp[v + 1];
-    double s = 0;
+    double s = mass[v] * (X[3 * v + l] - Xt[3 * v + l]);
 #pragma unroll 8
     for (int k = vcp[v]; k < k1; ++k) {
         const int code = vc[k];  // tet*4 + corner
         s += tg[12 * (long)(code >> 2) + 3 * (code & 3) + l];
     }
-    g[3 * v + l] = s + mass[v] * (X[3 * v + l] - Xt[3 * v + l]);
+    g[3 * v + l] = s;
 }
 
 __global__ void k_inertia_energy(const Chunk* __restrict__ chunks, const unsigned char* __restrict__ active,
